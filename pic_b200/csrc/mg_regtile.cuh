@@ -1,0 +1,657 @@
+// Register tiles of the multigrid's graph- and host-loop V-cycle (included by
+// multigrid.cu): the down and up phases of one level, and of two levels in one
+// launch, for up to kRtMaxSweeps red-black sweeps.
+//
+// A block of 8 warps works a 64 x 64 region of a level held in registers: warp
+// w has rows 8w .. 8w+7, lane l the columns 2l and 2l+1 of each.  Region
+// origins are even in both directions, so a node's colour follows from its row
+// and column index at compile time, every lane updates one node per row in
+// every half-sweep, and a half-sweep costs one warp shuffle (the neighbour in
+// the next lane) and about eight arithmetic instructions per update.  Rows on
+// either side of a warp's eight travel through shared memory, two values per
+// lane and one barrier per half-sweep.  The Dirichlet mask comes as bit columns
+// (LevelDev::fb), two words per lane and column.
+//
+// What bounds these phases is instruction issue at large grids and the chain
+// load - sweeps - store at small ones; shared-memory tiles of 32 x 32 (down_tile,
+// up_tile) spend about 370 instructions per node, most of them on addresses,
+// index bounds and mask bytes, with half their threads idle in a half-sweep.
+#pragma once
+
+namespace pic {
+
+constexpr int kRtWarps = 8;
+constexpr int kRtRows = 8;
+constexpr int kRtThreads = 32 * kRtWarps;
+constexpr int kRtSide = 64;  // region side, = kRtWarps * kRtRows = 2 * 32
+constexpr int kRtMaxSweeps = 3;
+
+// How far a phase of S sweeps reaches into the region, from its border (depth
+// 0).  A half-sweep is right one node deeper than what it reads; the first
+// half-sweep of a down phase starts from zero and reads no neighbour.
+//   down   e at depth 2S - 1, the residual at 2S, its restriction at 2S + 1
+//   up     e at depth 2S; with the FP64 residual, e one node around the core
+// Core and left halo are even (two levels: multiples of four), so that every
+// origin keeps its parity.
+template <int S>
+struct RtDown {
+    static constexpr int HL = 2 * S + 2, CORE = kRtSide - HL - 2 * S;
+};
+template <int S, bool RES>
+struct RtUp {
+    static constexpr int HL = RES ? 2 * S + 2 : 2 * S, CORE = RES ? kRtSide - 2 * HL : kRtSide - 4 * S;
+};
+// Two levels, F (the region) and C (32 x 32, one node per lane and row, four
+// rows per warp).
+//   down2  C's right-hand side is right on C nodes [ceil((2S+1)/2),
+//          floor((62-2S)/2)], its restriction 2S + 1 nodes inside that
+//   up2    C is right on [2S, 30 - 2S] (the last lane's prolongation is not
+//          formed), F's prolongation on [4S, 60 - 4S], F on [6S, 60 - 6S]
+template <int S>
+struct RtDown2 {
+    static constexpr int LO = (2 * S + 2) / 2, HI = (62 - 2 * S) / 2;
+    static constexpr int C0 = (LO + 2 * S + 1 + 1) / 2 * 2, C1 = (HI - 2 * S - 1) / 2 * 2;  // first and last C2 centre
+    static constexpr int HL = 2 * C0, CORE = 2 * (C1 + 2 - C0);
+};
+template <int S>
+struct RtUp2 {
+    static constexpr int HL = (6 * S + 3) / 4 * 4, CORE = (60 - 6 * S - HL + 1) / 4 * 4;
+};
+
+// Column bits of 8 (N <= 32) rows from row j of column i: bit r is 1 when node
+// (i, j + r) is free.
+__device__ __forceinline__ unsigned rt_free_bits(const uint32_t* __restrict__ fb, int nx, int nwords, int i, int j,
+                                                 unsigned mask) {
+    const int w = j >> 5;  // floor, j may be negative
+    const bool ci = i >= 0 && i < nx;
+    const unsigned lo = (ci && w >= 0 && w < nwords) ? __ldg(fb + long(w) * nx + i) : 0u;
+    const unsigned hi = (ci && w + 1 >= 0 && w + 1 < nwords) ? __ldg(fb + long(w + 1) * nx + i) : 0u;
+    return __funnelshift_r(lo, hi, unsigned(j & 31)) & mask;
+}
+
+// The coefficients of an over-relaxed Gauss-Seidel update
+//   e <- q e + a (w + e) + bs s + bn n - k g
+// (e + omega (upd - e) with upd = (cx (w + e) + wS s + wN n - g) / diag).
+template <class T>
+struct RtRow {
+    T a, bs, bn, k;
+};
+
+// r-z rows keep {wN, wS, 1/diag, D} in registers; Cartesian rows share one set.
+template <class T, int ROWS, bool CYL>
+struct RtCoef {
+    T cx, cy, omega;
+    RtRow<T> c;             // Cartesian
+    T rz[CYL ? ROWS : 1][4];
+    __device__ __forceinline__ void load(const LevelDev<T>& L, T om, int j0) {
+        cx = L.cx;
+        cy = L.cy;
+        omega = om;
+        if constexpr (CYL) {
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) {
+                const int j = j0 + r;
+                const bool in = j >= 0 && j < L.ny;
+#pragma unroll
+                for (int q = 0; q < 4; ++q) rz[r][q] = in ? __ldg(L.rz + 4 * j + q) : T(0);
+            }
+        } else {
+            c.k = om * L.inv_diag;
+            c.a = c.k * L.cx;
+            c.bs = c.bn = c.k * L.cy;
+        }
+    }
+    __device__ __forceinline__ RtRow<T> row(int r) const {
+        if constexpr (CYL) {
+            const T k = omega * rz[r][2];
+            return RtRow<T>{k * cx, k * rz[r][1], k * rz[r][0], k};
+        } else {
+            return c;
+        }
+    }
+};
+
+// One region of F: 8 rows x 2 columns per lane, and the rows on either side.
+template <class T>
+struct RtTile {
+    T e[kRtRows][2], g[kRtRows][2];
+    T up[2], dn[2];  // row -1 (the warp above) and row 8, per column
+    unsigned fr[2];  // free bits of the rows, per column
+};
+
+// Shared exchange rows, two buffers used in turn: a buffer is written again
+// only after the barrier between its readers and the next-but-one exchange.
+template <class T>
+struct RtShared {
+    T x[2][kRtWarps][2][32];
+};
+
+// Publishes, of the nodes of one colour, row 0 (its column COLOR & 1) and row
+// 7 (its other column), and reads the neighbouring warps' into up and dn.
+template <class T, int COLOR>
+__device__ __forceinline__ void rt_exchange(RtTile<T>& t, RtShared<T>& s, int& buf) {
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    constexpr int c0 = COLOR & 1, c7 = (kRtRows - 1 + COLOR) & 1;
+    s.x[buf][w][0][l] = t.e[0][c0];
+    s.x[buf][w][1][l] = t.e[kRtRows - 1][c7];
+    __syncthreads();
+    if (w > 0) t.up[c7] = s.x[buf][w - 1][1][l];
+    if (w < kRtWarps - 1) t.dn[c0] = s.x[buf][w + 1][0][l];
+    buf ^= 1;
+}
+
+// One half-sweep (COLOR 0: red, (i + j) even).
+template <class T, int COLOR, bool CYL>
+__device__ __forceinline__ void rt_half_sweep(RtTile<T>& t, const RtCoef<T, kRtRows, CYL>& cf) {
+    const T q = T(1) - cf.omega;
+#pragma unroll
+    for (int r = 0; r < kRtRows; ++r) {
+        const int c = (r + COLOR) & 1;
+        const RtRow<T> k = cf.row(r);
+        const T side = c ? __shfl_down_sync(0xffffffffu, t.e[r][0], 1) : __shfl_up_sync(0xffffffffu, t.e[r][1], 1);
+        const T s = r > 0 ? t.e[r - 1][c] : t.up[c];
+        const T n = r < kRtRows - 1 ? t.e[r + 1][c] : t.dn[c];
+        T v = q * t.e[r][c] - k.k * t.g[r][c];
+        v += k.a * (side + t.e[r][1 - c]);
+        if constexpr (CYL) v += k.bs * s + k.bn * n;
+        else v += k.bs * (s + n);
+        if ((t.fr[c] >> r) & 1u) t.e[r][c] = v;
+    }
+}
+
+// S sweeps.  FROM_ZERO: e = 0 everywhere before the first half-sweep, which
+// reads no neighbour; else the initial rows are exchanged first.  LAST: the
+// black rows after the last half-sweep are exchanged too (for a residual).
+template <class T, int S, bool CYL, bool FROM_ZERO, bool LAST>
+__device__ __forceinline__ void rt_sweeps(RtTile<T>& t, const RtCoef<T, kRtRows, CYL>& cf, RtShared<T>& sh, int& buf) {
+    t.up[0] = t.up[1] = t.dn[0] = t.dn[1] = T(0);
+    if constexpr (!FROM_ZERO) {
+        rt_exchange<T, 1>(t, sh, buf);
+    }
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        if (FROM_ZERO && s == 0) {
+#pragma unroll
+            for (int r = 0; r < kRtRows; ++r) {
+                const int c = r & 1;
+                t.e[r][c] = ((t.fr[c] >> r) & 1u) ? -(cf.row(r).k * t.g[r][c]) : T(0);
+                t.e[r][1 - c] = T(0);
+            }
+        } else {
+            rt_half_sweep<T, 0, CYL>(t, cf);
+        }
+        rt_exchange<T, 0>(t, sh, buf);
+        rt_half_sweep<T, 1, CYL>(t, cf);
+        if (LAST || s < S - 1) rt_exchange<T, 1>(t, sh, buf);
+    }
+}
+
+// The residual g - A e of the region, 0 on Dirichlet nodes (r-z: weighted by
+// the row's volume), returned as its horizontal full weighting at the even
+// columns, h = r/2 + (r_west + r_east)/4.
+template <class T, bool CYL>
+__device__ __forceinline__ void rt_residual_h(const RtTile<T>& t, const RtCoef<T, kRtRows, CYL>& cf,
+                                              T (&h)[kRtRows]) {
+#pragma unroll
+    for (int r = 0; r < kRtRows; ++r) {
+        T res[2];
+        const T w = __shfl_up_sync(0xffffffffu, t.e[r][1], 1), ea = __shfl_down_sync(0xffffffffu, t.e[r][0], 1);
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const T e = t.e[r][c];
+            const T wv = c ? t.e[r][0] : w, ev = c ? ea : t.e[r][1];
+            const T s = r > 0 ? t.e[r - 1][c] : t.up[c];
+            const T n = r < kRtRows - 1 ? t.e[r + 1][c] : t.dn[c];
+            T v;
+            if constexpr (CYL) {
+                const T lap = cf.cx * (wv + ev - T(2) * e) + cf.rz[r][0] * (n - e) + cf.rz[r][1] * (s - e);
+                v = cf.rz[r][3] * (t.g[r][c] - lap);
+            } else {
+                v = t.g[r][c] - (cf.cx * (wv + ev - T(2) * e) + cf.cy * (s + n - T(2) * e));
+            }
+            res[c] = ((t.fr[c] >> r) & 1u) ? v : T(0);
+        }
+        const T rw = __shfl_up_sync(0xffffffffu, res[1], 1);
+        h[r] = T(0.5) * res[0] + T(0.25) * (rw + res[1]);
+    }
+}
+
+// Full weighting of the four coarse rows of this warp (the fine rows 0, 2, 4,
+// 6) from the horizontal weights; J0: the coarse row of fine row 0.
+template <class T, bool CYL>
+__device__ __forceinline__ void rt_restrict(const T (&h)[kRtRows], RtShared<T>& sh, int& buf, int J0, T (&out)[4]) {
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    sh.x[buf][w][1][l] = h[kRtRows - 1];
+    __syncthreads();
+    const T above = w > 0 ? sh.x[buf][w - 1][1][l] : T(0);
+    buf ^= 1;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const T s = q > 0 ? h[2 * q - 1] : above;
+        T v = T(0.5) * h[2 * q] + T(0.25) * (s + h[2 * q + 1]);
+        // r-z: divided by the stencil's weighted volume (2J; 5/16 on the axis)
+        if constexpr (CYL) v *= J0 + q == 0 ? T(3.2) : T(0.5) / T(J0 + q);
+        out[q] = v;
+    }
+}
+
+// Loads g of the region (from g64, the FP64 residual, when given) and the
+// free bits.
+template <class T>
+__device__ __forceinline__ void rt_load_bits(const LevelDev<T>& L, int i0, int j0, RtTile<T>& t) {
+    const int nw = (L.ny + 31) >> 5;
+    t.fr[0] = rt_free_bits(L.fb, L.nx, nw, i0, j0, 0xffu);
+    t.fr[1] = rt_free_bits(L.fb, L.nx, nw, i0 + 1, j0, 0xffu);
+}
+
+template <class T, class G>
+__device__ __forceinline__ void rt_load_rows(const G* __restrict__ src, int nx, int ny, int i0, int j0,
+                                             T (&v)[kRtRows][2]) {
+    const bool c0 = i0 >= 0 && i0 < nx, c1 = i0 + 1 >= 0 && i0 + 1 < nx;
+    const G* p = src + long(j0) * nx + i0;
+#pragma unroll
+    for (int r = 0; r < kRtRows; ++r) {
+        const bool in = j0 + r >= 0 && j0 + r < ny;
+        v[r][0] = (in && c0) ? T(p[long(r) * nx]) : T(0);
+        v[r][1] = (in && c1) ? T(p[long(r) * nx + 1]) : T(0);
+    }
+}
+
+// Stores the core's nodes of a field of the region.
+template <class T, int HL, int CORE>
+__device__ __forceinline__ void rt_store_core(T* __restrict__ dst, const T (&v)[kRtRows][2], int nx, int ny, int i0,
+                                              int j0) {
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    if (2 * l < HL || 2 * l >= HL + CORE) return;
+    T* p = dst + long(j0) * nx + i0;
+#pragma unroll
+    for (int r = 0; r < kRtRows; ++r) {
+        const int lr = w * kRtRows + r;
+        if (lr < HL || lr >= HL + CORE || j0 + r >= ny) continue;
+        if (i0 < nx) p[long(r) * nx] = v[r][0];
+        if (i0 + 1 < nx) p[long(r) * nx + 1] = v[r][1];
+    }
+}
+
+// ---- one level -----------------------------------------------------------------------
+
+// The down phase (see k_mg_down): smooth from zero, restrict the residual.
+template <class T, int S, bool CYL>
+__global__ void __launch_bounds__(kRtThreads) k_rt_down(LevelDev<T> F, LevelDev<T> C, T omega,
+                                                        const double* __restrict__ g64) {
+    using G = RtDown<S>;
+    __shared__ RtShared<T> sh;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int i0 = int(blockIdx.x) * G::CORE - G::HL + 2 * l, j0 = int(blockIdx.y) * G::CORE - G::HL + kRtRows * w;
+    // the coarse column and rows this lane restricts to (i0, j0 are even)
+    const int I = i0 >> 1, J0 = j0 >> 1;
+    RtTile<T> t;
+    RtCoef<T, kRtRows, CYL> cf;
+    rt_load_bits(F, i0, j0, t);
+    const unsigned cfr = rt_free_bits(C.fb, C.nx, (C.ny + 31) >> 5, I, J0, 0xfu);
+    cf.load(F, omega, j0);
+    pdl_wait();
+    pdl_trigger();
+    if (g64) rt_load_rows<T, double>(g64, F.nx, F.ny, i0, j0, t.g);
+    else rt_load_rows<T, T>(F.g, F.nx, F.ny, i0, j0, t.g);
+    int buf = 0;
+    rt_sweeps<T, S, CYL, true, true>(t, cf, sh, buf);
+    rt_store_core<T, G::HL, G::CORE>(F.e, t.e, F.nx, F.ny, i0, j0);
+    if (g64) rt_store_core<T, G::HL, G::CORE>(F.g, t.g, F.nx, F.ny, i0, j0);
+    T h[kRtRows], out[4];
+    rt_residual_h<T, CYL>(t, cf, h);
+    rt_restrict<T, CYL>(h, sh, buf, J0, out);
+    if (2 * l < G::HL || 2 * l >= G::HL + G::CORE || I >= C.nx) return;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int lr = w * kRtRows + 2 * q;
+        if (lr < G::HL || lr >= G::HL + G::CORE || J0 + q >= C.ny) continue;
+        C.g[long(J0 + q) * C.nx + I] = ((cfr >> q) & 1u) ? out[q] : T(0);
+    }
+}
+
+// Adds the bilinear prolongation of the coarse rows cv (coarse rows of fine
+// rows 0, 2, 4, 6 and 8) and their east neighbours ce on the free nodes; e is 0
+// elsewhere.
+template <class T>
+__device__ __forceinline__ void rt_prolong(RtTile<T>& t, const T (&cv)[5], const T (&ce)[5]) {
+#pragma unroll
+    for (int r = 0; r < kRtRows; ++r) {
+        const int q = r >> 1;
+        T a = cv[q], b = T(0.5) * (cv[q] + ce[q]);
+        if (r & 1) {
+            a = T(0.5) * (cv[q] + cv[q + 1]);
+            b = T(0.25) * (cv[q] + ce[q] + cv[q + 1] + ce[q + 1]);
+        }
+        t.e[r][0] = ((t.fr[0] >> r) & 1u) ? t.e[r][0] + a : T(0);
+        t.e[r][1] = ((t.fr[1] >> r) & 1u) ? t.e[r][1] + b : T(0);
+    }
+}
+
+// The up phase (see k_mg_up, k_mg_up_res): add the prolonged coarse
+// correction and smooth; RES (level 0): phi += e and the FP64 residual
+// r -= A e on the core, its norm and the loop decision.
+template <class T, int S, bool CYL, bool RES>
+__global__ void __launch_bounds__(kRtThreads) k_rt_up(LevelDev<T> F, LevelDev<T> C, T omega, double* __restrict__ phi,
+                                                      ResArgs R) {
+    using G = RtUp<S, RES>;
+    __shared__ RtShared<T> sh;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int i0 = int(blockIdx.x) * G::CORE - G::HL + 2 * l, j0 = int(blockIdx.y) * G::CORE - G::HL + kRtRows * w;
+    RtTile<T> t;
+    RtCoef<T, kRtRows, CYL> cf;
+    rt_load_bits(F, i0, j0, t);
+    cf.load(F, omega, j0);
+    // everything but the coarse correction was written two or more launches back
+    rt_load_rows<T, T>(F.e, F.nx, F.ny, i0, j0, t.e);
+    rt_load_rows<T, T>(F.g, F.nx, F.ny, i0, j0, t.g);
+    const bool core_col = 2 * l >= G::HL && 2 * l < G::HL + G::CORE;
+    double pv[RES ? kRtRows : 1][2], rv[RES ? kRtRows : 1][2];
+    if constexpr (RES) {
+#pragma unroll
+        for (int r = 0; r < kRtRows; ++r) {
+            const int lr = w * kRtRows + r;
+            const bool in = core_col && lr >= G::HL && lr < G::HL + G::CORE && j0 + r < F.ny;
+            const long k = long(j0 + r) * F.nx + i0;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                const bool ic = in && i0 + c < F.nx;
+                pv[r][c] = ic ? phi[k + c] : 0.0;
+                rv[r][c] = ic ? R.r64[k + c] : 0.0;
+            }
+        }
+    }
+    pdl_wait();
+    pdl_trigger();
+    {
+        const int I = i0 >> 1, J0 = j0 >> 1;
+        T cv[5], ce[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            const int J = J0 + q;
+            const bool in = J >= 0 && J < C.ny;
+            const T* p = C.ec + long(J) * C.nx + I;
+            cv[q] = (in && I >= 0 && I < C.nx) ? p[0] : T(0);
+            // the last lane's east neighbour is not in the warp
+            const T x = (l == 31 && in && I + 1 >= 0 && I + 1 < C.nx) ? p[1] : T(0);
+            const T y = __shfl_down_sync(0xffffffffu, cv[q], 1);
+            ce[q] = l == 31 ? x : y;
+        }
+        rt_prolong(t, cv, ce);
+    }
+    int buf = 0;
+    // the red rows' neighbours are black: they are exchanged before the first half-sweep
+    rt_sweeps<T, S, CYL, false, RES>(t, cf, sh, buf);
+    if constexpr (!RES) {
+        rt_store_core<T, G::HL, G::CORE>(F.ec, t.e, F.nx, F.ny, i0, j0);
+    } else {
+        double r2 = 0.0;
+#pragma unroll
+        for (int r = 0; r < kRtRows; ++r) {
+            const int lr = w * kRtRows + r, j = j0 + r;
+            const T ww = __shfl_up_sync(0xffffffffu, t.e[r][1], 1), ee = __shfl_down_sync(0xffffffffu, t.e[r][0], 1);
+            const bool in = core_col && lr >= G::HL && lr < G::HL + G::CORE && j < F.ny;
+            const long k = long(j) * F.nx + i0;
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                if (!in || i0 + c >= F.nx) continue;
+                phi[k + c] = pv[r][c] + double(t.e[r][c]);
+                if (!((t.fr[c] >> r) & 1u)) continue;
+                // f - A(phi + e) = r - A e, in the association of k_mg_r0's Laplacian
+                const double e = double(t.e[r][c]);
+                const double wv = double(c ? t.e[r][0] : ww), ev = double(c ? ee : t.e[r][1]);
+                const double s = double(r > 0 ? t.e[r - 1][c] : t.up[c]);
+                const double n = double(r < kRtRows - 1 ? t.e[r + 1][c] : t.dn[c]);
+                double lap;
+                if constexpr (CYL)
+                    lap = R.cx * ((wv - e) + (ev - e)) + R.rz0[4 * j] * (n - e) + R.rz0[4 * j + 1] * (s - e);
+                else
+                    lap = R.cx * ((wv - e) + (ev - e)) + R.cy * ((s - e) + (n - e));
+                const double rr = rv[r][c] - lap;
+                R.r64[k + c] = rr;
+                r2 += rr * rr;
+            }
+        }
+        norm_reduce_decide(r2, 0.0, R.N, R.tol2, R.max_cycles, 0, R.cond, R.use_cond);
+    }
+}
+
+// ---- two levels in one launch ---------------------------------------------------------
+//
+// C's region: lane l has column C-origin + l, warp w the rows 4w .. 4w+3.  The
+// origin is even, so a node's colour is (l + row) & 1: in a half-sweep a lane
+// updates one row of each pair of rows, the odd or the even one by its parity.
+
+template <class T>
+struct RtCTile {
+    T e[4], g[4];
+    T up, dn;  // rows -1 and 4
+    unsigned fr;
+};
+
+template <class T>
+__device__ __forceinline__ void rt_c_exchange(RtCTile<T>& t, RtShared<T>& s, int& buf) {
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    s.x[buf][w][0][l] = t.e[0];
+    s.x[buf][w][1][l] = t.e[3];
+    __syncthreads();
+    if (w > 0) t.up = s.x[buf][w - 1][1][l];
+    if (w < kRtWarps - 1) t.dn = s.x[buf][w + 1][0][l];
+    buf ^= 1;
+}
+
+template <class T, bool CYL>
+__device__ __forceinline__ void rt_c_half_sweep(RtCTile<T>& t, const RtCoef<T, 4, CYL>& cf, int color) {
+    const bool odd = ((threadIdx.x + color) & 1) != 0;  // this lane's row of each pair
+    const T q = T(1) - cf.omega;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+        const int a = 2 * p, b = a + 1;
+        // the neighbouring lanes update the pair's other row: they send this lane's
+        const T send = odd ? t.e[a] : t.e[b];
+        const T wv = __shfl_up_sync(0xffffffffu, send, 1), ev = __shfl_down_sync(0xffffffffu, send, 1);
+        const T below = a > 0 ? t.e[a - 1] : t.up, above = b < 3 ? t.e[b + 1] : t.dn;
+        const T s = odd ? t.e[a] : below, n = odd ? above : t.e[b];
+        const T old = odd ? t.e[b] : t.e[a], g = odd ? t.g[b] : t.g[a];
+        T v;
+        if constexpr (CYL) {
+            const RtRow<T> ka = cf.row(a), kb = cf.row(b);
+            const T kk = odd ? kb.k : ka.k, bs = odd ? kb.bs : ka.bs, bn = odd ? kb.bn : ka.bn;
+            v = q * old - kk * g + (kk * cf.cx) * (wv + ev) + (bs * s + bn * n);
+        } else {
+            v = q * old - cf.c.k * g + cf.c.a * (wv + ev) + cf.c.bs * (s + n);
+        }
+        const bool fa = (t.fr >> a) & 1u, fb = (t.fr >> b) & 1u;
+        if (!odd && fa) t.e[a] = v;
+        if (odd && fb) t.e[b] = v;
+    }
+}
+
+// S sweeps of C; every exchange carries both colours' boundary rows.
+template <class T, int S, bool CYL, bool FROM_ZERO>
+__device__ __forceinline__ void rt_c_sweeps(RtCTile<T>& t, const RtCoef<T, 4, CYL>& cf, RtShared<T>& sh, int& buf) {
+    t.up = t.dn = T(0);
+    if (!FROM_ZERO) rt_c_exchange(t, sh, buf);
+#pragma unroll
+    for (int s = 0; s < S; ++s) {
+        rt_c_half_sweep<T, CYL>(t, cf, 0);
+        rt_c_exchange(t, sh, buf);
+        rt_c_half_sweep<T, CYL>(t, cf, 1);
+        rt_c_exchange(t, sh, buf);
+    }
+}
+
+template <class T, int S, bool CYL>
+__global__ void __launch_bounds__(kRtThreads) k_rt_down2(LevelDev<T> F, LevelDev<T> C, LevelDev<T> C2, T omega) {
+    using G = RtDown2<S>;
+    __shared__ RtShared<T> sh;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int i0 = int(blockIdx.x) * G::CORE - G::HL + 2 * l, j0 = int(blockIdx.y) * G::CORE - G::HL + kRtRows * w;
+    const int I = i0 >> 1, J0 = j0 >> 1;
+    RtTile<T> t;
+    RtCTile<T> ct;
+    RtCoef<T, kRtRows, CYL> cf;
+    RtCoef<T, 4, CYL> cc;
+    rt_load_bits(F, i0, j0, t);
+    ct.fr = rt_free_bits(C.fb, C.nx, (C.ny + 31) >> 5, I, J0, 0xfu);
+    const unsigned c2fr = rt_free_bits(C2.fb, C2.nx, (C2.ny + 31) >> 5, I >> 1, J0 >> 1, 0x3u);
+    cf.load(F, omega, j0);
+    cc.load(C, omega, J0);
+    pdl_wait();
+    pdl_trigger();
+    rt_load_rows<T, T>(F.g, F.nx, F.ny, i0, j0, t.g);
+    int buf = 0;
+    rt_sweeps<T, S, CYL, true, true>(t, cf, sh, buf);
+    rt_store_core<T, G::HL, G::CORE>(F.e, t.e, F.nx, F.ny, i0, j0);
+    T h[kRtRows], out[4];
+    rt_residual_h<T, CYL>(t, cf, h);
+    rt_restrict<T, CYL>(h, sh, buf, J0, out);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        ct.g[q] = ((ct.fr >> q) & 1u) ? out[q] : T(0);
+        ct.e[q] = T(0);
+    }
+    rt_c_sweeps<T, S, CYL, true>(ct, cc, sh, buf);
+    // C's core: its e and g for the up phase
+    const bool ccol = 2 * l >= G::HL && 2 * l < G::HL + G::CORE && I < C.nx;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const int lr = w * kRtRows + 2 * q;
+        if (!ccol || lr < G::HL || lr >= G::HL + G::CORE || J0 + q >= C.ny) continue;
+        const long K = long(J0 + q) * C.nx + I;
+        C.e[K] = ct.e[q];
+        C.g[K] = ct.g[q];
+    }
+    // C's residual, weighted along the row at the even columns (even lanes)
+    T hc[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const T e = ct.e[q];
+        const T wv = __shfl_up_sync(0xffffffffu, e, 1), ev = __shfl_down_sync(0xffffffffu, e, 1);
+        const T s = q > 0 ? ct.e[q - 1] : ct.up, n = q < 3 ? ct.e[q + 1] : ct.dn;
+        T v;
+        if constexpr (CYL) {
+            const T lap = cc.cx * (wv + ev - T(2) * e) + cc.rz[q][0] * (n - e) + cc.rz[q][1] * (s - e);
+            v = cc.rz[q][3] * (ct.g[q] - lap);
+        } else {
+            v = ct.g[q] - (cc.cx * (wv + ev - T(2) * e) + cc.cy * (s + n - T(2) * e));
+        }
+        const T r = ((ct.fr >> q) & 1u) ? v : T(0);
+        const T rw = __shfl_up_sync(0xffffffffu, r, 1), re = __shfl_down_sync(0xffffffffu, r, 1);
+        hc[q] = T(0.5) * r + T(0.25) * (rw + re);
+    }
+    sh.x[buf][w][1][l] = hc[3];
+    __syncthreads();
+    const T above = w > 0 ? sh.x[buf][w - 1][1][l] : T(0);
+    const int I2 = I >> 1, J2 = J0 >> 1;
+    if ((l & 1) || !ccol || I2 >= C2.nx) return;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int lr = w * kRtRows + 4 * q, J = J2 + q;
+        if (lr < G::HL || lr >= G::HL + G::CORE || J >= C2.ny) continue;
+        T v = T(0.5) * hc[2 * q] + T(0.25) * ((q > 0 ? hc[1] : above) + hc[2 * q + 1]);
+        if constexpr (CYL) v *= J == 0 ? T(3.2) : T(0.5) / T(J);
+        C2.g[long(J) * C2.nx + I2] = ((c2fr >> q) & 1u) ? v : T(0);
+    }
+}
+
+template <class T, int S, bool CYL>
+__global__ void __launch_bounds__(kRtThreads) k_rt_up2(LevelDev<T> F, LevelDev<T> C, LevelDev<T> C2, T omega) {
+    using G = RtUp2<S>;
+    __shared__ RtShared<T> sh;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int i0 = int(blockIdx.x) * G::CORE - G::HL + 2 * l, j0 = int(blockIdx.y) * G::CORE - G::HL + kRtRows * w;
+    const int I = i0 >> 1, J0 = j0 >> 1;
+    RtTile<T> t;
+    RtCTile<T> ct;
+    RtCoef<T, kRtRows, CYL> cf;
+    RtCoef<T, 4, CYL> cc;
+    rt_load_bits(F, i0, j0, t);
+    ct.fr = rt_free_bits(C.fb, C.nx, (C.ny + 31) >> 5, I, J0, 0xfu);
+    cf.load(F, omega, j0);
+    cc.load(C, omega, J0);
+    rt_load_rows<T, T>(F.e, F.nx, F.ny, i0, j0, t.e);
+    rt_load_rows<T, T>(F.g, F.nx, F.ny, i0, j0, t.g);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const bool in = J0 + q >= 0 && J0 + q < C.ny && I >= 0 && I < C.nx;
+        const long K = long(J0 + q) * C.nx + I;
+        ct.e[q] = in ? C.e[K] : T(0);
+        ct.g[q] = in ? C.g[K] : T(0);
+    }
+    pdl_wait();
+    pdl_trigger();
+    {
+        // C2's correction prolonged onto C: an odd column takes the mean of
+        // its own C2 column and the next lane's
+        const int I2 = I >> 1, J2 = J0 >> 1;
+        T v2[3];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const int J = J2 + q;
+            const bool in = J >= 0 && J < C2.ny && I2 >= 0 && I2 < C2.nx;
+            const T v = in ? C2.ec[long(J) * C2.nx + I2] : T(0);
+            const T e = __shfl_down_sync(0xffffffffu, v, 1);
+            v2[q] = (l & 1) ? T(0.5) * (v + e) : v;
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const T v = (q & 1) ? T(0.5) * (v2[q >> 1] + v2[(q >> 1) + 1]) : v2[q >> 1];
+            ct.e[q] = ((ct.fr >> q) & 1u) ? ct.e[q] + v : T(0);
+        }
+    }
+    int buf = 0;
+    rt_c_sweeps<T, S, CYL, false>(ct, cc, sh, buf);
+    {
+        T cv[5] = {ct.e[0], ct.e[1], ct.e[2], ct.e[3], ct.dn}, ce[5];
+#pragma unroll
+        for (int q = 0; q < 5; ++q) ce[q] = __shfl_down_sync(0xffffffffu, cv[q], 1);
+        rt_prolong(t, cv, ce);
+    }
+    rt_sweeps<T, S, CYL, false, false>(t, cf, sh, buf);
+    rt_store_core<T, G::HL, G::CORE>(F.ec, t.e, F.nx, F.ny, i0, j0);
+}
+
+// ---- launch tables ----------------------------------------------------------------------
+
+template <class T>
+using RtUpKernel = void (*)(LevelDev<T>, LevelDev<T>, T, double*, ResArgs);
+
+template <class T, bool CYL>
+static DownKernel<T> rt_down_kernel(int s) {
+    static const DownKernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_down<T, 1, CYL>, k_rt_down<T, 2, CYL>,
+                                                      k_rt_down<T, 3, CYL>};
+    return k[s];
+}
+
+template <class T, bool CYL, bool RES>
+static RtUpKernel<T> rt_up_kernel(int s) {
+    static const RtUpKernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_up<T, 1, CYL, RES>, k_rt_up<T, 2, CYL, RES>,
+                                                      k_rt_up<T, 3, CYL, RES>};
+    return k[s];
+}
+
+template <class T, bool CYL>
+static Fused2Kernel<T> rt_down2_kernel(int s) {
+    static const Fused2Kernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_down2<T, 1, CYL>, k_rt_down2<T, 2, CYL>,
+                                                        k_rt_down2<T, 3, CYL>};
+    return k[s];
+}
+
+template <class T, bool CYL>
+static Fused2Kernel<T> rt_up2_kernel(int s) {
+    static const Fused2Kernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_up2<T, 1, CYL>, k_rt_up2<T, 2, CYL>,
+                                                        k_rt_up2<T, 3, CYL>};
+    return k[s];
+}
+
+// Core sides of the phases (tiles per direction = ceil(n / core)).
+static int rt_down_core(int s) { return s == 1 ? RtDown<1>::CORE : s == 2 ? RtDown<2>::CORE : RtDown<3>::CORE; }
+static int rt_up_core(int s, bool res) {
+    if (res) return s == 1 ? RtUp<1, true>::CORE : s == 2 ? RtUp<2, true>::CORE : RtUp<3, true>::CORE;
+    return s == 1 ? RtUp<1, false>::CORE : s == 2 ? RtUp<2, false>::CORE : RtUp<3, false>::CORE;
+}
+static int rt_down2_core(int s) { return s == 1 ? RtDown2<1>::CORE : s == 2 ? RtDown2<2>::CORE : RtDown2<3>::CORE; }
+static int rt_up2_core(int s) { return s == 1 ? RtUp2<1>::CORE : s == 2 ? RtUp2<2>::CORE : RtUp2<3>::CORE; }
+
+}  // namespace pic

@@ -72,6 +72,7 @@ struct LevelDev {
     int nx, ny;
     T cx, cy, inv_diag;
     const uint8_t* mask;  // 1 = Dirichlet
+    const uint32_t* fb;   // free nodes as bit columns: word [j >> 5][i], bit j & 31 (edges and mask applied)
     T* e;
     T* eu;
     T* ec;
@@ -836,6 +837,12 @@ static Fused2Kernel<T> up2_kernel(int s) {
         k_mg_up2<T, 5>,  k_mg_up2<T, 6>, k_mg_up2<T, 7>, k_mg_up2<T, 8>};
     return k[s];
 }
+
+}  // namespace pic
+
+#include "mg_regtile.cuh"
+
+namespace pic {
 
 template <class T>
 static size_t down2_smem(int s) {
@@ -1786,6 +1793,17 @@ static int alloc_levels(MgImpl& M, std::vector<LevelDev<T>>& lv, const std::vect
         M.allocs.push_back(mk);
         PIC_CUDA(cudaMemcpy(mk, masks[l].data(), G, cudaMemcpyHostToDevice));
         v.mask = mk;
+        // the free nodes (not Dirichlet, not on a grid edge; in r-z the axis
+        // row is free) as bit columns
+        std::vector<uint32_t> fb(size_t((v.ny + 31) / 32) * v.nx, 0u);
+        for (int j = M.rz ? 0 : 1; j < v.ny - 1; ++j)
+            for (int i = 1; i < v.nx - 1; ++i)
+                if (!masks[l][size_t(j) * v.nx + i]) fb[size_t(j >> 5) * v.nx + i] |= 1u << (j & 31);
+        uint32_t* fbd = nullptr;
+        PIC_CUDA(cudaMalloc(&fbd, fb.size() * sizeof(uint32_t)));
+        M.allocs.push_back(fbd);
+        PIC_CUDA(cudaMemcpy(fbd, fb.data(), fb.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
+        v.fb = fbd;
         // padded to 16 bytes: the coarse kernel reads g in 16-byte words
         const size_t bytes = (G * sizeof(T) + 15) / 16 * 16;
         PIC_CUDA(cudaMalloc(&v.e, bytes));
@@ -2258,7 +2276,10 @@ int mg_create(int nx, int ny, double dx, double dy, const uint8_t* h_mask, const
     if (st == PIC_OK && M.Lc >= 1 &&
         (M.o.launch_mode == PIC_MG_GRAPH_LOOP || M.o.launch_mode == PIC_MG_HOST_LOOP))
         st = configure_direct(M, nxs, nys, masks);
-    if (st == PIC_OK && M.direct && !M.rz && M.Lc >= 3)
+    // two levels per launch: Cartesian, or both phases on register tiles
+    const bool rt2 = M.o.pre_sweeps <= kRtMaxSweeps && M.o.post_sweeps <= kRtMaxSweeps;
+    if (st == PIC_OK && M.direct && M.Lc >= 3 && rt2) M.fuse2 = true;
+    else if (st == PIC_OK && M.direct && !M.rz && M.Lc >= 3)
         st = M.precision == PIC_MG_MIXED ? configure_fuse2<float>(M) : configure_fuse2<double>(M);
     if (st != PIC_OK) return bail(st);
     M.grd0 = dim3(div_up(nx, M.blk0.x), div_up(ny, M.blk0.y * kR0Rows));
@@ -2323,28 +2344,38 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
     const int Ltile = hyb ? M.Lt : M.Lc;
     const std::vector<LevelDev<T>> lv = with_corrections(lv_in, hyb ? M.Lp : M.Lc);
     const T omega = T(M.o.omega);
-    const size_t down = down_smem<T>(M.o.pre_sweeps, M.rz), up = up_smem<T>(M.o.post_sweeps, M.rz);
-    const DownKernel<T> kdown = M.rz ? down_kernel<T, true>(M.o.pre_sweeps) : down_kernel<T, false>(M.o.pre_sweeps);
-    const UpKernel<T> kup = M.rz ? up_kernel<T, true>(M.o.post_sweeps) : up_kernel<T, false>(M.o.post_sweeps);
+    // register tiles (mg_regtile.cuh) up to kRtMaxSweeps sweeps, shared-memory
+    // tiles for more: the register tile's halo grows with the sweeps and its
+    // region does not
+    const int pre = M.o.pre_sweeps, post = M.o.post_sweeps;
+    const bool rtd = pre <= kRtMaxSweeps, rtu = post <= kRtMaxSweeps;
+    const size_t down = rtd ? 0 : down_smem<T>(pre, M.rz), up = rtu ? 0 : up_smem<T>(post, M.rz);
+    const dim3 bd(rtd ? kRtThreads : kMgThreads), bu(rtu ? kRtThreads : kMgThreads);
+    const DownKernel<T> kdown = rtd ? (M.rz ? rt_down_kernel<T, true>(pre) : rt_down_kernel<T, false>(pre))
+                                    : (M.rz ? down_kernel<T, true>(pre) : down_kernel<T, false>(pre));
+    auto tiles = [&](int l, int side) { return dim3(div_up(lv[l].nx, side), div_up(lv[l].ny, side)); };
     count = 0;
     // levels Lc-2 and Lc-1 in one launch each way where that applies
     const bool f2 = M.fuse2 && !hyb;
     const int Lsingle = f2 ? Ltile - 2 : Ltile;
     for (int l = 0; l < Lsingle; ++l) {
-        const dim3 g(div_up(lv[l].nx, kMgTile), div_up(lv[l].ny, kMgTile));
+        const dim3 g = tiles(l, rtd ? rt_down_core(pre) : kMgTile);
         // the finest down phase waits for its predecessor to finish before it
         // is placed: launched ahead, its CTAs would take the SMs its
         // predecessor leaves free first, several to an SM (measured 8.5 us
         // instead of 4.8 at 513^2)
-        if (l == 0) kdown<<<g, dim3(kMgThreads), down, st>>>(lv[0], lv[1], omega, (const double*)M.r64);
-        else launch_pdl(kdown, g, dim3(kMgThreads), down, st, lv[l], lv[l + 1], omega, (const double*)nullptr);
+        if (l == 0) kdown<<<g, bd, down, st>>>(lv[0], lv[1], omega, (const double*)M.r64);
+        else launch_pdl(kdown, g, bd, down, st, lv[l], lv[l + 1], omega, (const double*)nullptr);
         ++count;
     }
     if (f2) {
         const int l = Lsingle;
-        const dim3 g(div_up(lv[l].nx, kMgTile), div_up(lv[l].ny, kMgTile));
-        launch_pdl(down2_kernel<T>(M.o.pre_sweeps), g, dim3(kMgThreads), down2_smem<T>(M.o.pre_sweeps), st, lv[l],
-                   lv[l + 1], lv[l + 2], omega);
+        if (rtd)
+            launch_pdl(M.rz ? rt_down2_kernel<T, true>(pre) : rt_down2_kernel<T, false>(pre),
+                       tiles(l, rt_down2_core(pre)), bd, 0, st, lv[l], lv[l + 1], lv[l + 2], omega);
+        else
+            launch_pdl(down2_kernel<T>(pre), tiles(l, kMgTile), bd, down2_smem<T>(pre), st, lv[l], lv[l + 1],
+                       lv[l + 2], omega);
         ++count;
     }
     if constexpr (std::is_same<T, float>::value) {
@@ -2367,14 +2398,22 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
     }
     if (f2) {
         const int l = Lsingle;
-        const dim3 g(div_up(lv[l].nx, kMgTile), div_up(lv[l].ny, kMgTile));
-        launch_pdl(up2_kernel<T>(M.o.post_sweeps), g, dim3(kMgThreads), up2_smem<T>(M.o.post_sweeps), st, lv[l],
-                   lv[l + 1], lv[l + 2], omega);
+        if (rtu)
+            launch_pdl(M.rz ? rt_up2_kernel<T, true>(post) : rt_up2_kernel<T, false>(post), tiles(l, rt_up2_core(post)),
+                       bu, 0, st, lv[l], lv[l + 1], lv[l + 2], omega);
+        else
+            launch_pdl(up2_kernel<T>(post), tiles(l, kMgTile), bu, up2_smem<T>(post), st, lv[l], lv[l + 1], lv[l + 2],
+                       omega);
         ++count;
     }
     for (int l = Lsingle - 1; l >= 1; --l) {
-        const dim3 g(div_up(lv[l].nx, kMgTile), div_up(lv[l].ny, kMgTile));
-        launch_pdl(kup, g, dim3(kMgThreads), up, st, lv[l], lv[l + 1], omega, (double*)nullptr);
+        if (rtu)
+            launch_pdl(M.rz ? rt_up_kernel<T, true, false>(post) : rt_up_kernel<T, false, false>(post),
+                       tiles(l, rt_up_core(post, false)), bu, 0, st, lv[l], lv[l + 1], omega, (double*)nullptr,
+                       ResArgs{});
+        else
+            launch_pdl(M.rz ? up_kernel<T, true>(post) : up_kernel<T, false>(post), tiles(l, kMgTile), bu, up, st,
+                       lv[l], lv[l + 1], omega, (double*)nullptr);
         ++count;
     }
     if (Ltile >= 1) {
@@ -2388,11 +2427,12 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
         R.max_cycles = max_cycles;
         R.cond = cond;
         R.use_cond = use_cond;
-        const UpResKernel<T> kres =
-            M.rz ? up_res_kernel<T, true>(M.o.post_sweeps) : up_res_kernel<T, false>(M.o.post_sweeps);
-        const dim3 g(div_up(lv[0].nx, kMgTile), div_up(lv[0].ny, kMgTile));
-        launch_pdl(kres, g, dim3(kMgThreads), up_smem<T>(M.o.post_sweeps, M.rz, true), st, lv[0], lv[1], omega, phi,
-                   R);
+        if (rtu)
+            launch_pdl(M.rz ? rt_up_kernel<T, true, true>(post) : rt_up_kernel<T, false, true>(post),
+                       tiles(0, rt_up_core(post, true)), bu, 0, st, lv[0], lv[1], omega, phi, R);
+        else
+            launch_pdl(M.rz ? up_res_kernel<T, true>(post) : up_res_kernel<T, false>(post), tiles(0, kMgTile), bu,
+                       up_smem<T>(post, M.rz, true), st, lv[0], lv[1], omega, phi, R);
     } else {
         launch_r0(M, lv, phi, f, tol, max_cycles, 0, cond, use_cond, st);
     }
