@@ -2,15 +2,16 @@
 // multigrid.cu): the down and up phases of one level, and of two levels in one
 // launch, for up to kRtMaxSweeps red-black sweeps.
 //
-// A block of 8 warps works a 64 x 64 region of a level held in registers: warp
-// w has rows 8w .. 8w+7, lane l the columns 2l and 2l+1 of each.  Region
-// origins are even in both directions, so a node's colour follows from its row
-// and column index at compile time, every lane updates one node per row in
-// every half-sweep, and a half-sweep costs one warp shuffle (the neighbour in
-// the next lane) and about eight arithmetic instructions per update.  Rows on
-// either side of a warp's eight travel through shared memory, two values per
-// lane and one barrier per half-sweep.  The Dirichlet mask comes as bit columns
-// (LevelDev::fb), two words per lane and column.
+// A block of 8, 12 or 16 warps works a region of a level held in registers, 64
+// columns by 4 rows per warp: warp w has rows 4w .. 4w+3, lane l the columns 2l
+// and 2l+1 of each.  Region origins are even in both directions, so a node's
+// colour follows from its row and column index at compile time, every lane
+// updates one node per row in every half-sweep, and a half-sweep costs one warp
+// shuffle (the neighbour in the next lane) and about eight arithmetic
+// instructions per update.  Rows on either side of a warp's four travel through
+// shared memory, two values per lane and one barrier per half-sweep.  The
+// Dirichlet mask comes as bit columns (LevelDev::fb), two words per lane and
+// column.
 //
 // What bounds these phases is instruction issue at large grids and the chain
 // load - sweeps - store at small ones; shared-memory tiles of 32 x 32 (down_tile,
@@ -20,11 +21,12 @@
 
 namespace pic {
 
-constexpr int kRtWarps = 8;
-constexpr int kRtRows = 8;
-constexpr int kRtThreads = 32 * kRtWarps;
-constexpr int kRtSide = 64;  // region side, = kRtWarps * kRtRows = 2 * 32
+constexpr int kRtRows = 4;       // rows per warp
+constexpr int kRtMaxWarps = 16;
+constexpr int kRtMaxThreads = 32 * kRtMaxWarps;
+constexpr int kRtCols = 64;      // region columns, = 2 * 32
 constexpr int kRtMaxSweeps = 3;
+constexpr unsigned kRtRowMask = (1u << kRtRows) - 1u;
 
 // How far a phase of S sweeps reaches into the region, from its border (depth
 // 0).  A half-sweep is right one node deeper than what it reads; the first
@@ -32,33 +34,42 @@ constexpr int kRtMaxSweeps = 3;
 //   down   e at depth 2S - 1, the residual at 2S, its restriction at 2S + 1
 //   up     e at depth 2S; with the FP64 residual, e one node around the core
 // Core and left halo are even (two levels: multiples of four), so that every
-// origin keeps its parity.
+// origin keeps its parity.  core(n): the core of n region rows or columns.
 template <int S>
 struct RtDown {
-    static constexpr int HL = 2 * S + 2, CORE = kRtSide - HL - 2 * S;
+    static constexpr int HL = 2 * S + 2;
+    static constexpr __host__ __device__ int core(int n) { return n - HL - 2 * S; }
 };
 template <int S, bool RES>
 struct RtUp {
-    static constexpr int HL = RES ? 2 * S + 2 : 2 * S, CORE = RES ? kRtSide - 2 * HL : kRtSide - 4 * S;
+    static constexpr int HL = RES ? 2 * S + 2 : 2 * S;
+    static constexpr __host__ __device__ int core(int n) { return n - 2 * HL; }
 };
-// Two levels, F (the region) and C (32 x 32, one node per lane and row, four
-// rows per warp).
+// Two levels, F (the region) and C (half as many columns and rows, one node
+// per lane and row).
 //   down2  C's right-hand side is right on C nodes [ceil((2S+1)/2),
-//          floor((62-2S)/2)], its restriction 2S + 1 nodes inside that
-//   up2    C is right on [2S, 30 - 2S] (the last lane's prolongation is not
-//          formed), F's prolongation on [4S, 60 - 4S], F on [6S, 60 - 6S]
+//          floor((n-2-2S)/2)], its restriction 2S + 1 nodes inside that
+//   up2    C is right on [2S, n/2 - 2 - 2S] (the last lane's prolongation is
+//          not formed), F's prolongation on [4S, n - 4 - 4S], F on
+//          [6S, n - 4 - 6S]
 template <int S>
 struct RtDown2 {
-    static constexpr int LO = (2 * S + 2) / 2, HI = (62 - 2 * S) / 2;
-    static constexpr int C0 = (LO + 2 * S + 1 + 1) / 2 * 2, C1 = (HI - 2 * S - 1) / 2 * 2;  // first and last C2 centre
-    static constexpr int HL = 2 * C0, CORE = 2 * (C1 + 2 - C0);
+    static constexpr int C0 = (S + 1 + 2 * S + 1 + 1) / 2 * 2, HL = 2 * C0;  // C0: the first C2 centre
+    static constexpr __host__ __device__ int core(int n) {
+        const int c1 = ((n - 2 - 2 * S) / 2 - 2 * S - 1) / 2 * 2;  // the last one
+        return 2 * (c1 + 2 - C0);
+    }
 };
 template <int S>
 struct RtUp2 {
-    static constexpr int HL = (6 * S + 3) / 4 * 4, CORE = (60 - 6 * S - HL + 1) / 4 * 4;
+    static constexpr int HL = (6 * S + 3) / 4 * 4;
+    static constexpr __host__ __device__ int core(int n) { return (n - 4 - 6 * S - HL + 1) / 4 * 4; }
 };
 
-// Column bits of 8 (N <= 32) rows from row j of column i: bit r is 1 when node
+__device__ __forceinline__ int rt_warps() { return int(blockDim.x) >> 5; }
+__device__ __forceinline__ int rt_side() { return kRtRows * rt_warps(); }  // region rows
+
+// Column bits of up to 32 rows from row j of column i: bit r is 1 when node
 // (i, j + r) is free.
 __device__ __forceinline__ unsigned rt_free_bits(const uint32_t* __restrict__ fb, int nx, int nwords, int i, int j,
                                                  unsigned mask) {
@@ -111,11 +122,11 @@ struct RtCoef {
     }
 };
 
-// One region of F: 8 rows x 2 columns per lane, and the rows on either side.
+// One region of F: 4 rows x 2 columns per lane, and the rows on either side.
 template <class T>
 struct RtTile {
     T e[kRtRows][2], g[kRtRows][2];
-    T up[2], dn[2];  // row -1 (the warp above) and row 8, per column
+    T up[2], dn[2];  // row -1 (the warp above) and row 4, per column
     unsigned fr[2];  // free bits of the rows, per column
 };
 
@@ -123,20 +134,20 @@ struct RtTile {
 // only after the barrier between its readers and the next-but-one exchange.
 template <class T>
 struct RtShared {
-    T x[2][kRtWarps][2][32];
+    T x[2][kRtMaxWarps][2][32];
 };
 
-// Publishes, of the nodes of one colour, row 0 (its column COLOR & 1) and row
-// 7 (its other column), and reads the neighbouring warps' into up and dn.
+// Publishes, of the nodes of one colour, row 0 (its column COLOR & 1) and the
+// last row (its other column), and reads the neighbouring warps' into up and dn.
 template <class T, int COLOR>
 __device__ __forceinline__ void rt_exchange(RtTile<T>& t, RtShared<T>& s, int& buf) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    constexpr int c0 = COLOR & 1, c7 = (kRtRows - 1 + COLOR) & 1;
+    constexpr int c0 = COLOR & 1, c1 = (kRtRows - 1 + COLOR) & 1;
     s.x[buf][w][0][l] = t.e[0][c0];
-    s.x[buf][w][1][l] = t.e[kRtRows - 1][c7];
+    s.x[buf][w][1][l] = t.e[kRtRows - 1][c1];
     __syncthreads();
-    if (w > 0) t.up[c7] = s.x[buf][w - 1][1][l];
-    if (w < kRtWarps - 1) t.dn[c0] = s.x[buf][w + 1][0][l];
+    if (w > 0) t.up[c1] = s.x[buf][w - 1][1][l];
+    if (w < rt_warps() - 1) t.dn[c0] = s.x[buf][w + 1][0][l];
     buf ^= 1;
 }
 
@@ -216,17 +227,17 @@ __device__ __forceinline__ void rt_residual_h(const RtTile<T>& t, const RtCoef<T
     }
 }
 
-// Full weighting of the four coarse rows of this warp (the fine rows 0, 2, 4,
-// 6) from the horizontal weights; J0: the coarse row of fine row 0.
+// Full weighting of the coarse rows of this warp (the fine rows 0 and 2) from
+// the horizontal weights; J0: the coarse row of fine row 0.
 template <class T, bool CYL>
-__device__ __forceinline__ void rt_restrict(const T (&h)[kRtRows], RtShared<T>& sh, int& buf, int J0, T (&out)[4]) {
+__device__ __forceinline__ void rt_restrict(const T (&h)[kRtRows], RtShared<T>& sh, int& buf, int J0, T (&out)[kRtRows / 2]) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     sh.x[buf][w][1][l] = h[kRtRows - 1];
     __syncthreads();
     const T above = w > 0 ? sh.x[buf][w - 1][1][l] : T(0);
     buf ^= 1;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < kRtRows / 2; ++q) {
         const T s = q > 0 ? h[2 * q - 1] : above;
         T v = T(0.5) * h[2 * q] + T(0.25) * (s + h[2 * q + 1]);
         // r-z: divided by the stencil's weighted volume (2J; 5/16 on the axis)
@@ -240,34 +251,36 @@ __device__ __forceinline__ void rt_restrict(const T (&h)[kRtRows], RtShared<T>& 
 template <class T>
 __device__ __forceinline__ void rt_load_bits(const LevelDev<T>& L, int i0, int j0, RtTile<T>& t) {
     const int nw = (L.ny + 31) >> 5;
-    t.fr[0] = rt_free_bits(L.fb, L.nx, nw, i0, j0, 0xffu);
-    t.fr[1] = rt_free_bits(L.fb, L.nx, nw, i0 + 1, j0, 0xffu);
+    t.fr[0] = rt_free_bits(L.fb, L.nx, nw, i0, j0, kRtRowMask);
+    t.fr[1] = rt_free_bits(L.fb, L.nx, nw, i0 + 1, j0, kRtRowMask);
 }
 
+// The region's nodes of a field; nodes outside the grid take the value of the
+// nearest one inside (they are never free, and what a Dirichlet node holds is
+// not used), so that no load carries a bound test.
 template <class T, class G>
-__device__ __forceinline__ void rt_load_rows(const G* __restrict__ src, int nx, int ny, int i0, int j0,
-                                             T (&v)[kRtRows][2]) {
-    const bool c0 = i0 >= 0 && i0 < nx, c1 = i0 + 1 >= 0 && i0 + 1 < nx;
-    const G* p = src + long(j0) * nx + i0;
+__device__ __forceinline__ void rt_load_rows(const G* src, int nx, int ny, int i0, int j0, T (&v)[kRtRows][2]) {
+    const int c0 = min(max(i0, 0), nx - 1), c1 = min(max(i0 + 1, 0), nx - 1);
 #pragma unroll
     for (int r = 0; r < kRtRows; ++r) {
-        const bool in = j0 + r >= 0 && j0 + r < ny;
-        v[r][0] = (in && c0) ? T(p[long(r) * nx]) : T(0);
-        v[r][1] = (in && c1) ? T(p[long(r) * nx + 1]) : T(0);
+        const G* p = src + long(min(max(j0 + r, 0), ny - 1)) * nx;
+        v[r][0] = T(p[c0]);
+        v[r][1] = T(p[c1]);
     }
 }
 
 // Stores the core's nodes of a field of the region.
-template <class T, int HL, int CORE>
-__device__ __forceinline__ void rt_store_core(T* __restrict__ dst, const T (&v)[kRtRows][2], int nx, int ny, int i0,
-                                              int j0) {
+// (cx, cy: the core's columns and rows; HL: its left halo)
+template <class T, int HL>
+__device__ __forceinline__ void rt_store_core(T* dst, const T (&v)[kRtRows][2], int nx, int ny, int i0, int j0, int cx,
+                                              int cy) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (2 * l < HL || 2 * l >= HL + CORE) return;
+    if (2 * l < HL || 2 * l >= HL + cx) return;
     T* p = dst + long(j0) * nx + i0;
 #pragma unroll
     for (int r = 0; r < kRtRows; ++r) {
         const int lr = w * kRtRows + r;
-        if (lr < HL || lr >= HL + CORE || j0 + r >= ny) continue;
+        if (lr < HL || lr >= HL + cy || j0 + r >= ny) continue;
         if (i0 < nx) p[long(r) * nx] = v[r][0];
         if (i0 + 1 < nx) p[long(r) * nx + 1] = v[r][1];
     }
@@ -277,18 +290,19 @@ __device__ __forceinline__ void rt_store_core(T* __restrict__ dst, const T (&v)[
 
 // The down phase (see k_mg_down): smooth from zero, restrict the residual.
 template <class T, int S, bool CYL>
-__global__ void __launch_bounds__(kRtThreads) k_rt_down(LevelDev<T> F, LevelDev<T> C, T omega,
-                                                        const double* __restrict__ g64) {
-    using G = RtDown<S>;
+__global__ void __launch_bounds__(kRtMaxThreads) k_rt_down(LevelDev<T> F, LevelDev<T> C, T omega,
+                                                           const double* __restrict__ g64) {
+    constexpr int HL = RtDown<S>::HL;
     __shared__ RtShared<T> sh;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const int i0 = int(blockIdx.x) * G::CORE - G::HL + 2 * l, j0 = int(blockIdx.y) * G::CORE - G::HL + kRtRows * w;
+    const int cx = RtDown<S>::core(kRtCols), cy = RtDown<S>::core(rt_side());
+    const int i0 = int(blockIdx.x) * cx - HL + 2 * l, j0 = int(blockIdx.y) * cy - HL + kRtRows * w;
     // the coarse column and rows this lane restricts to (i0, j0 are even)
     const int I = i0 >> 1, J0 = j0 >> 1;
     RtTile<T> t;
     RtCoef<T, kRtRows, CYL> cf;
     rt_load_bits(F, i0, j0, t);
-    const unsigned cfr = rt_free_bits(C.fb, C.nx, (C.ny + 31) >> 5, I, J0, 0xfu);
+    const unsigned cfr = rt_free_bits(C.fb, C.nx, (C.ny + 31) >> 5, I, J0, (1u << (kRtRows / 2)) - 1u);
     cf.load(F, omega, j0);
     pdl_wait();
     pdl_trigger();
@@ -296,25 +310,24 @@ __global__ void __launch_bounds__(kRtThreads) k_rt_down(LevelDev<T> F, LevelDev<
     else rt_load_rows<T, T>(F.g, F.nx, F.ny, i0, j0, t.g);
     int buf = 0;
     rt_sweeps<T, S, CYL, true, true>(t, cf, sh, buf);
-    rt_store_core<T, G::HL, G::CORE>(F.e, t.e, F.nx, F.ny, i0, j0);
-    if (g64) rt_store_core<T, G::HL, G::CORE>(F.g, t.g, F.nx, F.ny, i0, j0);
-    T h[kRtRows], out[4];
+    rt_store_core<T, HL>(F.e, t.e, F.nx, F.ny, i0, j0, cx, cy);
+    if (g64) rt_store_core<T, HL>(F.g, t.g, F.nx, F.ny, i0, j0, cx, cy);
+    T h[kRtRows], out[kRtRows / 2];
     rt_residual_h<T, CYL>(t, cf, h);
     rt_restrict<T, CYL>(h, sh, buf, J0, out);
-    if (2 * l < G::HL || 2 * l >= G::HL + G::CORE || I >= C.nx) return;
+    if (2 * l < HL || 2 * l >= HL + cx || I >= C.nx) return;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < kRtRows / 2; ++q) {
         const int lr = w * kRtRows + 2 * q;
-        if (lr < G::HL || lr >= G::HL + G::CORE || J0 + q >= C.ny) continue;
+        if (lr < HL || lr >= HL + cy || J0 + q >= C.ny) continue;
         C.g[long(J0 + q) * C.nx + I] = ((cfr >> q) & 1u) ? out[q] : T(0);
     }
 }
 
-// Adds the bilinear prolongation of the coarse rows cv (coarse rows of fine
-// rows 0, 2, 4, 6 and 8) and their east neighbours ce on the free nodes; e is 0
-// elsewhere.
+// Adds the bilinear prolongation of the coarse rows cv (of the fine rows 0, 2
+// and 4) and their east neighbours ce on the free nodes; e is 0 elsewhere.
 template <class T>
-__device__ __forceinline__ void rt_prolong(RtTile<T>& t, const T (&cv)[5], const T (&ce)[5]) {
+__device__ __forceinline__ void rt_prolong(RtTile<T>& t, const T (&cv)[kRtRows / 2 + 1], const T (&ce)[kRtRows / 2 + 1]) {
 #pragma unroll
     for (int r = 0; r < kRtRows; ++r) {
         const int q = r >> 1;
@@ -332,12 +345,13 @@ __device__ __forceinline__ void rt_prolong(RtTile<T>& t, const T (&cv)[5], const
 // correction and smooth; RES (level 0): phi += e and the FP64 residual
 // r -= A e on the core, its norm and the loop decision.
 template <class T, int S, bool CYL, bool RES>
-__global__ void __launch_bounds__(kRtThreads) k_rt_up(LevelDev<T> F, LevelDev<T> C, T omega, double* __restrict__ phi,
-                                                      ResArgs R) {
+__global__ void __launch_bounds__(kRtMaxThreads) k_rt_up(LevelDev<T> F, LevelDev<T> C, T omega,
+                                                         double* __restrict__ phi, ResArgs R) {
     using G = RtUp<S, RES>;
     __shared__ RtShared<T> sh;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const int i0 = int(blockIdx.x) * G::CORE - G::HL + 2 * l, j0 = int(blockIdx.y) * G::CORE - G::HL + kRtRows * w;
+    const int cx = G::core(kRtCols), cy = G::core(rt_side());
+    const int i0 = int(blockIdx.x) * cx - G::HL + 2 * l, j0 = int(blockIdx.y) * cy - G::HL + kRtRows * w;
     RtTile<T> t;
     RtCoef<T, kRtRows, CYL> cf;
     rt_load_bits(F, i0, j0, t);
@@ -345,13 +359,13 @@ __global__ void __launch_bounds__(kRtThreads) k_rt_up(LevelDev<T> F, LevelDev<T>
     // everything but the coarse correction was written two or more launches back
     rt_load_rows<T, T>(F.e, F.nx, F.ny, i0, j0, t.e);
     rt_load_rows<T, T>(F.g, F.nx, F.ny, i0, j0, t.g);
-    const bool core_col = 2 * l >= G::HL && 2 * l < G::HL + G::CORE;
+    const bool core_col = 2 * l >= G::HL && 2 * l < G::HL + cx;
     double pv[RES ? kRtRows : 1][2], rv[RES ? kRtRows : 1][2];
     if constexpr (RES) {
 #pragma unroll
         for (int r = 0; r < kRtRows; ++r) {
             const int lr = w * kRtRows + r;
-            const bool in = core_col && lr >= G::HL && lr < G::HL + G::CORE && j0 + r < F.ny;
+            const bool in = core_col && lr >= G::HL && lr < G::HL + cy && j0 + r < F.ny;
             const long k = long(j0 + r) * F.nx + i0;
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
@@ -365,9 +379,9 @@ __global__ void __launch_bounds__(kRtThreads) k_rt_up(LevelDev<T> F, LevelDev<T>
     pdl_trigger();
     {
         const int I = i0 >> 1, J0 = j0 >> 1;
-        T cv[5], ce[5];
+        T cv[kRtRows / 2 + 1], ce[kRtRows / 2 + 1];
 #pragma unroll
-        for (int q = 0; q < 5; ++q) {
+        for (int q = 0; q < kRtRows / 2 + 1; ++q) {
             const int J = J0 + q;
             const bool in = J >= 0 && J < C.ny;
             const T* p = C.ec + long(J) * C.nx + I;
@@ -383,14 +397,14 @@ __global__ void __launch_bounds__(kRtThreads) k_rt_up(LevelDev<T> F, LevelDev<T>
     // the red rows' neighbours are black: they are exchanged before the first half-sweep
     rt_sweeps<T, S, CYL, false, RES>(t, cf, sh, buf);
     if constexpr (!RES) {
-        rt_store_core<T, G::HL, G::CORE>(F.ec, t.e, F.nx, F.ny, i0, j0);
+        rt_store_core<T, G::HL>(F.ec, t.e, F.nx, F.ny, i0, j0, cx, cy);
     } else {
         double r2 = 0.0;
 #pragma unroll
         for (int r = 0; r < kRtRows; ++r) {
             const int lr = w * kRtRows + r, j = j0 + r;
             const T ww = __shfl_up_sync(0xffffffffu, t.e[r][1], 1), ee = __shfl_down_sync(0xffffffffu, t.e[r][0], 1);
-            const bool in = core_col && lr >= G::HL && lr < G::HL + G::CORE && j < F.ny;
+            const bool in = core_col && lr >= G::HL && lr < G::HL + cy && j < F.ny;
             const long k = long(j) * F.nx + i0;
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
@@ -418,14 +432,17 @@ __global__ void __launch_bounds__(kRtThreads) k_rt_up(LevelDev<T> F, LevelDev<T>
 
 // ---- two levels in one launch ---------------------------------------------------------
 //
-// C's region: lane l has column C-origin + l, warp w the rows 4w .. 4w+3.  The
+// C's region: lane l has column C-origin + l, warp w the rows 2w and 2w+1.  The
 // origin is even, so a node's colour is (l + row) & 1: in a half-sweep a lane
-// updates one row of each pair of rows, the odd or the even one by its parity.
+// updates one of its two rows, the odd or the even one by its parity.
+
+constexpr int kRtCRows = kRtRows / 2;
+static_assert(kRtCRows == 2, "one pair of coarse rows per warp");
 
 template <class T>
 struct RtCTile {
-    T e[4], g[4];
-    T up, dn;  // rows -1 and 4
+    T e[2], g[2];
+    T up, dn;  // rows -1 and 2
     unsigned fr;
 };
 
@@ -433,43 +450,37 @@ template <class T>
 __device__ __forceinline__ void rt_c_exchange(RtCTile<T>& t, RtShared<T>& s, int& buf) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     s.x[buf][w][0][l] = t.e[0];
-    s.x[buf][w][1][l] = t.e[3];
+    s.x[buf][w][1][l] = t.e[1];
     __syncthreads();
     if (w > 0) t.up = s.x[buf][w - 1][1][l];
-    if (w < kRtWarps - 1) t.dn = s.x[buf][w + 1][0][l];
+    if (w < rt_warps() - 1) t.dn = s.x[buf][w + 1][0][l];
     buf ^= 1;
 }
 
 template <class T, bool CYL>
-__device__ __forceinline__ void rt_c_half_sweep(RtCTile<T>& t, const RtCoef<T, 4, CYL>& cf, int color) {
-    const bool odd = ((threadIdx.x + color) & 1) != 0;  // this lane's row of each pair
+__device__ __forceinline__ void rt_c_half_sweep(RtCTile<T>& t, const RtCoef<T, kRtCRows, CYL>& cf, int color) {
+    const bool odd = ((threadIdx.x + color) & 1) != 0;  // which of its rows this lane updates
     const T q = T(1) - cf.omega;
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-        const int a = 2 * p, b = a + 1;
-        // the neighbouring lanes update the pair's other row: they send this lane's
-        const T send = odd ? t.e[a] : t.e[b];
-        const T wv = __shfl_up_sync(0xffffffffu, send, 1), ev = __shfl_down_sync(0xffffffffu, send, 1);
-        const T below = a > 0 ? t.e[a - 1] : t.up, above = b < 3 ? t.e[b + 1] : t.dn;
-        const T s = odd ? t.e[a] : below, n = odd ? above : t.e[b];
-        const T old = odd ? t.e[b] : t.e[a], g = odd ? t.g[b] : t.g[a];
-        T v;
-        if constexpr (CYL) {
-            const RtRow<T> ka = cf.row(a), kb = cf.row(b);
-            const T kk = odd ? kb.k : ka.k, bs = odd ? kb.bs : ka.bs, bn = odd ? kb.bn : ka.bn;
-            v = q * old - kk * g + (kk * cf.cx) * (wv + ev) + (bs * s + bn * n);
-        } else {
-            v = q * old - cf.c.k * g + cf.c.a * (wv + ev) + cf.c.bs * (s + n);
-        }
-        const bool fa = (t.fr >> a) & 1u, fb = (t.fr >> b) & 1u;
-        if (!odd && fa) t.e[a] = v;
-        if (odd && fb) t.e[b] = v;
+    // the neighbouring lanes update the other row: they send this lane's
+    const T send = odd ? t.e[0] : t.e[1];
+    const T wv = __shfl_up_sync(0xffffffffu, send, 1), ev = __shfl_down_sync(0xffffffffu, send, 1);
+    const T s = odd ? t.e[0] : t.up, n = odd ? t.dn : t.e[1];
+    const T old = odd ? t.e[1] : t.e[0], g = odd ? t.g[1] : t.g[0];
+    T v;
+    if constexpr (CYL) {
+        const RtRow<T> ka = cf.row(0), kb = cf.row(1);
+        const T kk = odd ? kb.k : ka.k, bs = odd ? kb.bs : ka.bs, bn = odd ? kb.bn : ka.bn;
+        v = q * old - kk * g + (kk * cf.cx) * (wv + ev) + (bs * s + bn * n);
+    } else {
+        v = q * old - cf.c.k * g + cf.c.a * (wv + ev) + cf.c.bs * (s + n);
     }
+    if (!odd && (t.fr & 1u)) t.e[0] = v;
+    if (odd && (t.fr & 2u)) t.e[1] = v;
 }
 
 // S sweeps of C; every exchange carries both colours' boundary rows.
 template <class T, int S, bool CYL, bool FROM_ZERO>
-__device__ __forceinline__ void rt_c_sweeps(RtCTile<T>& t, const RtCoef<T, 4, CYL>& cf, RtShared<T>& sh, int& buf) {
+__device__ __forceinline__ void rt_c_sweeps(RtCTile<T>& t, const RtCoef<T, kRtCRows, CYL>& cf, RtShared<T>& sh, int& buf) {
     t.up = t.dn = T(0);
     if (!FROM_ZERO) rt_c_exchange(t, sh, buf);
 #pragma unroll
@@ -482,19 +493,20 @@ __device__ __forceinline__ void rt_c_sweeps(RtCTile<T>& t, const RtCoef<T, 4, CY
 }
 
 template <class T, int S, bool CYL>
-__global__ void __launch_bounds__(kRtThreads) k_rt_down2(LevelDev<T> F, LevelDev<T> C, LevelDev<T> C2, T omega) {
+__global__ void __launch_bounds__(kRtMaxThreads) k_rt_down2(LevelDev<T> F, LevelDev<T> C, LevelDev<T> C2, T omega) {
     using G = RtDown2<S>;
     __shared__ RtShared<T> sh;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const int i0 = int(blockIdx.x) * G::CORE - G::HL + 2 * l, j0 = int(blockIdx.y) * G::CORE - G::HL + kRtRows * w;
+    const int cx = G::core(kRtCols), cy = G::core(rt_side());
+    const int i0 = int(blockIdx.x) * cx - G::HL + 2 * l, j0 = int(blockIdx.y) * cy - G::HL + kRtRows * w;
     const int I = i0 >> 1, J0 = j0 >> 1;
     RtTile<T> t;
     RtCTile<T> ct;
     RtCoef<T, kRtRows, CYL> cf;
-    RtCoef<T, 4, CYL> cc;
+    RtCoef<T, kRtCRows, CYL> cc;
     rt_load_bits(F, i0, j0, t);
-    ct.fr = rt_free_bits(C.fb, C.nx, (C.ny + 31) >> 5, I, J0, 0xfu);
-    const unsigned c2fr = rt_free_bits(C2.fb, C2.nx, (C2.ny + 31) >> 5, I >> 1, J0 >> 1, 0x3u);
+    ct.fr = rt_free_bits(C.fb, C.nx, (C.ny + 31) >> 5, I, J0, (1u << (kRtRows / 2)) - 1u);
+    const unsigned c2fr = rt_free_bits(C2.fb, C2.nx, (C2.ny + 31) >> 5, I >> 1, J0 >> 1, 1u);
     cf.load(F, omega, j0);
     cc.load(C, omega, J0);
     pdl_wait();
@@ -502,33 +514,33 @@ __global__ void __launch_bounds__(kRtThreads) k_rt_down2(LevelDev<T> F, LevelDev
     rt_load_rows<T, T>(F.g, F.nx, F.ny, i0, j0, t.g);
     int buf = 0;
     rt_sweeps<T, S, CYL, true, true>(t, cf, sh, buf);
-    rt_store_core<T, G::HL, G::CORE>(F.e, t.e, F.nx, F.ny, i0, j0);
-    T h[kRtRows], out[4];
+    rt_store_core<T, G::HL>(F.e, t.e, F.nx, F.ny, i0, j0, cx, cy);
+    T h[kRtRows], out[kRtCRows];
     rt_residual_h<T, CYL>(t, cf, h);
     rt_restrict<T, CYL>(h, sh, buf, J0, out);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < kRtCRows; ++q) {
         ct.g[q] = ((ct.fr >> q) & 1u) ? out[q] : T(0);
         ct.e[q] = T(0);
     }
     rt_c_sweeps<T, S, CYL, true>(ct, cc, sh, buf);
     // C's core: its e and g for the up phase
-    const bool ccol = 2 * l >= G::HL && 2 * l < G::HL + G::CORE && I < C.nx;
+    const bool ccol = 2 * l >= G::HL && 2 * l < G::HL + cx && I < C.nx;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < kRtCRows; ++q) {
         const int lr = w * kRtRows + 2 * q;
-        if (!ccol || lr < G::HL || lr >= G::HL + G::CORE || J0 + q >= C.ny) continue;
+        if (!ccol || lr < G::HL || lr >= G::HL + cy || J0 + q >= C.ny) continue;
         const long K = long(J0 + q) * C.nx + I;
         C.e[K] = ct.e[q];
         C.g[K] = ct.g[q];
     }
     // C's residual, weighted along the row at the even columns (even lanes)
-    T hc[4];
+    T hc[kRtCRows];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < kRtCRows; ++q) {
         const T e = ct.e[q];
         const T wv = __shfl_up_sync(0xffffffffu, e, 1), ev = __shfl_down_sync(0xffffffffu, e, 1);
-        const T s = q > 0 ? ct.e[q - 1] : ct.up, n = q < 3 ? ct.e[q + 1] : ct.dn;
+        const T s = q > 0 ? ct.e[q - 1] : ct.up, n = q < kRtCRows - 1 ? ct.e[q + 1] : ct.dn;
         T v;
         if constexpr (CYL) {
             const T lap = cc.cx * (wv + ev - T(2) * e) + cc.rz[q][0] * (n - e) + cc.rz[q][1] * (s - e);
@@ -540,44 +552,41 @@ __global__ void __launch_bounds__(kRtThreads) k_rt_down2(LevelDev<T> F, LevelDev
         const T rw = __shfl_up_sync(0xffffffffu, r, 1), re = __shfl_down_sync(0xffffffffu, r, 1);
         hc[q] = T(0.5) * r + T(0.25) * (rw + re);
     }
-    sh.x[buf][w][1][l] = hc[3];
+    sh.x[buf][w][1][l] = hc[1];
     __syncthreads();
     const T above = w > 0 ? sh.x[buf][w - 1][1][l] : T(0);
-    const int I2 = I >> 1, J2 = J0 >> 1;
-    if ((l & 1) || !ccol || I2 >= C2.nx) return;
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-        const int lr = w * kRtRows + 4 * q, J = J2 + q;
-        if (lr < G::HL || lr >= G::HL + G::CORE || J >= C2.ny) continue;
-        T v = T(0.5) * hc[2 * q] + T(0.25) * ((q > 0 ? hc[1] : above) + hc[2 * q + 1]);
-        if constexpr (CYL) v *= J == 0 ? T(3.2) : T(0.5) / T(J);
-        C2.g[long(J) * C2.nx + I2] = ((c2fr >> q) & 1u) ? v : T(0);
-    }
+    buf ^= 1;
+    // one C2 row per warp, on the even lanes
+    const int I2 = I >> 1, J2 = J0 >> 1, lr = w * kRtRows;
+    if ((l & 1) || !ccol || I2 >= C2.nx || lr < G::HL || lr >= G::HL + cy || J2 >= C2.ny) return;
+    T v = T(0.5) * hc[0] + T(0.25) * (above + hc[1]);
+    if constexpr (CYL) v *= J2 == 0 ? T(3.2) : T(0.5) / T(J2);
+    C2.g[long(J2) * C2.nx + I2] = (c2fr & 1u) ? v : T(0);
 }
 
 template <class T, int S, bool CYL>
-__global__ void __launch_bounds__(kRtThreads) k_rt_up2(LevelDev<T> F, LevelDev<T> C, LevelDev<T> C2, T omega) {
+__global__ void __launch_bounds__(kRtMaxThreads) k_rt_up2(LevelDev<T> F, LevelDev<T> C, LevelDev<T> C2, T omega) {
     using G = RtUp2<S>;
     __shared__ RtShared<T> sh;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const int i0 = int(blockIdx.x) * G::CORE - G::HL + 2 * l, j0 = int(blockIdx.y) * G::CORE - G::HL + kRtRows * w;
+    const int cx = G::core(kRtCols), cy = G::core(rt_side());
+    const int i0 = int(blockIdx.x) * cx - G::HL + 2 * l, j0 = int(blockIdx.y) * cy - G::HL + kRtRows * w;
     const int I = i0 >> 1, J0 = j0 >> 1;
     RtTile<T> t;
     RtCTile<T> ct;
     RtCoef<T, kRtRows, CYL> cf;
-    RtCoef<T, 4, CYL> cc;
+    RtCoef<T, kRtCRows, CYL> cc;
     rt_load_bits(F, i0, j0, t);
-    ct.fr = rt_free_bits(C.fb, C.nx, (C.ny + 31) >> 5, I, J0, 0xfu);
+    ct.fr = rt_free_bits(C.fb, C.nx, (C.ny + 31) >> 5, I, J0, (1u << (kRtRows / 2)) - 1u);
     cf.load(F, omega, j0);
     cc.load(C, omega, J0);
     rt_load_rows<T, T>(F.e, F.nx, F.ny, i0, j0, t.e);
     rt_load_rows<T, T>(F.g, F.nx, F.ny, i0, j0, t.g);
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const bool in = J0 + q >= 0 && J0 + q < C.ny && I >= 0 && I < C.nx;
-        const long K = long(J0 + q) * C.nx + I;
-        ct.e[q] = in ? C.e[K] : T(0);
-        ct.g[q] = in ? C.g[K] : T(0);
+    for (int q = 0; q < kRtCRows; ++q) {
+        const long K = long(min(max(J0 + q, 0), C.ny - 1)) * C.nx + min(max(I, 0), C.nx - 1);
+        ct.e[q] = C.e[K];
+        ct.g[q] = C.g[K];
     }
     pdl_wait();
     pdl_trigger();
@@ -585,9 +594,9 @@ __global__ void __launch_bounds__(kRtThreads) k_rt_up2(LevelDev<T> F, LevelDev<T
         // C2's correction prolonged onto C: an odd column takes the mean of
         // its own C2 column and the next lane's
         const int I2 = I >> 1, J2 = J0 >> 1;
-        T v2[3];
+        T v2[2];
 #pragma unroll
-        for (int q = 0; q < 3; ++q) {
+        for (int q = 0; q < 2; ++q) {
             const int J = J2 + q;
             const bool in = J >= 0 && J < C2.ny && I2 >= 0 && I2 < C2.nx;
             const T v = in ? C2.ec[long(J) * C2.nx + I2] : T(0);
@@ -595,21 +604,21 @@ __global__ void __launch_bounds__(kRtThreads) k_rt_up2(LevelDev<T> F, LevelDev<T
             v2[q] = (l & 1) ? T(0.5) * (v + e) : v;
         }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const T v = (q & 1) ? T(0.5) * (v2[q >> 1] + v2[(q >> 1) + 1]) : v2[q >> 1];
+        for (int q = 0; q < kRtCRows; ++q) {
+            const T v = q ? T(0.5) * (v2[0] + v2[1]) : v2[0];
             ct.e[q] = ((ct.fr >> q) & 1u) ? ct.e[q] + v : T(0);
         }
     }
     int buf = 0;
     rt_c_sweeps<T, S, CYL, false>(ct, cc, sh, buf);
     {
-        T cv[5] = {ct.e[0], ct.e[1], ct.e[2], ct.e[3], ct.dn}, ce[5];
+        T cv[kRtCRows + 1] = {ct.e[0], ct.e[1], ct.dn}, ce[kRtCRows + 1];
 #pragma unroll
-        for (int q = 0; q < 5; ++q) ce[q] = __shfl_down_sync(0xffffffffu, cv[q], 1);
+        for (int q = 0; q < kRtCRows + 1; ++q) ce[q] = __shfl_down_sync(0xffffffffu, cv[q], 1);
         rt_prolong(t, cv, ce);
     }
     rt_sweeps<T, S, CYL, false, false>(t, cf, sh, buf);
-    rt_store_core<T, G::HL, G::CORE>(F.ec, t.e, F.nx, F.ny, i0, j0);
+    rt_store_core<T, G::HL>(F.ec, t.e, F.nx, F.ny, i0, j0, cx, cy);
 }
 
 // ---- launch tables ----------------------------------------------------------------------
@@ -645,13 +654,44 @@ static Fused2Kernel<T> rt_up2_kernel(int s) {
     return k[s];
 }
 
-// Core sides of the phases (tiles per direction = ceil(n / core)).
-static int rt_down_core(int s) { return s == 1 ? RtDown<1>::CORE : s == 2 ? RtDown<2>::CORE : RtDown<3>::CORE; }
-static int rt_up_core(int s, bool res) {
-    if (res) return s == 1 ? RtUp<1, true>::CORE : s == 2 ? RtUp<2, true>::CORE : RtUp<3, true>::CORE;
-    return s == 1 ? RtUp<1, false>::CORE : s == 2 ? RtUp<2, false>::CORE : RtUp<3, false>::CORE;
+// The launch shape of a phase on an nx x ny level: of 8, 12 and 16 warps per
+// block, the one that gives the busiest SM the fewest warps (a region row costs
+// the same in every shape, but the halo is shared by more rows in the taller
+// ones: small levels spread over more SMs, large ones take 16).
+struct RtShape {
+    dim3 grid;
+    int threads;
+};
+template <class Core>
+static RtShape rt_shape(int nx, int ny, Core core) {
+    RtShape best{};
+    long cost = 0;
+    for (int w : {16, 12, 8}) {
+        const int cy = core(kRtRows * w);
+        if (cy < 4) continue;
+        const dim3 g(div_up(nx, core(kRtCols)), div_up(ny, cy));
+        const long c = long(div_up(long(g.x) * g.y, num_sms())) * w;
+        if (!best.threads || c < cost) {
+            best = RtShape{g, 32 * w};
+            cost = c;
+        }
+    }
+    return best;
 }
-static int rt_down2_core(int s) { return s == 1 ? RtDown2<1>::CORE : s == 2 ? RtDown2<2>::CORE : RtDown2<3>::CORE; }
-static int rt_up2_core(int s) { return s == 1 ? RtUp2<1>::CORE : s == 2 ? RtUp2<2>::CORE : RtUp2<3>::CORE; }
+static RtShape rt_down_shape(int s, int nx, int ny) {
+    return rt_shape(nx, ny, [=](int n) { return s == 1 ? RtDown<1>::core(n) : s == 2 ? RtDown<2>::core(n) : RtDown<3>::core(n); });
+}
+static RtShape rt_up_shape(int s, int nx, int ny, bool res) {
+    return rt_shape(nx, ny, [=](int n) {
+        if (res) return s == 1 ? RtUp<1, true>::core(n) : s == 2 ? RtUp<2, true>::core(n) : RtUp<3, true>::core(n);
+        return s == 1 ? RtUp<1, false>::core(n) : s == 2 ? RtUp<2, false>::core(n) : RtUp<3, false>::core(n);
+    });
+}
+static RtShape rt_down2_shape(int s, int nx, int ny) {
+    return rt_shape(nx, ny, [=](int n) { return s == 1 ? RtDown2<1>::core(n) : s == 2 ? RtDown2<2>::core(n) : RtDown2<3>::core(n); });
+}
+static RtShape rt_up2_shape(int s, int nx, int ny) {
+    return rt_shape(nx, ny, [=](int n) { return s == 1 ? RtUp2<1>::core(n) : s == 2 ? RtUp2<2>::core(n) : RtUp2<3>::core(n); });
+}
 
 }  // namespace pic

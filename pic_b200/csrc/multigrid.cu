@@ -37,6 +37,7 @@
 #include <cooperative_groups.h>
 #include <cuda/atomic>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <type_traits>
@@ -838,12 +839,6 @@ static Fused2Kernel<T> up2_kernel(int s) {
     return k[s];
 }
 
-}  // namespace pic
-
-#include "mg_regtile.cuh"
-
-namespace pic {
-
 template <class T>
 static size_t down2_smem(int s) {
     const size_t HC = 2 * s + 2, WC = kMgTile / 2 + 2 * HC, HF = 2 * HC + 2 + 2 * s, WF = kMgTile + 2 * HF;
@@ -1109,6 +1104,12 @@ __global__ void __launch_bounds__(kDirectRows * 32) k_mg_direct(DirectDesc<T> D)
     const double t = warp_sum(double(s));
     if (lane == 0 && out >= 0) D.e[out] = T(t);
 }
+
+}  // namespace pic
+
+#include "mg_regtile.cuh"
+
+namespace pic {
 
 // ---- FP64 residual, norms and the loop decision -----------------------------------
 
@@ -2286,7 +2287,7 @@ int mg_create(int nx, int ny, double dx, double dy, const uint8_t* h_mask, const
     // block partials of the residual norm: one pair per block of the level-0
     // tiling (k_mg_r0, k_mg_up_res) or of the persistent grid (k_mg_solve),
     // whichever is larger
-    const int nb = std::max(std::max(int(M.grd0.x * M.grd0.y), div_up(nx, kMgTile) * div_up(ny, kMgTile)),
+    const int nb = std::max(std::max(int(M.grd0.x * M.grd0.y), div_up(nx, 16) * div_up(ny, 16)),
                             M.solve_grid);
     if (cudaMalloc(&M.N.partial, sizeof(double) * 2 * nb) != cudaSuccess)
         return bail(fail(PIC_ERR_CUDA, "pic_mg_create: out of device memory"));
@@ -2350,31 +2351,33 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
     const int pre = M.o.pre_sweeps, post = M.o.post_sweeps;
     const bool rtd = pre <= kRtMaxSweeps, rtu = post <= kRtMaxSweeps;
     const size_t down = rtd ? 0 : down_smem<T>(pre, M.rz), up = rtu ? 0 : up_smem<T>(post, M.rz);
-    const dim3 bd(rtd ? kRtThreads : kMgThreads), bu(rtu ? kRtThreads : kMgThreads);
     const DownKernel<T> kdown = rtd ? (M.rz ? rt_down_kernel<T, true>(pre) : rt_down_kernel<T, false>(pre))
                                     : (M.rz ? down_kernel<T, true>(pre) : down_kernel<T, false>(pre));
-    auto tiles = [&](int l, int side) { return dim3(div_up(lv[l].nx, side), div_up(lv[l].ny, side)); };
+    auto tiles = [&](int l) {  // the shared-memory tiles' launch shape
+        return RtShape{dim3(div_up(lv[l].nx, kMgTile), div_up(lv[l].ny, kMgTile)), kMgThreads};
+    };
     count = 0;
     // levels Lc-2 and Lc-1 in one launch each way where that applies
     const bool f2 = M.fuse2 && !hyb;
     const int Lsingle = f2 ? Ltile - 2 : Ltile;
     for (int l = 0; l < Lsingle; ++l) {
-        const dim3 g = tiles(l, rtd ? rt_down_core(pre) : kMgTile);
+        const RtShape h = rtd ? rt_down_shape(pre, lv[l].nx, lv[l].ny) : tiles(l);
         // the finest down phase waits for its predecessor to finish before it
         // is placed: launched ahead, its CTAs would take the SMs its
         // predecessor leaves free first, several to an SM (measured 8.5 us
         // instead of 4.8 at 513^2)
-        if (l == 0) kdown<<<g, bd, down, st>>>(lv[0], lv[1], omega, (const double*)M.r64);
-        else launch_pdl(kdown, g, bd, down, st, lv[l], lv[l + 1], omega, (const double*)nullptr);
+        if (l == 0) kdown<<<h.grid, h.threads, down, st>>>(lv[0], lv[1], omega, (const double*)M.r64);
+        else launch_pdl(kdown, h.grid, dim3(h.threads), down, st, lv[l], lv[l + 1], omega, (const double*)nullptr);
         ++count;
     }
     if (f2) {
         const int l = Lsingle;
+        const RtShape h = rtd ? rt_down2_shape(pre, lv[l].nx, lv[l].ny) : tiles(l);
         if (rtd)
-            launch_pdl(M.rz ? rt_down2_kernel<T, true>(pre) : rt_down2_kernel<T, false>(pre),
-                       tiles(l, rt_down2_core(pre)), bd, 0, st, lv[l], lv[l + 1], lv[l + 2], omega);
+            launch_pdl(M.rz ? rt_down2_kernel<T, true>(pre) : rt_down2_kernel<T, false>(pre), h.grid, dim3(h.threads),
+                       0, st, lv[l], lv[l + 1], lv[l + 2], omega);
         else
-            launch_pdl(down2_kernel<T>(pre), tiles(l, kMgTile), bd, down2_smem<T>(pre), st, lv[l], lv[l + 1],
+            launch_pdl(down2_kernel<T>(pre), h.grid, dim3(h.threads), down2_smem<T>(pre), st, lv[l], lv[l + 1],
                        lv[l + 2], omega);
         ++count;
     }
@@ -2398,21 +2401,22 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
     }
     if (f2) {
         const int l = Lsingle;
+        const RtShape h = rtu ? rt_up2_shape(post, lv[l].nx, lv[l].ny) : tiles(l);
         if (rtu)
-            launch_pdl(M.rz ? rt_up2_kernel<T, true>(post) : rt_up2_kernel<T, false>(post), tiles(l, rt_up2_core(post)),
-                       bu, 0, st, lv[l], lv[l + 1], lv[l + 2], omega);
+            launch_pdl(M.rz ? rt_up2_kernel<T, true>(post) : rt_up2_kernel<T, false>(post), h.grid, dim3(h.threads), 0,
+                       st, lv[l], lv[l + 1], lv[l + 2], omega);
         else
-            launch_pdl(up2_kernel<T>(post), tiles(l, kMgTile), bu, up2_smem<T>(post), st, lv[l], lv[l + 1], lv[l + 2],
+            launch_pdl(up2_kernel<T>(post), h.grid, dim3(h.threads), up2_smem<T>(post), st, lv[l], lv[l + 1], lv[l + 2],
                        omega);
         ++count;
     }
     for (int l = Lsingle - 1; l >= 1; --l) {
+        const RtShape h = rtu ? rt_up_shape(post, lv[l].nx, lv[l].ny, false) : tiles(l);
         if (rtu)
-            launch_pdl(M.rz ? rt_up_kernel<T, true, false>(post) : rt_up_kernel<T, false, false>(post),
-                       tiles(l, rt_up_core(post, false)), bu, 0, st, lv[l], lv[l + 1], omega, (double*)nullptr,
-                       ResArgs{});
+            launch_pdl(M.rz ? rt_up_kernel<T, true, false>(post) : rt_up_kernel<T, false, false>(post), h.grid,
+                       dim3(h.threads), 0, st, lv[l], lv[l + 1], omega, (double*)nullptr, ResArgs{});
         else
-            launch_pdl(M.rz ? up_kernel<T, true>(post) : up_kernel<T, false>(post), tiles(l, kMgTile), bu, up, st,
+            launch_pdl(M.rz ? up_kernel<T, true>(post) : up_kernel<T, false>(post), h.grid, dim3(h.threads), up, st,
                        lv[l], lv[l + 1], omega, (double*)nullptr);
         ++count;
     }
@@ -2427,11 +2431,12 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
         R.max_cycles = max_cycles;
         R.cond = cond;
         R.use_cond = use_cond;
+        const RtShape h = rtu ? rt_up_shape(post, lv[0].nx, lv[0].ny, true) : tiles(0);
         if (rtu)
-            launch_pdl(M.rz ? rt_up_kernel<T, true, true>(post) : rt_up_kernel<T, false, true>(post),
-                       tiles(0, rt_up_core(post, true)), bu, 0, st, lv[0], lv[1], omega, phi, R);
+            launch_pdl(M.rz ? rt_up_kernel<T, true, true>(post) : rt_up_kernel<T, false, true>(post), h.grid,
+                       dim3(h.threads), 0, st, lv[0], lv[1], omega, phi, R);
         else
-            launch_pdl(M.rz ? up_res_kernel<T, true>(post) : up_res_kernel<T, false>(post), tiles(0, kMgTile), bu,
+            launch_pdl(M.rz ? up_res_kernel<T, true>(post) : up_res_kernel<T, false>(post), h.grid, dim3(h.threads),
                        up_smem<T>(post, M.rz, true), st, lv[0], lv[1], omega, phi, R);
     } else {
         launch_r0(M, lv, phi, f, tol, max_cycles, 0, cond, use_cond, st);
