@@ -288,30 +288,85 @@ __device__ __forceinline__ void rt_store_core(T* dst, const T (&v)[kRtRows][2], 
 
 // ---- one level -----------------------------------------------------------------------
 
-// The down phase (see k_mg_down): smooth from zero, restrict the residual.
-template <class T, int S, bool CYL>
-__global__ void __launch_bounds__(kRtMaxThreads) k_rt_down(LevelDev<T> F, LevelDev<T> C, T omega,
-                                                           const double* __restrict__ g64) {
-    constexpr int HL = RtDown<S>::HL;
-    __shared__ RtShared<T> sh;
+// The first residual of a solve, formed by the first cycle's down phase.
+struct RtInit {
+    const double *phi, *f, *rz0;
+    double* r64;
+    double cx, cy;
+};
+
+// Rows -1 and 4 of a warp's FP64 potential, both columns.
+struct RtShared64 {
+    double x[kRtMaxWarps][2][2][32];
+};
+
+// r = f - A phi on the region's free nodes (right from depth 1 on), 0
+// elsewhere, in the association of k_mg_r0; the core's r goes to r64 and its
+// squares, and those of f, to r2 and f2.
+template <class T, int HL, bool CYL>
+__device__ __forceinline__ void rt_first_residual(const RtInit& I, const LevelDev<T>& F, int i0, int j0, int cx,
+                                                  int cy, RtTile<T>& t, RtShared64& sh, double& r2, double& f2) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    const int cx = RtDown<S>::core(kRtCols), cy = RtDown<S>::core(rt_side());
-    const int i0 = int(blockIdx.x) * cx - HL + 2 * l, j0 = int(blockIdx.y) * cy - HL + kRtRows * w;
+    double p[kRtRows][2], fv[kRtRows][2], up[2] = {0.0, 0.0}, dn[2] = {0.0, 0.0};
+    rt_load_rows<double, double>(I.phi, F.nx, F.ny, i0, j0, p);
+    rt_load_rows<double, double>(I.f, F.nx, F.ny, i0, j0, fv);
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        sh.x[w][0][c][l] = p[0][c];
+        sh.x[w][1][c][l] = p[kRtRows - 1][c];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        if (w > 0) up[c] = sh.x[w - 1][1][c][l];
+        if (w < rt_warps() - 1) dn[c] = sh.x[w + 1][0][c][l];
+    }
+    const bool core_col = 2 * l >= HL && 2 * l < HL + cx;
+#pragma unroll
+    for (int r = 0; r < kRtRows; ++r) {
+        const int lr = w * kRtRows + r, j = j0 + r;
+        const double ww = __shfl_up_sync(0xffffffffu, p[r][1], 1), ee = __shfl_down_sync(0xffffffffu, p[r][0], 1);
+        const bool in = core_col && lr >= HL && lr < HL + cy && j < F.ny;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const double e = p[r][c];
+            const double wv = c ? p[r][0] : ww, ev = c ? ee : p[r][1];
+            const double s = r > 0 ? p[r - 1][c] : up[c], n = r < kRtRows - 1 ? p[r + 1][c] : dn[c];
+            const bool fr = (t.fr[c] >> r) & 1u;
+            double lap;
+            if constexpr (CYL) {
+                const bool jin = j >= 0 && j < F.ny;
+                const double wn = jin ? __ldg(I.rz0 + 4 * j) : 0.0, ws = jin ? __ldg(I.rz0 + 4 * j + 1) : 0.0;
+                lap = I.cx * ((wv - e) + (ev - e)) + wn * (n - e) + ws * (s - e);
+            } else {
+                lap = I.cx * ((wv - e) + (ev - e)) + I.cy * ((s - e) + (n - e));
+            }
+            const double res = fr ? fv[r][c] - lap : 0.0;
+            t.g[r][c] = T(res);
+            if (in && i0 + c < F.nx) {
+                I.r64[long(j) * F.nx + i0 + c] = res;
+                r2 += res * res;
+                if (fr) f2 += fv[r][c] * fv[r][c];
+            }
+        }
+    }
+}
+
+// What follows a down phase's right-hand side (in t.g): smooth from zero, store
+// the core's correction (and, on level 0, its right-hand side in the V-cycle's
+// precision), restrict the residual.  (cx, cy: the core's columns and rows.)
+template <class T, int S, bool CYL>
+__device__ __forceinline__ void rt_down_rest(const LevelDev<T>& F, const LevelDev<T>& C, RtTile<T>& t,
+                                             const RtCoef<T, kRtRows, CYL>& cf, RtShared<T>& sh, int i0, int j0, int cx,
+                                             int cy, bool store_g, unsigned cfr) {
+    constexpr int HL = RtDown<S>::HL;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     // the coarse column and rows this lane restricts to (i0, j0 are even)
     const int I = i0 >> 1, J0 = j0 >> 1;
-    RtTile<T> t;
-    RtCoef<T, kRtRows, CYL> cf;
-    rt_load_bits(F, i0, j0, t);
-    const unsigned cfr = rt_free_bits(C.fb, C.nx, (C.ny + 31) >> 5, I, J0, (1u << (kRtRows / 2)) - 1u);
-    cf.load(F, omega, j0);
-    pdl_wait();
-    pdl_trigger();
-    if (g64) rt_load_rows<T, double>(g64, F.nx, F.ny, i0, j0, t.g);
-    else rt_load_rows<T, T>(F.g, F.nx, F.ny, i0, j0, t.g);
     int buf = 0;
     rt_sweeps<T, S, CYL, true, true>(t, cf, sh, buf);
     rt_store_core<T, HL>(F.e, t.e, F.nx, F.ny, i0, j0, cx, cy);
-    if (g64) rt_store_core<T, HL>(F.g, t.g, F.nx, F.ny, i0, j0, cx, cy);
+    if (store_g) rt_store_core<T, HL>(F.g, t.g, F.nx, F.ny, i0, j0, cx, cy);
     T h[kRtRows], out[kRtRows / 2];
     rt_residual_h<T, CYL>(t, cf, h);
     rt_restrict<T, CYL>(h, sh, buf, J0, out);
@@ -321,6 +376,69 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_down(LevelDev<T> F, LevelD
         const int lr = w * kRtRows + 2 * q;
         if (lr < HL || lr >= HL + cy || J0 + q >= C.ny) continue;
         C.g[long(J0 + q) * C.nx + I] = ((cfr >> q) & 1u) ? out[q] : T(0);
+    }
+}
+
+// The down phase (see k_mg_down): smooth from zero, restrict the residual.
+template <class T, int S, bool CYL>
+__global__ void __launch_bounds__(kRtMaxThreads) k_rt_down(LevelDev<T> F, LevelDev<T> C, T omega,
+                                                           const double* __restrict__ g64, const int* stop) {
+    constexpr int HL = RtDown<S>::HL;
+    __shared__ RtShared<T> sh;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int cx = RtDown<S>::core(kRtCols), cy = RtDown<S>::core(rt_side());
+    const int i0 = int(blockIdx.x) * cx - HL + 2 * l, j0 = int(blockIdx.y) * cy - HL + kRtRows * w;
+    RtTile<T> t;
+    RtCoef<T, kRtRows, CYL> cf;
+    rt_load_bits(F, i0, j0, t);
+    const unsigned cfr = rt_free_bits(C.fb, C.nx, (C.ny + 31) >> 5, i0 >> 1, j0 >> 1, (1u << (kRtRows / 2)) - 1u);
+    cf.load(F, omega, j0);
+    pdl_wait();
+    pdl_trigger();
+    if (g64) rt_load_rows<T, double>(g64, F.nx, F.ny, i0, j0, t.g);
+    else rt_load_rows<T, T>(F.g, F.nx, F.ny, i0, j0, t.g);
+    if (stopped(stop)) return;
+    rt_down_rest<T, S, CYL>(F, C, t, cf, sh, i0, j0, cx, cy, g64 != nullptr, cfr);
+}
+
+// The finest down phase of a solve's first cycle: the right-hand side is the
+// first residual, formed here.  Its region is right from depth 1 on, so the
+// core is the residual up phase's.  decide: also the norms of the residual and
+// of f and the first loop decision; else the blocks' shares of ||f||^2, for the
+// decision after the first cycles (NormState::fpart).
+template <class T, int S, bool CYL>
+__global__ void __launch_bounds__(kRtMaxThreads) k_rt_init(LevelDev<T> F, LevelDev<T> C, T omega, RtInit I, NormState N,
+                                                           double tol2, int max_cycles, int decide,
+                                                           cudaGraphConditionalHandle cond, int use_cond) {
+    constexpr int HL = RtDown<S>::HL;
+    static_assert(HL == RtUp<S, true>::HL, "the first residual's tiles are the residual up phase's");
+    __shared__ RtShared<T> sh;
+    __shared__ RtShared64 sh64;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int cx = RtUp<S, true>::core(kRtCols), cy = RtUp<S, true>::core(rt_side());
+    const int i0 = int(blockIdx.x) * cx - HL + 2 * l, j0 = int(blockIdx.y) * cy - HL + kRtRows * w;
+    RtTile<T> t;
+    RtCoef<T, kRtRows, CYL> cf;
+    rt_load_bits(F, i0, j0, t);
+    const unsigned cfr = rt_free_bits(C.fb, C.nx, (C.ny + 31) >> 5, i0 >> 1, j0 >> 1, (1u << (kRtRows / 2)) - 1u);
+    cf.load(F, omega, j0);
+    pdl_wait();
+    pdl_trigger();
+    double r2 = 0.0, f2 = 0.0;
+    rt_first_residual<T, HL, CYL>(I, F, i0, j0, cx, cy, t, sh64, r2, f2);
+    rt_down_rest<T, S, CYL>(F, C, t, cf, sh, i0, j0, cx, cy, true, cfr);
+    if (decide) {
+        norm_reduce_decide(r2, f2, N, tol2, max_cycles, 1, cond, use_cond);
+        return;
+    }
+    __shared__ double ws[kRtMaxWarps];
+    f2 = warp_sum(f2);
+    if (l == 0) ws[w] = f2;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double s = 0.0;
+        for (int q = 0; q < rt_warps(); ++q) s += ws[q];
+        N.fpart[blockIdx.y * gridDim.x + blockIdx.x] = s;
     }
 }
 
@@ -346,7 +464,8 @@ __device__ __forceinline__ void rt_prolong(RtTile<T>& t, const T (&cv)[kRtRows /
 // r -= A e on the core, its norm and the loop decision.
 template <class T, int S, bool CYL, bool RES>
 __global__ void __launch_bounds__(kRtMaxThreads) k_rt_up(LevelDev<T> F, LevelDev<T> C, T omega,
-                                                         double* __restrict__ phi, ResArgs R) {
+                                                         double* __restrict__ phi, ResArgs R,
+                                                         const int* stop) {
     using G = RtUp<S, RES>;
     __shared__ RtShared<T> sh;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -391,6 +510,7 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_up(LevelDev<T> F, LevelDev
             const T y = __shfl_down_sync(0xffffffffu, cv[q], 1);
             ce[q] = l == 31 ? x : y;
         }
+        if (stopped(stop)) return;
         rt_prolong(t, cv, ce);
     }
     int buf = 0;
@@ -426,7 +546,8 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_up(LevelDev<T> F, LevelDev
                 r2 += rr * rr;
             }
         }
-        norm_reduce_decide(r2, 0.0, R.N, R.tol2, R.max_cycles, 0, R.cond, R.use_cond);
+        if (R.decide)
+            norm_reduce_decide(r2, 0.0, R.N, R.tol2, R.max_cycles, 0, R.cond, R.use_cond, R.inc, R.fblocks);
     }
 }
 
@@ -493,7 +614,8 @@ __device__ __forceinline__ void rt_c_sweeps(RtCTile<T>& t, const RtCoef<T, kRtCR
 }
 
 template <class T, int S, bool CYL>
-__global__ void __launch_bounds__(kRtMaxThreads) k_rt_down2(LevelDev<T> F, LevelDev<T> C, LevelDev<T> C2, T omega) {
+__global__ void __launch_bounds__(kRtMaxThreads) k_rt_down2(LevelDev<T> F, LevelDev<T> C, LevelDev<T> C2, T omega,
+                                                           const int* stop) {
     using G = RtDown2<S>;
     __shared__ RtShared<T> sh;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -512,6 +634,7 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_down2(LevelDev<T> F, Level
     pdl_wait();
     pdl_trigger();
     rt_load_rows<T, T>(F.g, F.nx, F.ny, i0, j0, t.g);
+    if (stopped(stop)) return;
     int buf = 0;
     rt_sweeps<T, S, CYL, true, true>(t, cf, sh, buf);
     rt_store_core<T, G::HL>(F.e, t.e, F.nx, F.ny, i0, j0, cx, cy);
@@ -565,7 +688,8 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_down2(LevelDev<T> F, Level
 }
 
 template <class T, int S, bool CYL>
-__global__ void __launch_bounds__(kRtMaxThreads) k_rt_up2(LevelDev<T> F, LevelDev<T> C, LevelDev<T> C2, T omega) {
+__global__ void __launch_bounds__(kRtMaxThreads) k_rt_up2(LevelDev<T> F, LevelDev<T> C, LevelDev<T> C2, T omega,
+                                                           const int* stop) {
     using G = RtUp2<S>;
     __shared__ RtShared<T> sh;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -609,6 +733,7 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_up2(LevelDev<T> F, LevelDe
             ct.e[q] = ((ct.fr >> q) & 1u) ? ct.e[q] + v : T(0);
         }
     }
+    if (stopped(stop)) return;
     int buf = 0;
     rt_c_sweeps<T, S, CYL, false>(ct, cc, sh, buf);
     {
@@ -624,12 +749,22 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_up2(LevelDev<T> F, LevelDe
 // ---- launch tables ----------------------------------------------------------------------
 
 template <class T>
-using RtUpKernel = void (*)(LevelDev<T>, LevelDev<T>, T, double*, ResArgs);
+using RtUpKernel = void (*)(LevelDev<T>, LevelDev<T>, T, double*, ResArgs, const int*);
+template <class T>
+using RtInitKernel = void (*)(LevelDev<T>, LevelDev<T>, T, RtInit, NormState, double, int, int,
+                              cudaGraphConditionalHandle, int);
 
 template <class T, bool CYL>
-static DownKernel<T> rt_down_kernel(int s) {
-    static const DownKernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_down<T, 1, CYL>, k_rt_down<T, 2, CYL>,
+static RtDownKernel<T> rt_down_kernel(int s) {
+    static const RtDownKernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_down<T, 1, CYL>, k_rt_down<T, 2, CYL>,
                                                       k_rt_down<T, 3, CYL>};
+    return k[s];
+}
+
+template <class T, bool CYL>
+static RtInitKernel<T> rt_init_kernel(int s) {
+    static const RtInitKernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_init<T, 1, CYL>, k_rt_init<T, 2, CYL>,
+                                                        k_rt_init<T, 3, CYL>};
     return k[s];
 }
 
@@ -641,15 +776,15 @@ static RtUpKernel<T> rt_up_kernel(int s) {
 }
 
 template <class T, bool CYL>
-static Fused2Kernel<T> rt_down2_kernel(int s) {
-    static const Fused2Kernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_down2<T, 1, CYL>, k_rt_down2<T, 2, CYL>,
+static RtFused2Kernel<T> rt_down2_kernel(int s) {
+    static const RtFused2Kernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_down2<T, 1, CYL>, k_rt_down2<T, 2, CYL>,
                                                         k_rt_down2<T, 3, CYL>};
     return k[s];
 }
 
 template <class T, bool CYL>
-static Fused2Kernel<T> rt_up2_kernel(int s) {
-    static const Fused2Kernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_up2<T, 1, CYL>, k_rt_up2<T, 2, CYL>,
+static RtFused2Kernel<T> rt_up2_kernel(int s) {
+    static const RtFused2Kernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_up2<T, 1, CYL>, k_rt_up2<T, 2, CYL>,
                                                         k_rt_up2<T, 3, CYL>};
     return k[s];
 }

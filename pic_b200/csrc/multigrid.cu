@@ -89,9 +89,11 @@ struct LevelDev {
 // blocks finished, and the solve's state.
 struct NormState {
     double* partial;   // [nblocks] r^2, then [nblocks] f^2
+    double* fpart;     // f^2 of the blocks of a first residual that took no decision
     unsigned* done;    // blocks finished
     double* norms;     // [||f||^2, ||r||^2]
     int* converged;
+    int* stop;         // converged or at the cycle limit: cycles launched ahead of the test do nothing
     int* cycles;       // V-cycles of the current solve
     long long* total;  // V-cycles since creation
 };
@@ -106,6 +108,9 @@ struct ResArgs {
     int max_cycles;
     cudaGraphConditionalHandle cond;
     int use_cond;
+    int decide;   // 0: no norm and no decision after this cycle (register tiles)
+    int inc;      // cycles since the last decision
+    int fblocks;  // the solve's first decision: blocks of ||f||^2 partials (NormState::fpart), else 0
 };
 
 // The levels as a launch mode uses them: up phases on the levels below
@@ -666,11 +671,13 @@ __global__ void __launch_bounds__(kMgThreads) k_mg_up2(LevelDev<T> F, LevelDev<T
 // Sums (a, b) over the grid: block partials into N.partial; the last block to
 // finish adds them in a fixed order (the same decision on every run) and
 // takes the loop decision: initial (first residual of a solve) records
-// ||f||^2 = b and zeroes the cycle count, else counts a V-cycle; converged
+// ||f||^2 = b and zeroes the cycle count, else counts `inc` V-cycles; converged
 // when ||r||^2 = a < tol2 ||f||^2; the WHILE node's condition (use_cond) is
-// to go on while neither converged nor at max_cycles.
+// to go on while neither converged nor at max_cycles.  fblocks: the solve's
+// first decision comes after its first cycles: ||f||^2 is the sum of so many
+// partials in N.fpart, and the count starts here.
 __device__ void norm_reduce_decide(double a, double b, const NormState& N, double tol2, int max_cycles, int initial,
-                                   cudaGraphConditionalHandle cond, int use_cond) {
+                                   cudaGraphConditionalHandle cond, int use_cond, int inc = 1, int fblocks = 0) {
     __shared__ double ws[2][32];
     __shared__ bool last;
     const int t = threadIdx.y * blockDim.x + threadIdx.x, nt = blockDim.x * blockDim.y, nw = nt >> 5;
@@ -711,8 +718,9 @@ __device__ void norm_reduce_decide(double a, double b, const NormState& N, doubl
     double sa = 0.0, sb = 0.0;
     for (int q = t; q < nb; q += nt) {
         sa += P[q];
-        sb += P[nb + q];
+        if (!fblocks) sb += P[nb + q];
     }
+    for (int q = t; q < fblocks; q += nt) sb += reinterpret_cast<const volatile double*>(N.fpart)[q];
     sa = warp_sum(sa);
     sb = warp_sum(sb);
     __syncthreads();
@@ -731,14 +739,20 @@ __device__ void norm_reduce_decide(double a, double b, const NormState& N, doubl
                 N.norms[0] = f2;
                 cyc = 0;
             } else {
-                cyc += 1;
-                *N.total = tot + 1;
+                if (fblocks) {
+                    ref0 = f2;
+                    N.norms[0] = f2;
+                    cyc = 0;
+                }
+                cyc += inc;
+                *N.total = tot + inc;
             }
             *N.cycles = cyc;
             N.norms[1] = r2;
             const int conv = r2 < tol2 * (ref0 > 0.0 ? ref0 : 1.0);
             *N.converged = conv;
             const int cont = !conv && cyc < max_cycles;
+            *N.stop = !cont;
             if (use_cond) cudaGraphSetConditional(cond, cont ? 1u : 0u);
             *N.done = 0u;
         }
@@ -754,6 +768,12 @@ __global__ void __launch_bounds__(kMgThreads) k_mg_up_res(LevelDev<T> F, LevelDe
     extern __shared__ __align__(16) unsigned char smem[];
     const double r2 = up_tile<T, S, CYL, true, true>(F, Cc, omega, phi, blockIdx.x, blockIdx.y, smem, &R);
     norm_reduce_decide(r2, 0.0, R.N, R.tol2, R.max_cycles, 0, R.cond, R.use_cond);
+}
+
+// A cycle launched ahead of the convergence test (`stop`: NormState::stop, null
+// for a cycle that always runs) does nothing once the solve has stopped.
+__device__ __forceinline__ bool stopped(const int* stop) {
+    return stop && *reinterpret_cast<const volatile int*>(stop);
 }
 
 // Runtime sweep counts (the persistent kernel) dispatched to the instances.
@@ -822,6 +842,10 @@ static UpResKernel<T> up_res_kernel(int s) {
 
 template <class T>
 using Fused2Kernel = void (*)(LevelDev<T>, LevelDev<T>, LevelDev<T>, T);
+template <class T>
+using RtDownKernel = void (*)(LevelDev<T>, LevelDev<T>, T, const double*, const int*);
+template <class T>
+using RtFused2Kernel = void (*)(LevelDev<T>, LevelDev<T>, LevelDev<T>, T, const int*);
 
 template <class T>
 static Fused2Kernel<T> down2_kernel(int s) {
@@ -1070,7 +1094,7 @@ struct DirectDesc {
 // MT: the precision of the inverse and of the products (double: the solve
 // in FP64 whatever the V-cycle's precision).
 template <class T, class MT>
-__global__ void __launch_bounds__(kDirectRows * 32) k_mg_direct(DirectDesc<T> D) {
+__global__ void __launch_bounds__(kDirectRows * 32) k_mg_direct(DirectDesc<T> D, const int* stop) {
     __shared__ MT gs[kDirectMaxFree];
     const int lane = threadIdx.x & 31, row = blockIdx.x * kDirectRows + int(threadIdx.x >> 5);
     const MT* __restrict__ ainv = static_cast<const MT*>(D.ainv);
@@ -1089,6 +1113,7 @@ __global__ void __launch_bounds__(kDirectRows * 32) k_mg_direct(DirectDesc<T> D)
     const int out = row < D.n ? __ldg(D.idx + row) : -1;
     pdl_wait();
     pdl_trigger();
+    if (stopped(stop)) return;
 #pragma unroll
     for (int u = 0; u < kDirectGather; ++u)
         if (gi[u] >= 0) gs[threadIdx.x + u * kDirectRows * 32] = MT(D.g[gi[u]]);
@@ -2292,6 +2317,9 @@ int mg_create(int nx, int ny, double dx, double dy, const uint8_t* h_mask, const
     if (cudaMalloc(&M.N.partial, sizeof(double) * 2 * nb) != cudaSuccess)
         return bail(fail(PIC_ERR_CUDA, "pic_mg_create: out of device memory"));
     M.allocs.push_back(M.N.partial);
+    if (cudaMalloc(&M.N.fpart, sizeof(double) * nb) != cudaSuccess)
+        return bail(fail(PIC_ERR_CUDA, "pic_mg_create: out of device memory"));
+    M.allocs.push_back(M.N.fpart);
     if (cudaMalloc(&M.r64, sizeof(double) * size_t(nx) * ny) != cudaSuccess)
         return bail(fail(PIC_ERR_CUDA, "pic_mg_create: out of device memory"));
     M.allocs.push_back(M.r64);
@@ -2305,6 +2333,7 @@ int mg_create(int nx, int ny, double dx, double dy, const uint8_t* h_mask, const
     M.N.done = reinterpret_cast<unsigned*>(small + 24);
     M.N.converged = reinterpret_cast<int*>(small + 28);
     M.N.cycles = reinterpret_cast<int*>(small + 32);
+    M.N.stop = reinterpret_cast<int*>(small + 36);
     M.bar = reinterpret_cast<GridBar*>(small + 40);
     M.error = reinterpret_cast<int*>(small + 48);
     if (cudaStreamCreateWithFlags(&M.side, cudaStreamNonBlocking) != cudaSuccess ||
@@ -2330,14 +2359,30 @@ static void launch_r0(MgImpl& M, const std::vector<LevelDev<T>>& lv, double* phi
                    tol * tol, max_cycles, initial, cond, use_cond, nul, M.r64);
 }
 
+// How a V-cycle sits in its solve.
+struct CycleOpts {
+    const int* stop = nullptr;  // the cycle does nothing once this flag is set (register tiles only)
+    bool decide = true;         // the cycle ends with the norm and the loop decision
+    int inc = 1;                // cycles since the last decision
+    int fblocks = 0;            // this is the solve's first decision, after a first residual of so many blocks
+    const RtInit* init = nullptr;  // the solve's first cycle: its finest down phase forms the first residual ...
+    bool init_decide = false;      // ... and takes the first decision
+};
+
+// Whether a cycle runs on register tiles throughout, with the direct solve.
+static bool rt_cycles(const MgImpl& M) {
+    return M.direct && !M.hybrid && M.o.pre_sweeps <= kRtMaxSweeps && M.o.post_sweeps <= kRtMaxSweeps;
+}
+
 // One V-cycle followed by the residual check, launched on stream st.  With
-// tile levels, the finest down phase reads the FP64 residual (r64, from
-// k_mg_r0 or the previous cycle) and the finest up phase updates it and takes
-// the loop decision (k_mg_up_res); a cycle of the coarse kernel alone ends
-// with k_mg_r0.
+// tile levels, the finest down phase reads the FP64 residual (r64, from the
+// first residual or the previous cycle) and the finest up phase updates it and
+// takes the loop decision; a cycle of the coarse kernel alone ends with
+// k_mg_r0.
 template <class T>
 static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi, const double* f, double tol,
-                        int max_cycles, cudaGraphConditionalHandle cond, int use_cond, cudaStream_t st, int& count) {
+                        int max_cycles, cudaGraphConditionalHandle cond, int use_cond, cudaStream_t st, int& count,
+                        const CycleOpts& O = CycleOpts{}) {
     // the hybrid cycle's coarse end starts at Lt (tiles above it); its
     // cluster kernel's bands write eu like the tile up phases, its CTA 0 the
     // levels from Lp
@@ -2351,8 +2396,6 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
     const int pre = M.o.pre_sweeps, post = M.o.post_sweeps;
     const bool rtd = pre <= kRtMaxSweeps, rtu = post <= kRtMaxSweeps;
     const size_t down = rtd ? 0 : down_smem<T>(pre, M.rz), up = rtu ? 0 : up_smem<T>(post, M.rz);
-    const DownKernel<T> kdown = rtd ? (M.rz ? rt_down_kernel<T, true>(pre) : rt_down_kernel<T, false>(pre))
-                                    : (M.rz ? down_kernel<T, true>(pre) : down_kernel<T, false>(pre));
     auto tiles = [&](int l) {  // the shared-memory tiles' launch shape
         return RtShape{dim3(div_up(lv[l].nx, kMgTile), div_up(lv[l].ny, kMgTile)), kMgThreads};
     };
@@ -2361,13 +2404,27 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
     const bool f2 = M.fuse2 && !hyb;
     const int Lsingle = f2 ? Ltile - 2 : Ltile;
     for (int l = 0; l < Lsingle; ++l) {
-        const RtShape h = rtd ? rt_down_shape(pre, lv[l].nx, lv[l].ny) : tiles(l);
-        // the finest down phase waits for its predecessor to finish before it
-        // is placed: launched ahead, its CTAs would take the SMs its
-        // predecessor leaves free first, several to an SM (measured 8.5 us
-        // instead of 4.8 at 513^2)
-        if (l == 0) kdown<<<h.grid, h.threads, down, st>>>(lv[0], lv[1], omega, (const double*)M.r64);
-        else launch_pdl(kdown, h.grid, dim3(h.threads), down, st, lv[l], lv[l + 1], omega, (const double*)nullptr);
+        const double* g64 = l == 0 ? M.r64 : nullptr;
+        if (l == 0 && O.init) {
+            const RtShape h = rt_up_shape(pre, lv[0].nx, lv[0].ny, true);
+            launch_pdl(M.rz ? rt_init_kernel<T, true>(pre) : rt_init_kernel<T, false>(pre), h.grid, dim3(h.threads), 0,
+                       st, lv[0], lv[1], omega, *O.init, M.N, tol * tol, max_cycles, int(O.init_decide), cond,
+                       int(use_cond && O.init_decide));
+        } else if (rtd) {
+            // the finest down phase waits for its predecessor to finish before
+            // it is placed: launched ahead, its blocks take the SMs the
+            // predecessor leaves free first, several to an SM (2049^2 solve
+            // 1009 us launched ahead, 942 us this way; 129^2 the same)
+            const RtDownKernel<T> kdown = M.rz ? rt_down_kernel<T, true>(pre) : rt_down_kernel<T, false>(pre);
+            const RtShape h = rt_down_shape(pre, lv[l].nx, lv[l].ny);
+            if (l == 0) kdown<<<h.grid, h.threads, 0, st>>>(lv[0], lv[1], omega, g64, O.stop);
+            else launch_pdl(kdown, h.grid, dim3(h.threads), 0, st, lv[l], lv[l + 1], omega, g64, O.stop);
+        } else {
+            const DownKernel<T> kdown = M.rz ? down_kernel<T, true>(pre) : down_kernel<T, false>(pre);
+            const RtShape h = tiles(l);
+            if (l == 0) kdown<<<h.grid, h.threads, down, st>>>(lv[0], lv[1], omega, g64);
+            else launch_pdl(kdown, h.grid, dim3(h.threads), down, st, lv[l], lv[l + 1], omega, g64);
+        }
         ++count;
     }
     if (f2) {
@@ -2375,7 +2432,7 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
         const RtShape h = rtd ? rt_down2_shape(pre, lv[l].nx, lv[l].ny) : tiles(l);
         if (rtd)
             launch_pdl(M.rz ? rt_down2_kernel<T, true>(pre) : rt_down2_kernel<T, false>(pre), h.grid, dim3(h.threads),
-                       0, st, lv[l], lv[l + 1], lv[l + 2], omega);
+                       0, st, lv[l], lv[l + 1], lv[l + 2], omega, O.stop);
         else
             launch_pdl(down2_kernel<T>(pre), h.grid, dim3(h.threads), down2_smem<T>(pre), st, lv[l], lv[l + 1],
                        lv[l + 2], omega);
@@ -2389,8 +2446,9 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
     }
     if (!hyb && M.direct) {
         const DirectDesc<T> D{M.dinv, M.didx, M.didx + M.dn, lv[M.Lc].g, lv[M.Lc].e, M.dn, M.dnz};
-        if (M.dinv64) launch_pdl(k_mg_direct<T, double>, dim3(div_up(M.dn, kDirectRows)), dim3(kDirectRows * 32), 0, st, D);
-        else launch_pdl(k_mg_direct<T, T>, dim3(div_up(M.dn, kDirectRows)), dim3(kDirectRows * 32), 0, st, D);
+        const dim3 g(div_up(M.dn, kDirectRows)), b(kDirectRows * 32);
+        if (M.dinv64) launch_pdl(k_mg_direct<T, double>, g, b, 0, st, D, O.stop);
+        else launch_pdl(k_mg_direct<T, T>, g, b, 0, st, D, O.stop);
         ++count;
     } else if (!hyb) {
         CoarseDesc<T> D{};
@@ -2404,7 +2462,7 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
         const RtShape h = rtu ? rt_up2_shape(post, lv[l].nx, lv[l].ny) : tiles(l);
         if (rtu)
             launch_pdl(M.rz ? rt_up2_kernel<T, true>(post) : rt_up2_kernel<T, false>(post), h.grid, dim3(h.threads), 0,
-                       st, lv[l], lv[l + 1], lv[l + 2], omega);
+                       st, lv[l], lv[l + 1], lv[l + 2], omega, O.stop);
         else
             launch_pdl(up2_kernel<T>(post), h.grid, dim3(h.threads), up2_smem<T>(post), st, lv[l], lv[l + 1], lv[l + 2],
                        omega);
@@ -2414,7 +2472,7 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
         const RtShape h = rtu ? rt_up_shape(post, lv[l].nx, lv[l].ny, false) : tiles(l);
         if (rtu)
             launch_pdl(M.rz ? rt_up_kernel<T, true, false>(post) : rt_up_kernel<T, false, false>(post), h.grid,
-                       dim3(h.threads), 0, st, lv[l], lv[l + 1], omega, (double*)nullptr, ResArgs{});
+                       dim3(h.threads), 0, st, lv[l], lv[l + 1], omega, (double*)nullptr, ResArgs{}, O.stop);
         else
             launch_pdl(M.rz ? up_kernel<T, true>(post) : up_kernel<T, false>(post), h.grid, dim3(h.threads), up, st,
                        lv[l], lv[l + 1], omega, (double*)nullptr);
@@ -2431,10 +2489,13 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
         R.max_cycles = max_cycles;
         R.cond = cond;
         R.use_cond = use_cond;
+        R.decide = O.decide ? 1 : 0;
+        R.inc = O.inc;
+        R.fblocks = O.fblocks;
         const RtShape h = rtu ? rt_up_shape(post, lv[0].nx, lv[0].ny, true) : tiles(0);
         if (rtu)
             launch_pdl(M.rz ? rt_up_kernel<T, true, true>(post) : rt_up_kernel<T, false, true>(post), h.grid,
-                       dim3(h.threads), 0, st, lv[0], lv[1], omega, phi, R);
+                       dim3(h.threads), 0, st, lv[0], lv[1], omega, phi, R, O.stop);
         else
             launch_pdl(M.rz ? up_res_kernel<T, true>(post) : up_res_kernel<T, false>(post), h.grid, dim3(h.threads),
                        up_smem<T>(post, M.rz, true), st, lv[0], lv[1], omega, phi, R);
@@ -2443,6 +2504,49 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
     }
     ++count;
     PIC_LAUNCH_CHECK();
+    return PIC_OK;
+}
+
+// The first cycles of a register-tile solve as plain launches.  The first
+// cycle's finest down phase forms the first residual (no launch of its own).
+// The first min_cycles cycles always run, and the ones before the last of them
+// end without a norm; the others do nothing once the solve has stopped.
+// How many: one past min_cycles, or kAheadCycles from a guess of unknown
+// quality: an iteration of the graph's WHILE node costs about 5.5 us more than
+// launches in line, a cycle that does nothing about 1 us per launch (a second
+// cycle in the node's body costs large grids more than it saves: 2049^2 solve
+// 1008 us against 942).
+constexpr int kAheadCycles = 4;
+
+static int first_cycles(int max_cycles, int min_cycles) {
+    return std::min(max_cycles, min_cycles > 0 ? min_cycles + 1 : kAheadCycles);
+}
+
+template <class T>
+static int launch_first_cycles(MgImpl& M, std::vector<LevelDev<T>>& lv, double* phi, const double* f, double tol,
+                               int max_cycles, int min_cycles, cudaGraphConditionalHandle cond, int use_cond,
+                               cudaStream_t st) {
+    const int kmin = std::max(0, std::min(min_cycles, max_cycles)), K = first_cycles(max_cycles, kmin);
+    const RtInit init{phi, f, M.rz0, M.r64, 1.0 / (M.dx * M.dx), 1.0 / (M.dy * M.dy)};
+    const RtShape h0 = rt_up_shape(M.o.pre_sweeps, M.nx, M.ny, true);
+    int last = 0;  // cycles finished at the last decision
+    for (int k = 0; k < K; ++k) {
+        CycleOpts O;
+        if (k == 0) {
+            O.init = &init;
+            O.init_decide = kmin == 0;
+        }
+        O.stop = k < kmin ? nullptr : M.N.stop;
+        O.decide = k + 1 >= kmin;
+        if (O.decide) {
+            O.inc = k + 1 - last;
+            O.fblocks = last == 0 && kmin > 0 ? int(h0.grid.x * h0.grid.y) : 0;
+            last = k + 1;
+        }
+        int count = 0;
+        PIC_TRY(launch_cycle(M, lv, phi, f, tol, max_cycles, cond, use_cond, st, count, O));
+        M.body_launches = count;
+    }
     return PIC_OK;
 }
 
@@ -2458,14 +2562,21 @@ static int capture_solve(MgImpl& M, std::vector<LevelDev<T>>& lv, double* phi, c
     size_t nd = 0;
     PIC_CUDA(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, &nd));
     if (cs != cudaStreamCaptureStatusActive) return fail(PIC_ERR_BAD_ARG, "multigrid: stream is not capturing");
+    const bool rt = rt_cycles(M) && max_cycles > 0;
+    if (rt && first_cycles(max_cycles, min_cycles) >= max_cycles)  // no loop left
+        return launch_first_cycles(M, lv, phi, f, tol, max_cycles, min_cycles, cudaGraphConditionalHandle{}, 0, st);
     cudaGraphConditionalHandle h;
     PIC_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
-    const int K = std::max(0, std::min(min_cycles, max_cycles));
-    launch_r0(M, lv, phi, f, tol, max_cycles, 1, h, K == 0, st);
-    PIC_LAUNCH_CHECK();
-    for (int k = 0; k < K; ++k) {
-        int count = 0;
-        PIC_TRY(launch_cycle(M, lv, phi, f, tol, max_cycles, h, k == K - 1, st, count));
+    if (rt) {
+        PIC_TRY(launch_first_cycles(M, lv, phi, f, tol, max_cycles, min_cycles, h, 1, st));
+    } else {
+        const int K = std::max(0, std::min(min_cycles, max_cycles));
+        launch_r0(M, lv, phi, f, tol, max_cycles, 1, h, K == 0, st);
+        PIC_LAUNCH_CHECK();
+        for (int k = 0; k < K; ++k) {
+            int count = 0;
+            PIC_TRY(launch_cycle(M, lv, phi, f, tol, max_cycles, h, k == K - 1, st, count));
+        }
     }
     PIC_CUDA(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, &nd));
     cudaGraphNodeParams p{};
@@ -2733,9 +2844,13 @@ int mg_body_launches(pic_mg* mg) {
                             (M.o.launch_mode == PIC_MG_CLUSTER && M.cluster_ok);
     return one_kernel ? 0 : M.body_launches;
 }
-// Kernels a solve runs besides its V-cycles: the residual, or the three
-// sine-transform kernels and the residual.
-int mg_fixed_launches(pic_mg* mg) { return mg && mg->m.dst ? 4 : 1; }
+// Kernels a solve runs besides its V-cycles: the first residual (the first
+// cycle's own on register tiles), or the three sine-transform kernels and the
+// residual.
+int mg_fixed_launches(pic_mg* mg) {
+    if (!mg) return 1;
+    return mg->m.dst ? 4 : mg->m.o.launch_mode == PIC_MG_GRAPH_LOOP && rt_cycles(mg->m) ? 0 : 1;
+}
 int mg_capture_into(pic_mg* mg, double* phi, const double* f, double tol, int max_cycles, int min_cycles,
                     cudaStream_t st) {
     return mg_capture(mg->m, phi, f, tol, max_cycles, min_cycles, st);
