@@ -80,6 +80,24 @@ int pic_update_V(const float* d_x, const float* d_y, float* d_vx, float* d_vy, i
 int pic_deposit(const float* d_x, const float* d_y, int n, float scale, float* d_rho, int nx, int ny,
                 void* stream);
 
+/* The same two operators by 16-byte accesses, for many particles per node
+ * (more than about two) in any order; the caller keeps the scratch (4 floats
+ * per node, 16-byte aligned).
+ *
+ * pic_deposit_cells: adds scale*w of each live particle to its cell's four
+ *   corner sums, d_cells[4*(j*nx + i) + {0, 1, 2, 3}] for the nodes (i, j),
+ *   (i+1, j), (i, j+1), (i+1, j+1).  The caller zeroes d_cells once.
+ * pic_cells_density: d_rho (written, not added to) = each node's corners.
+ * pic_field_pairs: d_pairs[4*(j*nx + i) + ...] = (Ex, Ey) at node (i, j) and
+ *   at (min(i+1, nx-1), j).
+ * pic_update_V_pairs: pic_update_V from d_pairs, bit for bit. */
+int pic_deposit_cells(const float* d_x, const float* d_y, int n, float scale, float* d_cells, int nx, int ny,
+                      void* stream);
+int pic_cells_density(const float* d_cells, float* d_rho, int nx, int ny, void* stream);
+int pic_field_pairs(const float* d_Ex, const float* d_Ey, float* d_pairs, int nx, int ny, void* stream);
+int pic_update_V_pairs(const float* d_x, const float* d_y, float* d_vx, float* d_vy, int n, const float* d_pairs,
+                       int nx, int ny, float kq, void* stream);
+
 /* Grid2D.update_E (src/Grid.py:232-243, kernel :157-196): E = -grad(phi),
  * central differences inside, one-sided at the edges, computed in FP64 and
  * stored as float32 planes d_Ex, d_Ey (nx*ny each). */

@@ -210,11 +210,17 @@ class Particles2D:
     def update_V(self, grid, dt):
         """Gather E at each particle and kick v += q/m E dt (src/Particles.py:378-410)."""
         self.grid = grid
+        pairs = grid.field_pairs(self) if hasattr(grid, "field_pairs") else None
         for s in self.species:
-            if s.n:
+            if not s.n:
+                continue
+            kq = float(s.charge / s.mass * dt)
+            if pairs is not None:
+                _lib.call("pic_update_V_pairs", _lib.ptr(s.x), _lib.ptr(s.y), _lib.ptr(s.vx), _lib.ptr(s.vy), s.n,
+                          _lib.ptr(pairs), grid.m, grid.n, kq, _lib.stream_ptr())
+            else:
                 _lib.call("pic_update_V", _lib.ptr(s.x), _lib.ptr(s.y), _lib.ptr(s.vx), _lib.ptr(s.vy), s.n,
-                          _lib.ptr(grid.E[0]), _lib.ptr(grid.E[1]), grid.m, grid.n, float(s.charge / s.mass * dt),
-                          _lib.stream_ptr())
+                          _lib.ptr(grid.E[0]), _lib.ptr(grid.E[1]), grid.m, grid.n, kq, _lib.stream_ptr())
 
     # ---- removal and sorting ----
     def compact(self):

@@ -146,6 +146,10 @@ SIGNATURES = {
     "pic_absorb": [_vp, _vp, _i, _i, _i, _vp, _vp],
     "pic_update_V": [_vp, _vp, _vp, _vp, _i, _vp, _vp, _i, _i, _f, _vp],
     "pic_deposit": [_vp, _vp, _i, _f, _vp, _i, _i, _vp],
+    "pic_deposit_cells": [_vp, _vp, _i, _f, _vp, _i, _i, _vp],
+    "pic_cells_density": [_vp, _vp, _i, _i, _vp],
+    "pic_field_pairs": [_vp, _vp, _vp, _i, _i, _vp],
+    "pic_update_V_pairs": [_vp, _vp, _vp, _vp, _i, _vp, _i, _i, _f, _vp],
     "pic_update_E": [_vp, _vp, _vp, _i, _i, _d, _d, _vp],
     "pic_form_rhs": [_vp, _vp, _d, _vp, _i, _i, _vp],
     "pic_update_E_rz": [_vp, _vp, _vp, _i, _i, _d, _d, _vp],

@@ -13,7 +13,7 @@
 // stop) stay on the device: each kernel's last block to finish adds the block
 // partials in a fixed order and derives what the next kernel needs, so an
 // iteration is three launches besides the V-cycle's and no host round trip
-// (three of about 20 us each before; 385 x 257, tol 1e-9: 690 -> 215 us).  The
+// (three of about 20 us each before; 385 x 257, tol 1e-9: the call 691 -> 435 us).  The
 // host runs one iteration ahead of the stop flag it reads back; what is enqueued
 // past the end does nothing.
 #include <cmath>
