@@ -107,9 +107,10 @@ class MccOperator:
         self.seed = int(seed)
         self.step = 0
         dev = "cuda"
-        z = lambda: torch.zeros(birth_capacity, dtype=torch.float32, device=dev)  # noqa: E731
-        self.bx, self.by, self.bvx, self.bvy, self.bvz = z(), z(), z(), z(), z()
-        self.bspecies = torch.zeros(birth_capacity, dtype=torch.int32, device=dev)
+        # the birth buffer's arrays are rows of one tensor, so that taking births is one copy
+        self._births = torch.zeros((6, birth_capacity), dtype=torch.float32, device=dev)
+        self.bx, self.by, self.bvx, self.bvy, self.bvz = self._births[:5].unbind()
+        self.bspecies = self._births[5].view(torch.int32)
         self.bcount = torch.zeros(1, dtype=torch.int32, device=dev)
         self.counters = torch.zeros(30, dtype=torch.int64, device=dev)
         self._bb = _lib.BirthBuffer(self.bx.data_ptr(), self.by.data_ptr(), self.bvx.data_ptr(), self.bvy.data_ptr(),
@@ -130,8 +131,8 @@ class MccOperator:
 
     def take_births(self):
         k = min(int(self.bcount.item()), self.bx.numel())
-        out = (self.bspecies[:k].clone(), self.bx[:k].clone(), self.by[:k].clone(), self.bvx[:k].clone(),
-               self.bvy[:k].clone(), self.bvz[:k].clone())
+        rows = self._births[:, :k].clone()
+        out = (rows[5].view(torch.int32), *rows[:5].unbind())
         self.bcount.zero_()
         return out
 

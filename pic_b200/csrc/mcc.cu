@@ -98,44 +98,91 @@ void mcc_free(MccHost* H) {
     H->allocs.clear();
 }
 
-// One block per 4096 slots (16 candidate segments, one lane each).
-constexpr int kMccBlockSlots = 4096;
+// The collision operator on its own.  What bounds it is the chain of one
+// candidate (draws, the bin's table loads, Philox rounds, the scattering), so
+// the block gives every thread a segment to draw and then every thread a
+// candidate, however the candidates fall on the segments: kMccBlockSegments
+// segments of 256 slots per block, the candidates numbered by a scan of the
+// segments' counts.  Counts are summed in shared memory first.  (One lane in
+// sixteen drawing, the block then stepping over its slots: 20.5 us for 4M
+// electrons; this way 8.5 us.)
+constexpr int kMccBlockSegments = 128;
+constexpr int kMccWords = int(kMccSegment) / 32;
 
-__global__ void __launch_bounds__(256) k_mcc_apply(MccDev M, int s, const float* __restrict__ x,
-                                                   const float* __restrict__ y, float* __restrict__ vx,
-                                                   float* __restrict__ vy, float* __restrict__ vz, int n,
-                                                   uint32_t step, uint2 key, BirthDev B,
-                                                   unsigned long long* __restrict__ ctr) {
-    __shared__ unsigned bits[kMccBlockSlots / 32];
+__global__ void __launch_bounds__(kMccBlockSegments) k_mcc_apply(const __grid_constant__ MccDev M, int s,
+                                                                 const float* __restrict__ x,
+                                                                 const float* __restrict__ y, float* __restrict__ vx,
+                                                                 float* __restrict__ vy, float* __restrict__ vz, int n,
+                                                                 uint32_t step, uint2 key, BirthDev B,
+                                                                 unsigned long long* __restrict__ ctr) {
+    __shared__ unsigned bits[kMccBlockSegments * (kMccWords + 1)];  // a segment's words, padded against bank conflicts
+    __shared__ int first[kMccBlockSegments + 1];                    // the number of each segment's first candidate
+    __shared__ int warp_tot[kMccBlockSegments / 32];
+    __shared__ unsigned cnt[PIC_MAX_PROCESSES + 3];  // collisions, candidates, overflows, dropped births
     const MccSpeciesDev& S = M.sp[s];
-    const int b = blockIdx.x * kMccBlockSlots, e = min(n, b + kMccBlockSlots);
-    for (int q = threadIdx.x; q < kMccBlockSlots / 32; q += blockDim.x) bits[q] = 0;
-    __syncthreads();
-    constexpr int segs = kMccBlockSlots / int(kMccSegment);
-    if (threadIdx.x < segs) {
-        const long g = long(b) / kMccSegment + threadIdx.x;
-        if (g * long(kMccSegment) < e) mcc_mark_segment(S, uint32_t(s), g, n, b, e, step, key, bits);
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const long g = long(blockIdx.x) * kMccBlockSegments + t;
+    unsigned* mine = bits + t * (kMccWords + 1);
+#pragma unroll
+    for (int q = 0; q < kMccWords; ++q) mine[q] = 0u;
+    if (t < PIC_MAX_PROCESSES + 3) cnt[t] = 0u;
+    const long b = g * long(kMccSegment);
+    if (b < n)
+        mcc_mark_segment(S, uint32_t(s), g, n, int(b), int(min(long(n), b + long(kMccSegment))), step, key, mine);
+    int c = 0;
+#pragma unroll
+    for (int q = 0; q < kMccWords; ++q) c += __popc(mine[q]);
+    int incl = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
     }
+    if (lane == 31) warp_tot[w] = incl;
     __syncthreads();
-    for (int l = threadIdx.x; l < e - b; l += blockDim.x) {
-        if (!(bits[l >> 5] & (1u << (l & 31)))) continue;
-        const int p = b + l;
+    int before = 0;
+    for (int q = 0; q < w; ++q) before += warp_tot[q];
+    first[t] = before + incl - c;
+    if (t == kMccBlockSegments - 1) first[kMccBlockSegments] = before + incl;
+    __syncthreads();
+    const int total = first[kMccBlockSegments];
+    for (int k = t; k < total; k += kMccBlockSegments) {
+        int lo = 0, hi = kMccBlockSegments - 1;  // the last segment whose first candidate is <= k
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (first[mid] <= k) lo = mid;
+            else hi = mid - 1;
+        }
+        // the (k - first)-th set bit of its words
+        int r = k - first[lo], q = 0;
+        const unsigned* words = bits + lo * (kMccWords + 1);
+        while (r >= __popc(words[q])) r -= __popc(words[q++]);
+        const int p = int((long(blockIdx.x) * kMccBlockSegments + lo) * long(kMccSegment)) + 32 * q +
+                      int(__fns(words[q], 0u, r + 1));
         const float px = x[p], py = y[p];
         if (!is_live(px)) continue;
-        atomicAdd(ctr + kCtrCandidates + s, 1ull);
-        float a = vx[p], c = vy[p], d = vz[p];
-        const MccOutcome o = mcc_collide(M, S, uint32_t(s), uint32_t(p), step, key, a, c, d);
-        if (o.overflow) atomicAdd(ctr + kCtrOverflow, 1ull);
+        atomicAdd(&cnt[PIC_MAX_PROCESSES], 1u);
+        float a = vx[p], d = vy[p], e = vz[p];
+        const MccOutcome o = mcc_collide(M, S, uint32_t(s), uint32_t(p), step, key, a, d, e);
+        if (o.overflow) atomicAdd(&cnt[PIC_MAX_PROCESSES + 1], 1u);
         if (o.proc < 0) continue;
-        atomicAdd(ctr + kCtrCollisions + s * PIC_MAX_PROCESSES + o.proc, 1ull);
+        atomicAdd(&cnt[o.proc], 1u);
         vx[p] = a;
-        vy[p] = c;
-        vz[p] = d;
+        vy[p] = d;
+        vz[p] = e;
         if (o.born) {
             const bool ok_e = birth_push(B, S.born_e, px, py, o.be[0], o.be[1], o.be[2]);
             const bool ok_i = birth_push(B, S.born_i, px, py, o.bi[0], o.bi[1], o.bi[2]);
-            if (!ok_e || !ok_i) atomicAdd(ctr + kCtrDropped, 1ull);
+            if (!ok_e || !ok_i) atomicAdd(&cnt[PIC_MAX_PROCESSES + 2], 1u);
         }
+    }
+    __syncthreads();
+    if (t < PIC_MAX_PROCESSES + 3 && cnt[t]) {
+        const int at = t < PIC_MAX_PROCESSES        ? kCtrCollisions + s * PIC_MAX_PROCESSES + t
+                       : t == PIC_MAX_PROCESSES     ? kCtrCandidates + s
+                       : t == PIC_MAX_PROCESSES + 1 ? kCtrOverflow
+                                                    : kCtrDropped;
+        atomicAdd(ctr + at, (unsigned long long)cnt[t]);
     }
 }
 
@@ -193,8 +240,8 @@ int pic_mcc_apply(pic_mcc* m, int s, const float* d_x, const float* d_y, float* 
     BirthDev B{births->x, births->y, births->vx, births->vy, births->vz, births->species, births->count,
                births->capacity};
     const uint2 key = make_uint2(uint32_t(seed), uint32_t(seed >> 32));
-    const int blocks = div_up(n, kMccBlockSlots);
-    k_mcc_apply<<<blocks, 256, 0, as_stream(stream)>>>(m->h.dev, s, d_x, d_y, d_vx, d_vy, d_vz, n, step, key, B,
+    const int blocks = div_up(n, long(kMccBlockSegments) * kMccSegment);
+    k_mcc_apply<<<blocks, kMccBlockSegments, 0, as_stream(stream)>>>(m->h.dev, s, d_x, d_y, d_vx, d_vy, d_vz, n, step, key, B,
                                                        d_counters);
     PIC_LAUNCH_CHECK();
     return PIC_OK;
