@@ -1764,13 +1764,16 @@ struct MgImpl {
     unsigned long long wait_polls = kBarrierPolls;  // grid-barrier wait limit of the persistent solve
     cudaStream_t side = nullptr;
     cudaStream_t cap = nullptr;
-    // cached solve graph
-    cudaGraphExec_t exec = nullptr;
-    double* g_phi = nullptr;
-    const double* g_f = nullptr;
-    double g_tol = 0;
-    int g_max = -1;
-    int g_min = -1;
+    // cached solve graphs: [0] on the first pair of buffers a solve was given
+    // (its limits may change), [1] on the solver's own copies
+    struct Graph {
+        cudaGraphExec_t exec = nullptr;
+        double* phi = nullptr;
+        const double* f = nullptr;
+        double tol = 0;
+        int max = -1, min = -1;
+    } graph[2];
+    double *s_phi = nullptr, *s_f = nullptr;
 };
 
 }  // namespace pic
@@ -1822,9 +1825,12 @@ static int alloc_levels(MgImpl& M, std::vector<LevelDev<T>>& lv, const std::vect
         // the free nodes (not Dirichlet, not on a grid edge; in r-z the axis
         // row is free) as bit columns
         std::vector<uint32_t> fb(size_t((v.ny + 31) / 32) * v.nx, 0u);
-        for (int j = M.rz ? 0 : 1; j < v.ny - 1; ++j)
-            for (int i = 1; i < v.nx - 1; ++i)
-                if (!masks[l][size_t(j) * v.nx + i]) fb[size_t(j >> 5) * v.nx + i] |= 1u << (j & 31);
+        for (int j = M.rz ? 0 : 1; j < v.ny - 1; ++j) {
+            const uint8_t* __restrict__ m = masks[l].data() + size_t(j) * v.nx;
+            uint32_t* __restrict__ w = fb.data() + size_t(j >> 5) * v.nx;
+            const int n = v.nx - 1, bit = j & 31;
+            for (int i = 1; i < n; ++i) w[i] |= uint32_t(m[i] == 0) << bit;
+        }
         uint32_t* fbd = nullptr;
         PIC_CUDA(cudaMalloc(&fbd, fb.size() * sizeof(uint32_t)));
         M.allocs.push_back(fbd);
@@ -2146,7 +2152,8 @@ static int configure_cluster(MgImpl& M, const std::vector<int>& nxs, const std::
 static void mg_release(pic_mg* mg) {
     if (!mg) return;
     MgImpl& M = mg->m;
-    if (M.exec) cudaGraphExecDestroy(M.exec);
+    for (auto& g : M.graph)
+        if (g.exec) cudaGraphExecDestroy(g.exec);
     if (M.side) cudaStreamDestroy(M.side);
     if (M.cap) cudaStreamDestroy(M.cap);
     if (M.dst) dst_destroy(M.dst);
@@ -2724,12 +2731,14 @@ int mg_capture(MgImpl& M, double* phi, const double* f, double tol, int max_cycl
                                        : capture_solve(M, M.ld, phi, f, tol, max_cycles, min_cycles, st);
 }
 
-static int ensure_graph(MgImpl& M, double* phi, const double* f, double tol, int max_cycles, int min_cycles) {
-    if (M.exec && M.g_phi == phi && M.g_f == f && M.g_tol == tol && M.g_max == max_cycles && M.g_min == min_cycles)
+// A solve's graph, built again where its buffers or limits change.
+static int ensure_graph(MgImpl& M, MgImpl::Graph& G, double* phi, const double* f, double tol, int max_cycles,
+                        int min_cycles) {
+    if (G.exec && G.phi == phi && G.f == f && G.tol == tol && G.max == max_cycles && G.min == min_cycles)
         return PIC_OK;
-    if (M.exec) {
-        cudaGraphExecDestroy(M.exec);
-        M.exec = nullptr;
+    if (G.exec) {
+        cudaGraphExecDestroy(G.exec);
+        G.exec = nullptr;
     }
     PIC_CUDA(cudaStreamBeginCapture(M.cap, cudaStreamCaptureModeThreadLocal));
     const int rc = mg_capture(M, phi, f, tol, max_cycles, min_cycles, M.cap);
@@ -2740,14 +2749,47 @@ static int ensure_graph(MgImpl& M, double* phi, const double* f, double tol, int
         return rc;
     }
     if (ec != cudaSuccess) return fail(PIC_ERR_CUDA, "multigrid capture: %s", cudaGetErrorString(ec));
-    const cudaError_t ei = cudaGraphInstantiate(&M.exec, g, 0);
+    const cudaError_t ei = cudaGraphInstantiate(&G.exec, g, 0);
     cudaGraphDestroy(g);
     if (ei != cudaSuccess) return fail(PIC_ERR_CUDA, "multigrid graph instantiate: %s", cudaGetErrorString(ei));
-    M.g_phi = phi;
-    M.g_f = f;
-    M.g_tol = tol;
-    M.g_max = max_cycles;
-    M.g_min = min_cycles;
+    G.phi = phi;
+    G.f = f;
+    G.tol = tol;
+    G.max = max_cycles;
+    G.min = min_cycles;
+    return PIC_OK;
+}
+
+// A graph-loop solve.  Building a graph takes several hundred microseconds, so
+// buffers other than the first pair do not get one of their own: they are
+// copied to the solver's and back (a copy takes a few microseconds at 513^2, 16
+// at 2049^2).
+static int launch_graph(MgImpl& M, double* phi, const double* f, double tol, int max_cycles, int min_cycles,
+                        cudaStream_t st) {
+    const size_t nodes = size_t(M.nx) * M.ny, bytes = sizeof(double) * nodes;
+    MgImpl::Graph& own = M.graph[0];
+    bool copy = own.phi && (own.phi != phi || own.f != f);
+    if (copy && !M.s_phi) {
+        double* b = nullptr;
+        if (cudaMalloc(&b, 2 * bytes) == cudaSuccess) {
+            M.allocs.push_back(b);
+            M.s_phi = b;
+            M.s_f = b + nodes;
+        } else {
+            cudaGetLastError();  // no room: the first graph is built again for these buffers
+            copy = false;
+        }
+    }
+    if (!copy) {
+        PIC_TRY(ensure_graph(M, own, phi, f, tol, max_cycles, min_cycles));
+        PIC_CUDA(cudaGraphLaunch(own.exec, st));
+        return PIC_OK;
+    }
+    PIC_TRY(ensure_graph(M, M.graph[1], M.s_phi, M.s_f, tol, max_cycles, min_cycles));
+    PIC_CUDA(cudaMemcpyAsync(M.s_phi, phi, bytes, cudaMemcpyDeviceToDevice, st));
+    PIC_CUDA(cudaMemcpyAsync(M.s_f, f, bytes, cudaMemcpyDeviceToDevice, st));
+    PIC_CUDA(cudaGraphLaunch(M.graph[1].exec, st));
+    PIC_CUDA(cudaMemcpyAsync(phi, M.s_phi, bytes, cudaMemcpyDeviceToDevice, st));
     return PIC_OK;
 }
 
@@ -2816,9 +2858,7 @@ int mg_launch(MgImpl& M, double* phi, const double* f, double tol, int max_cycle
     if (M.o.launch_mode == PIC_MG_HOST_LOOP)
         return M.precision == PIC_MG_MIXED ? solve_eager(M, M.lf, phi, f, tol, max_cycles, min_cycles, st)
                                            : solve_eager(M, M.ld, phi, f, tol, max_cycles, min_cycles, st);
-    PIC_TRY(ensure_graph(M, phi, f, tol, max_cycles, min_cycles));
-    PIC_CUDA(cudaGraphLaunch(M.exec, st));
-    return PIC_OK;
+    return launch_graph(M, phi, f, tol, max_cycles, min_cycles, st);
 }
 
 int mg_solve(MgImpl& M, double* phi, const double* f, double tol, int max_cycles, pic_mg_info* info,

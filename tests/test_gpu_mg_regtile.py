@@ -180,3 +180,28 @@ def test_cycles_launched_ahead_stop_where_the_host_loop_stops(precision, max_cyc
             assert na == nb and abs(ra - rb) <= 1e-6 * rb + 1e-14
             scale = float(b.abs().max())
             assert float((a - b).abs().max()) <= 1e-12 * scale
+
+
+@pytest.mark.gpu
+def test_changing_buffers_and_limits():
+    """A solver given a new pair of buffers on each call, and the first pair again with
+    other limits, solves each as a solver of its own would."""
+    nx, ny = 129, 97
+    free, phi0, f = problem(nx, ny, False, electrode=True)
+    mask = (~free).astype(np.uint8).reshape(-1)
+    shared = MultigridSolver(mask, nx, ny, DX, hy=DY)
+    keep = []
+    for k, tol in enumerate((1e-6, 1e-6, 1e-9, 1e-9, 1e-6)):
+        F = torch.as_tensor((f * (k + 1)).reshape(-1).copy(), device="cuda")
+        a = torch.as_tensor(phi0.reshape(-1).copy(), device="cuda")
+        b = a.clone()
+        keep += [F, a]  # no buffer is handed out twice
+        _, (na, ra) = shared.solve(a, F, tol=tol)
+        _, (nb, rb) = MultigridSolver(mask, nx, ny, DX, hy=DY).solve(b, F, tol=tol)
+        assert na == nb and torch.equal(a, b)
+    first = keep[1]
+    first.copy_(torch.as_tensor(phi0.reshape(-1).copy()))
+    b = first.clone()
+    shared.solve(first, keep[0], tol=1e-10)
+    MultigridSolver(mask, nx, ny, DX, hy=DY).solve(b, keep[0], tol=1e-10)
+    assert torch.equal(first, b)
