@@ -352,6 +352,23 @@ __device__ __forceinline__ void rt_first_residual(const RtInit& I, const LevelDe
     }
 }
 
+// How a tile's phase follows the one before it.  RtLaunched: a launch of its own
+// in the chain, which waits for its predecessor and does nothing once the solve
+// has stopped.  RtInLoop: a phase of k_rt_rest, after a grid barrier.  Loads of
+// what the phase before did not write come ahead of wait().
+struct RtLaunched {
+    const int* stop;
+    __device__ __forceinline__ void wait() const {
+        pdl_wait();
+        pdl_trigger();
+    }
+    __device__ __forceinline__ bool done() const { return stopped(stop); }
+};
+struct RtInLoop {
+    __device__ __forceinline__ void wait() const {}
+    __device__ __forceinline__ bool done() const { return false; }
+};
+
 // What follows a down phase's right-hand side (in t.g): smooth from zero, store
 // the core's correction (and, on level 0, its right-hand side in the V-cycle's
 // precision), restrict the residual.  (cx, cy: the core's columns and rows.)
@@ -379,26 +396,32 @@ __device__ __forceinline__ void rt_down_rest(const LevelDev<T>& F, const LevelDe
     }
 }
 
-// The down phase (see k_mg_down): smooth from zero, restrict the residual.
-template <class T, int S, bool CYL>
-__global__ void __launch_bounds__(kRtMaxThreads) k_rt_down(LevelDev<T> F, LevelDev<T> C, T omega,
-                                                           const double* __restrict__ g64, const int* stop) {
+// The down phase (see k_mg_down) of the tile (bx, by): smooth from zero,
+// restrict the residual.
+template <class T, int S, bool CYL, class Sync>
+__device__ __forceinline__ void rt_down_tile(const LevelDev<T>& F, const LevelDev<T>& C, T omega, const double* g64,
+                                             int bx, int by, RtShared<T>& sh, const Sync& sync) {
     constexpr int HL = RtDown<S>::HL;
-    __shared__ RtShared<T> sh;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int cx = RtDown<S>::core(kRtCols), cy = RtDown<S>::core(rt_side());
-    const int i0 = int(blockIdx.x) * cx - HL + 2 * l, j0 = int(blockIdx.y) * cy - HL + kRtRows * w;
+    const int i0 = bx * cx - HL + 2 * l, j0 = by * cy - HL + kRtRows * w;
     RtTile<T> t;
     RtCoef<T, kRtRows, CYL> cf;
     rt_load_bits(F, i0, j0, t);
     const unsigned cfr = rt_free_bits(C.fb, C.nx, (C.ny + 31) >> 5, i0 >> 1, j0 >> 1, (1u << (kRtRows / 2)) - 1u);
     cf.load(F, omega, j0);
-    pdl_wait();
-    pdl_trigger();
+    sync.wait();
     if (g64) rt_load_rows<T, double>(g64, F.nx, F.ny, i0, j0, t.g);
     else rt_load_rows<T, T>(F.g, F.nx, F.ny, i0, j0, t.g);
-    if (stopped(stop)) return;
+    if (sync.done()) return;
     rt_down_rest<T, S, CYL>(F, C, t, cf, sh, i0, j0, cx, cy, g64 != nullptr, cfr);
+}
+
+template <class T, int S, bool CYL>
+__global__ void __launch_bounds__(kRtMaxThreads) k_rt_down(LevelDev<T> F, LevelDev<T> C, T omega,
+                                                           const double* __restrict__ g64, const int* stop) {
+    __shared__ RtShared<T> sh;
+    rt_down_tile<T, S, CYL>(F, C, omega, g64, blockIdx.x, blockIdx.y, sh, RtLaunched{stop});
 }
 
 // The finest down phase of a solve's first cycle: the right-hand side is the
@@ -459,18 +482,17 @@ __device__ __forceinline__ void rt_prolong(RtTile<T>& t, const T (&cv)[kRtRows /
     }
 }
 
-// The up phase (see k_mg_up, k_mg_up_res): add the prolonged coarse
-// correction and smooth; RES (level 0): phi += e and the FP64 residual
-// r -= A e on the core, its norm and the loop decision.
-template <class T, int S, bool CYL, bool RES>
-__global__ void __launch_bounds__(kRtMaxThreads) k_rt_up(LevelDev<T> F, LevelDev<T> C, T omega,
-                                                         double* __restrict__ phi, ResArgs R,
-                                                         const int* stop) {
+// The up phase (see k_mg_up, k_mg_up_res) of the tile (bx, by): add the
+// prolonged coarse correction and smooth; RES (level 0): phi += e and the FP64
+// residual r -= A e on the core, its squares in r2.
+template <class T, int S, bool CYL, bool RES, class Sync>
+__device__ __forceinline__ bool rt_up_tile(const LevelDev<T>& F, const LevelDev<T>& C, T omega, double* phi,
+                                           const ResArgs& R, int bx, int by, RtShared<T>& sh, double& r2,
+                                           const Sync& sync) {
     using G = RtUp<S, RES>;
-    __shared__ RtShared<T> sh;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int cx = G::core(kRtCols), cy = G::core(rt_side());
-    const int i0 = int(blockIdx.x) * cx - G::HL + 2 * l, j0 = int(blockIdx.y) * cy - G::HL + kRtRows * w;
+    const int i0 = bx * cx - G::HL + 2 * l, j0 = by * cy - G::HL + kRtRows * w;
     RtTile<T> t;
     RtCoef<T, kRtRows, CYL> cf;
     rt_load_bits(F, i0, j0, t);
@@ -494,8 +516,7 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_up(LevelDev<T> F, LevelDev
             }
         }
     }
-    pdl_wait();
-    pdl_trigger();
+    sync.wait();
     {
         const int I = i0 >> 1, J0 = j0 >> 1;
         T cv[kRtRows / 2 + 1], ce[kRtRows / 2 + 1];
@@ -510,7 +531,7 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_up(LevelDev<T> F, LevelDev
             const T y = __shfl_down_sync(0xffffffffu, cv[q], 1);
             ce[q] = l == 31 ? x : y;
         }
-        if (stopped(stop)) return;
+        if (sync.done()) return false;
         rt_prolong(t, cv, ce);
     }
     int buf = 0;
@@ -519,7 +540,7 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_up(LevelDev<T> F, LevelDev
     if constexpr (!RES) {
         rt_store_core<T, G::HL>(F.ec, t.e, F.nx, F.ny, i0, j0, cx, cy);
     } else {
-        double r2 = 0.0;
+        r2 = 0.0;
 #pragma unroll
         for (int r = 0; r < kRtRows; ++r) {
             const int lr = w * kRtRows + r, j = j0 + r;
@@ -546,6 +567,19 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_up(LevelDev<T> F, LevelDev
                 r2 += rr * rr;
             }
         }
+    }
+    return true;
+}
+
+// The phase as a launch; RES: its norm and the loop decision too.
+template <class T, int S, bool CYL, bool RES>
+__global__ void __launch_bounds__(kRtMaxThreads) k_rt_up(LevelDev<T> F, LevelDev<T> C, T omega,
+                                                         double* __restrict__ phi, ResArgs R,
+                                                         const int* stop) {
+    __shared__ RtShared<T> sh;
+    double r2 = 0.0;
+    if (!rt_up_tile<T, S, CYL, RES>(F, C, omega, phi, R, blockIdx.x, blockIdx.y, sh, r2, RtLaunched{stop})) return;
+    if constexpr (RES) {
         if (R.decide)
             norm_reduce_decide(r2, 0.0, R.N, R.tol2, R.max_cycles, 0, R.cond, R.use_cond, R.inc, R.fblocks);
     }
@@ -613,14 +647,13 @@ __device__ __forceinline__ void rt_c_sweeps(RtCTile<T>& t, const RtCoef<T, kRtCR
     }
 }
 
-template <class T, int S, bool CYL>
-__global__ void __launch_bounds__(kRtMaxThreads) k_rt_down2(LevelDev<T> F, LevelDev<T> C, LevelDev<T> C2, T omega,
-                                                           const int* stop) {
+template <class T, int S, bool CYL, class Sync>
+__device__ __forceinline__ void rt_down2_tile(const LevelDev<T>& F, const LevelDev<T>& C, const LevelDev<T>& C2, T omega,
+                                             int bx, int by, RtShared<T>& sh, const Sync& sync) {
     using G = RtDown2<S>;
-    __shared__ RtShared<T> sh;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int cx = G::core(kRtCols), cy = G::core(rt_side());
-    const int i0 = int(blockIdx.x) * cx - G::HL + 2 * l, j0 = int(blockIdx.y) * cy - G::HL + kRtRows * w;
+    const int i0 = bx * cx - G::HL + 2 * l, j0 = by * cy - G::HL + kRtRows * w;
     const int I = i0 >> 1, J0 = j0 >> 1;
     RtTile<T> t;
     RtCTile<T> ct;
@@ -631,10 +664,9 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_down2(LevelDev<T> F, Level
     const unsigned c2fr = rt_free_bits(C2.fb, C2.nx, (C2.ny + 31) >> 5, I >> 1, J0 >> 1, 1u);
     cf.load(F, omega, j0);
     cc.load(C, omega, J0);
-    pdl_wait();
-    pdl_trigger();
+    sync.wait();
     rt_load_rows<T, T>(F.g, F.nx, F.ny, i0, j0, t.g);
-    if (stopped(stop)) return;
+    if (sync.done()) return;
     int buf = 0;
     rt_sweeps<T, S, CYL, true, true>(t, cf, sh, buf);
     rt_store_core<T, G::HL>(F.e, t.e, F.nx, F.ny, i0, j0, cx, cy);
@@ -688,13 +720,19 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_down2(LevelDev<T> F, Level
 }
 
 template <class T, int S, bool CYL>
-__global__ void __launch_bounds__(kRtMaxThreads) k_rt_up2(LevelDev<T> F, LevelDev<T> C, LevelDev<T> C2, T omega,
+__global__ void __launch_bounds__(kRtMaxThreads) k_rt_down2(LevelDev<T> F, LevelDev<T> C, LevelDev<T> C2, T omega,
                                                            const int* stop) {
-    using G = RtUp2<S>;
     __shared__ RtShared<T> sh;
+    rt_down2_tile<T, S, CYL>(F, C, C2, omega, blockIdx.x, blockIdx.y, sh, RtLaunched{stop});
+}
+
+template <class T, int S, bool CYL, class Sync>
+__device__ __forceinline__ void rt_up2_tile(const LevelDev<T>& F, const LevelDev<T>& C, const LevelDev<T>& C2, T omega,
+                                             int bx, int by, RtShared<T>& sh, const Sync& sync) {
+    using G = RtUp2<S>;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int cx = G::core(kRtCols), cy = G::core(rt_side());
-    const int i0 = int(blockIdx.x) * cx - G::HL + 2 * l, j0 = int(blockIdx.y) * cy - G::HL + kRtRows * w;
+    const int i0 = bx * cx - G::HL + 2 * l, j0 = by * cy - G::HL + kRtRows * w;
     const int I = i0 >> 1, J0 = j0 >> 1;
     RtTile<T> t;
     RtCTile<T> ct;
@@ -712,8 +750,7 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_up2(LevelDev<T> F, LevelDe
         ct.e[q] = C.e[K];
         ct.g[q] = C.g[K];
     }
-    pdl_wait();
-    pdl_trigger();
+    sync.wait();
     {
         // C2's correction prolonged onto C: an odd column takes the mean of
         // its own C2 column and the next lane's
@@ -733,7 +770,7 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_up2(LevelDev<T> F, LevelDe
             ct.e[q] = ((ct.fr >> q) & 1u) ? ct.e[q] + v : T(0);
         }
     }
-    if (stopped(stop)) return;
+    if (sync.done()) return;
     int buf = 0;
     rt_c_sweeps<T, S, CYL, false>(ct, cc, sh, buf);
     {
@@ -744,6 +781,138 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_up2(LevelDev<T> F, LevelDe
     }
     rt_sweeps<T, S, CYL, false, false>(t, cf, sh, buf);
     rt_store_core<T, G::HL>(F.ec, t.e, F.nx, F.ny, i0, j0, cx, cy);
+}
+
+template <class T, int S, bool CYL>
+__global__ void __launch_bounds__(kRtMaxThreads) k_rt_up2(LevelDev<T> F, LevelDev<T> C, LevelDev<T> C2, T omega,
+                                                           const int* stop) {
+    __shared__ RtShared<T> sh;
+    rt_up2_tile<T, S, CYL>(F, C, C2, omega, blockIdx.x, blockIdx.y, sh, RtLaunched{stop});
+}
+
+// ---- the cycles after the launched ones, in one cooperative launch ----------------------
+
+// The cycles a solve still needs after those launched in line, on grids whose
+// every phase is one wave of tiles: nothing when the solve has stopped (the
+// usual case), else V-cycles with a grid barrier between phases until it
+// converges or reaches max_cycles.  A conditional node costs a solve 6.6 us on
+// the device also when its condition is false, and the graph that holds one
+// more time to launch; this launch costs 2 us (a simulation's step to 1e-8 with
+// the node and with this launch: 129 x 97 68.5 and 57.2 us, 513 x 513 104.9 and
+// 89.4).  A cycle in here takes about 10 us more than one of the node's (129 x
+// 129 27 us against 17.5): a barrier costs 1 to 2 us where a launch in line
+// costs 1, and the phases' code leaves the instruction cache.
+template <class T>
+struct RtRest {
+    int lc;     // levels above the direct solve: [0, lc)
+    int fuse2;  // levels lc - 2 and lc - 1 in one phase each way
+    LevelDev<T> lv[kMgMaxLevels];
+    DirectDesc<T> direct;
+    int direct64;  // its inverse is FP64
+    ResArgs res;
+    double* phi;
+    T omega;
+    GridBar* bar;
+    int* error;
+    unsigned long long polls;
+};
+
+template <class T, class MT>
+__device__ __forceinline__ void rt_direct(const DirectDesc<T>& D, MT* gs) {
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const MT* __restrict__ ainv = static_cast<const MT*>(D.ainv);
+    for (int k = threadIdx.x; k < D.n; k += blockDim.x) gs[k] = MT(D.g[__ldg(D.idx + k)]);
+    if (blockIdx.x == 0)
+        for (int k = threadIdx.x; k < D.nz; k += blockDim.x) D.e[D.zidx[k]] = T(0);
+    __syncthreads();
+    for (int row = int(blockIdx.x) * rt_warps() + w; row < D.n; row += int(gridDim.x) * rt_warps()) {
+        MT s = MT(0);
+#pragma unroll 5
+        for (int u = 0; u < kDirectCols; ++u) {
+            const int c = l + 32 * u;
+            if (c < D.n) s += __ldg(ainv + long(row) * D.n + c) * gs[c];
+        }
+        const double t = warp_sum(double(s));
+        if (l == 0) D.e[__ldg(D.idx + row)] = T(t);
+    }
+}
+
+template <class T, int S, bool CYL>
+__global__ void __launch_bounds__(kRtMaxThreads, 1) k_rt_rest(const __grid_constant__ RtRest<T> D) {
+    if (stopped(D.res.N.stop)) return;
+    __shared__ RtShared<T> sh;
+    __shared__ double gs[kDirectMaxFree];
+    __shared__ double ws[kRtMaxWarps];
+    const int bid = int(blockIdx.x), nb = int(gridDim.x), w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const NormState& N = D.res.N;
+    const int before = *N.cycles;
+    const double f2 = N.norms[0], lim = D.res.tol2 * (f2 > 0.0 ? f2 : 1.0);
+    const int lsingle = D.fuse2 ? D.lc - 2 : D.lc;
+    const RtInLoop go{};
+    int seq = 0, n = 0;
+    double r2 = 0.0;
+    bool conv = false;
+    auto barrier = [&]() { return grid_barrier(D.bar, D.error, seq++, D.polls); };
+    // this block's tile of a phase on level L (every phase has at most nb tiles)
+    auto tile = [&](const LevelDev<T>& L, int cx, int cy, int& bx, int& by) {
+        const int tx = (L.nx + cx - 1) / cx;
+        bx = bid % tx;
+        by = bid / tx;
+        return by * cy < L.ny;
+    };
+    do {
+        int bx, by;
+        for (int k = 0; k < lsingle; ++k) {
+            if (tile(D.lv[k], RtDown<S>::core(kRtCols), RtDown<S>::core(rt_side()), bx, by))
+                rt_down_tile<T, S, CYL>(D.lv[k], D.lv[k + 1], D.omega, k == 0 ? D.res.r64 : nullptr, bx, by, sh, go);
+            if (!barrier()) return;
+        }
+        if (D.fuse2) {
+            if (tile(D.lv[lsingle], RtDown2<S>::core(kRtCols), RtDown2<S>::core(rt_side()), bx, by))
+                rt_down2_tile<T, S, CYL>(D.lv[lsingle], D.lv[lsingle + 1], D.lv[lsingle + 2], D.omega, bx, by, sh, go);
+            if (!barrier()) return;
+        }
+        if (D.direct64) rt_direct<T, double>(D.direct, gs);
+        else rt_direct<T, T>(D.direct, reinterpret_cast<T*>(gs));
+        if (!barrier()) return;
+        if (D.fuse2) {
+            if (tile(D.lv[lsingle], RtUp2<S>::core(kRtCols), RtUp2<S>::core(rt_side()), bx, by))
+                rt_up2_tile<T, S, CYL>(D.lv[lsingle], D.lv[lsingle + 1], D.lv[lsingle + 2], D.omega, bx, by, sh, go);
+            if (!barrier()) return;
+        }
+        for (int k = lsingle - 1; k >= 1; --k) {
+            double u;
+            if (tile(D.lv[k], RtUp<S, false>::core(kRtCols), RtUp<S, false>::core(rt_side()), bx, by))
+                rt_up_tile<T, S, CYL, false>(D.lv[k], D.lv[k + 1], D.omega, nullptr, D.res, bx, by, sh, u, go);
+            if (!barrier()) return;
+        }
+        r2 = 0.0;
+        if (tile(D.lv[0], RtUp<S, true>::core(kRtCols), RtUp<S, true>::core(rt_side()), bx, by))
+            rt_up_tile<T, S, CYL, true>(D.lv[0], D.lv[1], D.omega, D.phi, D.res, bx, by, sh, r2, go);
+        // the norm: the blocks' sums, added by every block in the same order
+        r2 = warp_sum(r2);
+        if (l == 0) ws[w] = r2;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double s = 0.0;
+            for (int q = 0; q < rt_warps(); ++q) s += ws[q];
+            N.partial[bid] = s;
+        }
+        if (!barrier()) return;
+        r2 = 0.0;
+        for (int q = l; q < nb; q += 32) r2 += reinterpret_cast<const volatile double*>(N.partial)[q];
+        r2 = warp_sum(r2);
+        r2 = __shfl_sync(0xffffffffu, r2, 0);
+        ++n;
+        conv = r2 < lim;
+    } while (!conv && before + n < D.res.max_cycles);
+    if (bid == 0 && threadIdx.x == 0) {
+        N.norms[1] = r2;
+        *N.cycles = before + n;
+        *N.total += n;
+        *N.converged = conv ? 1 : 0;
+        *N.stop = 1;
+    }
 }
 
 // ---- launch tables ----------------------------------------------------------------------
@@ -786,6 +955,15 @@ template <class T, bool CYL>
 static RtFused2Kernel<T> rt_up2_kernel(int s) {
     static const RtFused2Kernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_up2<T, 1, CYL>, k_rt_up2<T, 2, CYL>,
                                                         k_rt_up2<T, 3, CYL>};
+    return k[s];
+}
+
+template <class T>
+using RtRestKernel = void (*)(const RtRest<T>);
+template <class T, bool CYL>
+static RtRestKernel<T> rt_rest_kernel(int s) {
+    static const RtRestKernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_rest<T, 1, CYL>, k_rt_rest<T, 2, CYL>,
+                                                        k_rt_rest<T, 3, CYL>};
     return k[s];
 }
 

@@ -1130,6 +1130,53 @@ __global__ void __launch_bounds__(kDirectRows * 32) k_mg_direct(DirectDesc<T> D,
     if (lane == 0 && out >= 0) D.e[out] = T(t);
 }
 
+// ---- grid barrier of the cooperative launches ----------------------------------------
+
+struct GridBar {
+    unsigned count;
+    unsigned gen;
+};
+
+// Grid-wide barrier of a cooperative launch; false (and *error set) if it
+// did not complete within `polls` polls (kBarrierPolls unless the solver's
+// wait limit was changed).  On a timeout the block also records, in
+// error[1..5], the barrier's sequence number, its block index and the counter
+// state it saw.
+__device__ __forceinline__ bool grid_barrier(GridBar* b, int* error, int seq, unsigned long long polls) {
+    __shared__ int s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        cuda::atomic_ref<unsigned, cuda::thread_scope_device> gen(b->gen), cnt(b->count);
+        const unsigned g = gen.load(cuda::memory_order_acquire);
+        const unsigned nb = gridDim.x * gridDim.y;
+        int ok = 1;
+        __threadfence();
+        if (cnt.fetch_add(1u, cuda::memory_order_acq_rel) == nb - 1u) {
+            cnt.store(0u, cuda::memory_order_relaxed);
+            gen.fetch_add(1u, cuda::memory_order_release);
+        } else {
+            unsigned long long k = 0;
+            while (gen.load(cuda::memory_order_acquire) == g) {
+                if (++k > polls) {
+                    ok = 0;
+                    if (atomicExch(error, 1) == 0) {
+                        error[1] = seq;
+                        error[2] = int(blockIdx.x);
+                        error[3] = int(cnt.load(cuda::memory_order_relaxed));
+                        error[4] = int(gen.load(cuda::memory_order_relaxed));
+                        error[5] = int(g);
+                    }
+                    break;
+                }
+            }
+        }
+        __threadfence();
+        s_ok = ok;
+    }
+    __syncthreads();
+    return s_ok != 0;
+}
+
 }  // namespace pic
 
 #include "mg_regtile.cuh"
@@ -1194,51 +1241,6 @@ __global__ void __launch_bounds__(256) k_mg_r0(const double* __restrict__ phi, c
 }
 
 // ---- persistent cooperative solve -------------------------------------------------
-
-struct GridBar {
-    unsigned count;
-    unsigned gen;
-};
-
-// Grid-wide barrier of a cooperative launch; false (and *error set) if it
-// did not complete within `polls` polls (kBarrierPolls unless the solver's
-// wait limit was changed).  On a timeout the block also records, in
-// error[1..5], the barrier's sequence number, its block index and the counter
-// state it saw.
-__device__ __forceinline__ bool grid_barrier(GridBar* b, int* error, int seq, unsigned long long polls) {
-    __shared__ int s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        cuda::atomic_ref<unsigned, cuda::thread_scope_device> gen(b->gen), cnt(b->count);
-        const unsigned g = gen.load(cuda::memory_order_acquire);
-        const unsigned nb = gridDim.x * gridDim.y;
-        int ok = 1;
-        __threadfence();
-        if (cnt.fetch_add(1u, cuda::memory_order_acq_rel) == nb - 1u) {
-            cnt.store(0u, cuda::memory_order_relaxed);
-            gen.fetch_add(1u, cuda::memory_order_release);
-        } else {
-            unsigned long long k = 0;
-            while (gen.load(cuda::memory_order_acquire) == g) {
-                if (++k > polls) {
-                    ok = 0;
-                    if (atomicExch(error, 1) == 0) {
-                        error[1] = seq;
-                        error[2] = int(blockIdx.x);
-                        error[3] = int(cnt.load(cuda::memory_order_relaxed));
-                        error[4] = int(gen.load(cuda::memory_order_relaxed));
-                        error[5] = int(g);
-                    }
-                    break;
-                }
-            }
-        }
-        __threadfence();
-        s_ok = ok;
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
 
 template <class T>
 struct SolveDesc {
@@ -1727,6 +1729,7 @@ struct MgImpl {
     int nx = 0, ny = 0, L = 0, Lc = 0;
     double dx = 0, dy = 0;
     bool rz = false;          // r-z geometry (PIC_GEOM_RZ)
+    bool edges_only = false;  // every Dirichlet node is on a grid edge
     double* rz0 = nullptr;    // level-0 row coefficients in FP64 (r-z)
     DstPlan* dst = nullptr;   // PIC_MG_DST: the sine-transform solve
     bool hybrid = false;      // PIC_MG_HYBRID: levels [Lt, L) in one cluster launch per cycle
@@ -2269,6 +2272,9 @@ int mg_create(int nx, int ny, double dx, double dy, const uint8_t* h_mask, const
         cudaMemset(M.cidx, 0, cb);
         cudaMemcpy(M.cidx, idx.data(), idx.size() * sizeof(int), cudaMemcpyHostToDevice);
     }
+    M.edges_only = true;
+    for (int j = M.rz ? 0 : 1; j < ny - 1 && M.edges_only; ++j)
+        M.edges_only = memchr(masks[0].data() + size_t(j) * nx + 1, 1, size_t(nx) - 2) == nullptr;
     const size_t esz = M.precision == PIC_MG_MIXED ? sizeof(float) : sizeof(double);
     M.Lp = 0;
     while (M.Lp < M.L && long(nxs[M.Lp]) * nys[M.Lp] > kPersistCoarseMax) ++M.Lp;
@@ -2294,16 +2300,9 @@ int mg_create(int nx, int ny, double dx, double dy, const uint8_t* h_mask, const
     if (st == PIC_OK && M.o.launch_mode == PIC_MG_DST) {
         // the sine-transform solve applies to Cartesian grids of 2^q + 1 nodes
         // whose Dirichlet nodes are the edges alone; otherwise the graph loop
-        bool edges_only = !M.rz;
-        for (int j = 1; j < ny - 1 && edges_only; ++j)
-            for (int i = 1; i < nx - 1; ++i)
-                if (masks[0][size_t(j) * nx + i]) {
-                    edges_only = false;
-                    break;
-                }
         const bool pow2 = nx - 1 >= 4 && ny - 1 >= 4 && nx - 1 <= 2048 && ny - 1 <= 2048 &&
                           ((nx - 1) & (nx - 2)) == 0 && ((ny - 1) & (ny - 2)) == 0;
-        if (edges_only && pow2) st = dst_create(nx, ny, dx, dy, &M.dst);
+        if (!M.rz && M.edges_only && pow2) st = dst_create(nx, ny, dx, dy, &M.dst);
         if (st == PIC_OK && !M.dst) M.o.launch_mode = PIC_MG_GRAPH_LOOP;
     }
     if (st == PIC_OK && M.Lc >= 1 &&
@@ -2518,22 +2517,30 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
 // cycle's finest down phase forms the first residual (no launch of its own).
 // The first min_cycles cycles always run, and the ones before the last of them
 // end without a norm; the others do nothing once the solve has stopped.
-// How many: one past min_cycles, or kAheadCycles from a guess of unknown
-// quality: an iteration of the graph's WHILE node costs about 5.5 us more than
-// launches in line, a cycle that does nothing about 1 us per launch (a second
-// cycle in the node's body costs large grids more than it saves: 2049^2 solve
-// 1008 us against 942).
-constexpr int kAheadCycles = 4;
+// How many (first_cycles): what the solve is expected to need.  A cycle divides
+// the residual by about 100 where all Dirichlet nodes are on the edges (r-z
+// sometimes takes one more).  A step's guess (min_cycles > 0), extrapolated from
+// the last two potentials, starts near 1e-2: 2, 3 and 4 cycles at tolerances
+// 1e-6, 1e-8 and 1e-10 from 97 x 65 to 2049^2.  Any other guess is taken as
+// cold.  A cycle that turns out not to be needed costs a launch of about 1 us
+// per phase (129 x 97 step at 1e-8: 63.5 us with one cycle more in line, 57.2
+// without; 2049^2: 703 and 624), one that was not launched 5.5 us more than
+// here in the graph's WHILE node (a second cycle in the node's body costs large
+// grids more than it saves: 2049^2 solve 1008 us against 942) and 10 more in
+// k_rt_rest.
+constexpr int kMaxAheadCycles = 8;
 
-static int first_cycles(int max_cycles, int min_cycles) {
-    return std::min(max_cycles, min_cycles > 0 ? min_cycles + 1 : kAheadCycles);
+static int first_cycles(int max_cycles, int min_cycles, double tol) {
+    const double d = tol > 0.0 ? std::min(-0.5 * std::log10(tol), double(kMaxAheadCycles)) : double(kMaxAheadCycles);
+    const int k = min_cycles > 0 ? std::max(min_cycles, int(std::ceil(d - 1.0))) : std::max(2, int(std::ceil(d + 1.0)));
+    return std::min(max_cycles, std::max(min_cycles, std::min(k, kMaxAheadCycles)));
 }
 
 template <class T>
 static int launch_first_cycles(MgImpl& M, std::vector<LevelDev<T>>& lv, double* phi, const double* f, double tol,
                                int max_cycles, int min_cycles, cudaGraphConditionalHandle cond, int use_cond,
                                cudaStream_t st) {
-    const int kmin = std::max(0, std::min(min_cycles, max_cycles)), K = first_cycles(max_cycles, kmin);
+    const int kmin = std::max(0, std::min(min_cycles, max_cycles)), K = first_cycles(max_cycles, kmin, tol);
     const RtInit init{phi, f, M.rz0, M.r64, 1.0 / (M.dx * M.dx), 1.0 / (M.dy * M.dy)};
     const RtShape h0 = rt_up_shape(M.o.pre_sweeps, M.nx, M.ny, true);
     int last = 0;  // cycles finished at the last decision
@@ -2557,12 +2564,81 @@ static int launch_first_cycles(MgImpl& M, std::vector<LevelDev<T>>& lv, double* 
     return PIC_OK;
 }
 
-// min_cycles: V-cycles chained in the capturing graph itself before the WHILE
-// node, which only then tests for convergence (each iteration of a WHILE
-// node costs a launch of its body graph).
+// Blocks of k_rt_rest for a solver: as many as the phase with the most tiles has
+// (and the direct solve can use); 0 where the WHILE node is used instead: more
+// tiles than SMs, sweeps that differ before and after, or a Dirichlet node off
+// the edges, where a solve takes twice the cycles that are launched in line
+// (385 x 193 FP64 with an electrode, to 1e-9: 432 us with k_rt_rest, 329
+// without).
+template <class T>
+static int rest_blocks(const MgImpl& M, const std::vector<LevelDev<T>>& lv) {
+    const int s = M.o.pre_sweeps;
+    if (!rt_cycles(M) || M.o.post_sweeps != s || !M.edges_only) return 0;
+    const int side = kRtRows * kRtMaxWarps, lsingle = M.fuse2 ? M.Lc - 2 : M.Lc;
+    auto core = [&](auto k1, auto k2, auto k3, int n) { return s == 1 ? k1(n) : s == 2 ? k2(n) : k3(n); };
+    auto tiles = [&](int l, int cx, int cy) { return long(div_up(lv[l].nx, cx)) * div_up(lv[l].ny, cy); };
+    long n = 0;
+    auto phase = [&](int l, auto k1, auto k2, auto k3) {
+        n = std::max(n, tiles(l, core(k1, k2, k3, kRtCols), core(k1, k2, k3, side)));
+    };
+    phase(0, RtUp<1, true>::core, RtUp<2, true>::core, RtUp<3, true>::core);
+    for (int l = 0; l < lsingle; ++l) {
+        phase(l, RtDown<1>::core, RtDown<2>::core, RtDown<3>::core);
+        if (l > 0) phase(l, RtUp<1, false>::core, RtUp<2, false>::core, RtUp<3, false>::core);
+    }
+    if (M.fuse2) {
+        phase(lsingle, RtDown2<1>::core, RtDown2<2>::core, RtDown2<3>::core);
+        phase(lsingle, RtUp2<1>::core, RtUp2<2>::core, RtUp2<3>::core);
+    }
+    if (n > num_sms()) return 0;
+    return int(std::max(n, std::min(long(num_sms()), long(div_up(M.dn, kRtMaxWarps)))));
+}
+
+template <class T>
+static int launch_rest(MgImpl& M, const std::vector<LevelDev<T>>& lv_in, double* phi, double tol, int max_cycles,
+                       int blocks, cudaStream_t st) {
+    const std::vector<LevelDev<T>> lv = with_corrections(lv_in, M.Lc);
+    RtRest<T> D{};
+    D.lc = M.Lc;
+    D.fuse2 = M.fuse2 ? 1 : 0;
+    for (int l = 0; l <= M.Lc; ++l) D.lv[l] = lv[l];
+    D.direct = DirectDesc<T>{M.dinv, M.didx, M.didx + M.dn, lv[M.Lc].g, lv[M.Lc].e, M.dn, M.dnz};
+    D.direct64 = M.dinv64 ? 1 : 0;
+    D.res.r64 = M.r64;
+    D.res.rz0 = M.rz ? (const double*)M.rz0 : nullptr;
+    D.res.cx = 1.0 / (M.dx * M.dx);
+    D.res.cy = 1.0 / (M.dy * M.dy);
+    D.res.N = M.N;
+    D.res.tol2 = tol * tol;
+    D.res.max_cycles = max_cycles;
+    D.phi = phi;
+    D.omega = T(M.o.omega);
+    D.bar = M.bar;
+    D.error = M.error;
+    D.polls = kBarrierPolls;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kRtMaxThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeCooperative;
+    attr[0].val.cooperative = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const int s = M.o.pre_sweeps;
+    PIC_CUDA(cudaLaunchKernelEx(&cfg, M.rz ? rt_rest_kernel<T, true>(s) : rt_rest_kernel<T, false>(s), D));
+    return PIC_OK;
+}
+
+// min_cycles: V-cycles that run before the first test for convergence.  The
+// cycles after those in line are a launch of k_rt_rest or a WHILE node.  alone:
+// the solve is not one of several that a graph runs side by side: a cooperative
+// launch waits until all of its blocks fit, also to do nothing, so that among 8
+// members' solves it costs more than the node (ensemble of 8 on 129 x 97 to
+// 257 x 193: 10 steps 4643 us against 3830).
 template <class T>
 static int capture_solve(MgImpl& M, std::vector<LevelDev<T>>& lv, double* phi, const double* f, double tol,
-                         int max_cycles, int min_cycles, cudaStream_t st) {
+                         int max_cycles, int min_cycles, bool alone, cudaStream_t st) {
     cudaStreamCaptureStatus cs;
     cudaGraph_t g = nullptr;
     const cudaGraphNode_t* deps = nullptr;
@@ -2570,8 +2646,12 @@ static int capture_solve(MgImpl& M, std::vector<LevelDev<T>>& lv, double* phi, c
     PIC_CUDA(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, &nd));
     if (cs != cudaStreamCaptureStatusActive) return fail(PIC_ERR_BAD_ARG, "multigrid: stream is not capturing");
     const bool rt = rt_cycles(M) && max_cycles > 0;
-    if (rt && first_cycles(max_cycles, min_cycles) >= max_cycles)  // no loop left
+    if (rt && first_cycles(max_cycles, min_cycles, tol) >= max_cycles)  // no loop left
         return launch_first_cycles(M, lv, phi, f, tol, max_cycles, min_cycles, cudaGraphConditionalHandle{}, 0, st);
+    if (const int blocks = rt && alone ? rest_blocks(M, lv) : 0) {
+        PIC_TRY(launch_first_cycles(M, lv, phi, f, tol, max_cycles, min_cycles, cudaGraphConditionalHandle{}, 0, st));
+        return launch_rest(M, lv, phi, tol, max_cycles, blocks, st);
+    }
     cudaGraphConditionalHandle h;
     PIC_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
     if (rt) {
@@ -2719,7 +2799,8 @@ static int launch_dst(MgImpl& M, double* phi, const double* f, double tol, int m
     return PIC_OK;
 }
 
-int mg_capture(MgImpl& M, double* phi, const double* f, double tol, int max_cycles, int min_cycles, cudaStream_t st) {
+int mg_capture(MgImpl& M, double* phi, const double* f, double tol, int max_cycles, int min_cycles, bool alone,
+               cudaStream_t st) {
     if (M.dst) return launch_dst(M, phi, f, tol, max_cycles, st);
     if (M.o.launch_mode == PIC_MG_CLUSTER && M.cluster_ok) return launch_cluster(M, phi, f, tol, max_cycles, st);
     if (M.o.launch_mode == PIC_MG_PERSISTENT)
@@ -2727,8 +2808,8 @@ int mg_capture(MgImpl& M, double* phi, const double* f, double tol, int max_cycl
                                            : launch_persistent(M, M.ld, phi, f, tol, max_cycles, st);
     if (M.o.launch_mode == PIC_MG_HOST_LOOP)
         return fail(PIC_ERR_BAD_ARG, "multigrid: the host-driven loop cannot be captured in a graph");
-    return M.precision == PIC_MG_MIXED ? capture_solve(M, M.lf, phi, f, tol, max_cycles, min_cycles, st)
-                                       : capture_solve(M, M.ld, phi, f, tol, max_cycles, min_cycles, st);
+    return M.precision == PIC_MG_MIXED ? capture_solve(M, M.lf, phi, f, tol, max_cycles, min_cycles, alone, st)
+                                       : capture_solve(M, M.ld, phi, f, tol, max_cycles, min_cycles, alone, st);
 }
 
 // A solve's graph, built again where its buffers or limits change.
@@ -2741,7 +2822,7 @@ static int ensure_graph(MgImpl& M, MgImpl::Graph& G, double* phi, const double* 
         G.exec = nullptr;
     }
     PIC_CUDA(cudaStreamBeginCapture(M.cap, cudaStreamCaptureModeThreadLocal));
-    const int rc = mg_capture(M, phi, f, tol, max_cycles, min_cycles, M.cap);
+    const int rc = mg_capture(M, phi, f, tol, max_cycles, min_cycles, true, M.cap);
     cudaGraph_t g = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(M.cap, &g);
     if (rc != PIC_OK) {
@@ -2891,9 +2972,9 @@ int mg_fixed_launches(pic_mg* mg) {
     if (!mg) return 1;
     return mg->m.dst ? 4 : mg->m.o.launch_mode == PIC_MG_GRAPH_LOOP && rt_cycles(mg->m) ? 0 : 1;
 }
-int mg_capture_into(pic_mg* mg, double* phi, const double* f, double tol, int max_cycles, int min_cycles,
+int mg_capture_into(pic_mg* mg, double* phi, const double* f, double tol, int max_cycles, int min_cycles, bool alone,
                     cudaStream_t st) {
-    return mg_capture(mg->m, phi, f, tol, max_cycles, min_cycles, st);
+    return mg_capture(mg->m, phi, f, tol, max_cycles, min_cycles, alone, st);
 }
 bool mg_uses_graph(pic_mg* mg) { return mg->m.o.launch_mode != PIC_MG_HOST_LOOP; }
 bool mg_is_rz(pic_mg* mg) { return mg->m.rz; }

@@ -43,7 +43,7 @@ int mg_create(int nx, int ny, double dx, double dy, const uint8_t* h_mask, const
 int mg_body_launches(pic_mg* mg);
 int mg_fixed_launches(pic_mg* mg);
 long long mg_total_cycles(pic_mg* mg);
-int mg_capture_into(pic_mg* mg, double* phi, const double* f, double tol, int max_cycles, int min_cycles,
+int mg_capture_into(pic_mg* mg, double* phi, const double* f, double tol, int max_cycles, int min_cycles, bool alone,
                     cudaStream_t st);
 int mg_launch_graph(pic_mg* mg, double* phi, const double* f, double tol, int max_cycles, int min_cycles,
                     cudaStream_t st);
@@ -1695,6 +1695,7 @@ struct SimImpl {
     cudaStream_t cap = nullptr, cap2 = nullptr;  // capture stream and the side branch of a captured step
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     // g_sort_step: the step whose side branch sorts for the next step
+    bool in_ensemble = false;  // being captured into an ensemble's loop
     cudaGraphExec_t g_step = nullptr, g_sort_step = nullptr;
     cudaGraphExec_t g_sort = nullptr;  // the cell sort alone (init, pic_sim_sort)
     long long sort_graph_launches = 0;
@@ -1922,7 +1923,8 @@ static int field_solve(SimImpl& S, cudaStream_t st, bool capturing) {
     }
     {
         PhaseTimer t(S, PIC_PHASE_SOLVE, st);
-        if (capturing) PIC_TRY(mg_capture_into(S.mg, S.phi, S.f, S.d.tol, S.d.max_cycles, S.d.min_cycles, st));
+        if (capturing)
+            PIC_TRY(mg_capture_into(S.mg, S.phi, S.f, S.d.tol, S.d.max_cycles, S.d.min_cycles, !S.in_ensemble, st));
         else PIC_TRY(mg_launch_graph(S.mg, S.phi, S.f, S.d.tol, S.d.max_cycles, S.d.min_cycles, st));
     }
     if (!S.have_prev) {
@@ -2397,9 +2399,11 @@ static int ens_capture(EnsImpl& E) {
         s0.push_back(S->solves);
         prof.push_back(S->profiling);
         S->profiling = false;
+        S->in_ensemble = true;
     }
     const int rc = ens_capture_body(E);
     for (size_t i = 0; i < E.m.size(); ++i) {
+        E.m[i]->in_ensemble = false;
         E.m[i]->launches = l0[i];
         E.m[i]->solves = s0[i];
         E.m[i]->profiling = prof[i];

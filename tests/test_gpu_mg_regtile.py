@@ -205,3 +205,33 @@ def test_changing_buffers_and_limits():
     shared.solve(first, keep[0], tol=1e-10)
     MultigridSolver(mask, nx, ny, DX, hy=DY).solve(b, keep[0], tol=1e-10)
     assert torch.equal(first, b)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sw", [1, 2, 3])
+@pytest.mark.parametrize("rz", [False, True])
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+@pytest.mark.parametrize("shape", [(49, 65), (129, 97), (321, 193), (609, 609), (641, 609)])
+def test_cycles_after_the_launched_ones(shape, precision, rz, sw):
+    """The cycles past those launched in line (one cooperative launch where a phase is one
+    wave of tiles, up to 609 x 609 here, and no electrode is inside; else the loop node) end in
+    the host loop's cycle, residual and potential, cut off by max_cycles and by the tolerance,
+    from a poor guess and from a good one.  FP64: as above.  FP32 cycles: the same operations on corrections that
+    are below 1e-2 of the potential by then, rounded at 6e-8: 1e-9 of it."""
+    nx, ny = shape
+    free, phi0, f = problem(nx, ny, rz, electrode=nx == 321)
+    mask = (~free).astype(np.uint8).reshape(-1)
+    F = torch.as_tensor(f.reshape(-1), device="cuda")
+    o = dict(precision=precision, hy=DY, pre_sweeps=sw, post_sweeps=sw, geometry="rz" if rz else "cartesian")
+    graph = MultigridSolver(mask, nx, ny, DX, **o)
+    host = MultigridSolver(mask, nx, ny, DX, launch="host", **o)
+    for tol, limit in ((1e-300, 10), (1e-3, 60), (1e-10, 60)):
+        a = torch.as_tensor(phi0.reshape(-1).copy(), device="cuda")
+        b = a.clone()
+        for _ in range(2):
+            _, (na, ra) = graph.solve(a, F, tol=tol, max_cycles=limit)
+            _, (nb, rb) = host.solve(b, F, tol=tol, max_cycles=limit)
+            assert na == nb and (tol > 1e-300 or na == limit)
+            assert abs(ra - rb) <= (1e-3 if precision == "mixed" else 1e-6) * rb + 1e-11
+            scale = float(b.abs().max())
+            assert float((a - b).abs().max()) <= (1e-9 if precision == "mixed" else 1e-12) * scale
