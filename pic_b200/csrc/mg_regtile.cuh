@@ -429,8 +429,10 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_down(LevelDev<T> F, LevelD
 // core is the residual up phase's.  decide: also the norms of the residual and
 // of f and the first loop decision; else the blocks' shares of ||f||^2, for the
 // decision after the first cycles (NormState::fpart).
+// Two blocks to an SM where 64 registers hold it (2049^2 69 us with one block,
+// 49 with two; r-z would spill: 129 x 97 step 1.7 us slower).
 template <class T, int S, bool CYL>
-__global__ void __launch_bounds__(kRtMaxThreads) k_rt_init(LevelDev<T> F, LevelDev<T> C, T omega, RtInit I, NormState N,
+__global__ void __launch_bounds__(kRtMaxThreads, sizeof(T) == 4 && !CYL ? 2 : 1) k_rt_init(LevelDev<T> F, LevelDev<T> C, T omega, RtInit I, NormState N,
                                                            double tol2, int max_cycles, int decide,
                                                            cudaGraphConditionalHandle cond, int use_cond) {
     constexpr int HL = RtDown<S>::HL;
@@ -482,13 +484,30 @@ __device__ __forceinline__ void rt_prolong(RtTile<T>& t, const T (&cv)[kRtRows /
     }
 }
 
+// An 8-byte copy from global to shared memory that the thread goes on past
+// (rows of an odd number of nodes allow no wider ones), and the wait for all of
+// this thread's.
+__device__ __forceinline__ void rt_copy8(double* dst, const double* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(unsigned(__cvta_generic_to_shared(dst))), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void rt_copy_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+constexpr int kRtUp = 0, kRtRes = 1, kRtResStaged = 2;  // the up phase's modes
+constexpr int kRtStage = 4 * kRtRows;  // staged doubles per thread of the residual up phase
+
 // The up phase (see k_mg_up, k_mg_up_res) of the tile (bx, by): add the
-// prolonged coarse correction and smooth; RES (level 0): phi += e and the FP64
-// residual r -= A e on the core, its squares in r2.
-template <class T, int S, bool CYL, bool RES, class Sync>
+// prolonged coarse correction and smooth; kRtRes (level 0): phi += e and the
+// FP64 residual r -= A e on the core, its squares in r2.  phi and r are loaded
+// before the wait, into registers (kRtRes) or shared memory (kRtResStaged, 128
+// bytes per thread and 64 registers): see rt_staged.  A 2049^2 grid's phase
+// moves 172 MB, 26 us at the copy rate, in 72 us from registers (one block of
+// 512 threads to an SM: load, sweeps and store follow each other) and in 50
+// staged (two).
+template <class T, int S, bool CYL, int MODE, class Sync>
 __device__ __forceinline__ bool rt_up_tile(const LevelDev<T>& F, const LevelDev<T>& C, T omega, double* phi,
-                                           const ResArgs& R, int bx, int by, RtShared<T>& sh, double& r2,
-                                           const Sync& sync) {
+                                           const ResArgs& R, int bx, int by, RtShared<T>& sh, double* stage,
+                                           double& r2, const Sync& sync) {
+    constexpr bool RES = MODE != kRtUp;
     using G = RtUp<S, RES>;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
     const int cx = G::core(kRtCols), cy = G::core(rt_side());
@@ -501,7 +520,9 @@ __device__ __forceinline__ bool rt_up_tile(const LevelDev<T>& F, const LevelDev<
     rt_load_rows<T, T>(F.e, F.nx, F.ny, i0, j0, t.e);
     rt_load_rows<T, T>(F.g, F.nx, F.ny, i0, j0, t.g);
     const bool core_col = 2 * l >= G::HL && 2 * l < G::HL + cx;
-    double pv[RES ? kRtRows : 1][2], rv[RES ? kRtRows : 1][2];
+    constexpr bool STAGED = MODE == kRtResStaged;
+    double pv[RES && !STAGED ? kRtRows : 1][2], rv[RES && !STAGED ? kRtRows : 1][2];
+    double* st = STAGED ? stage + threadIdx.x : nullptr;
     if constexpr (RES) {
 #pragma unroll
         for (int r = 0; r < kRtRows; ++r) {
@@ -511,8 +532,14 @@ __device__ __forceinline__ bool rt_up_tile(const LevelDev<T>& F, const LevelDev<
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 const bool ic = in && i0 + c < F.nx;
-                pv[r][c] = ic ? phi[k + c] : 0.0;
-                rv[r][c] = ic ? R.r64[k + c] : 0.0;
+                if constexpr (STAGED) {
+                    if (!ic) continue;
+                    rt_copy8(st + (4 * r + c) * blockDim.x, phi + k + c);
+                    rt_copy8(st + (4 * r + 2 + c) * blockDim.x, R.r64 + k + c);
+                } else {
+                    pv[r][c] = ic ? phi[k + c] : 0.0;
+                    rv[r][c] = ic ? R.r64[k + c] : 0.0;
+                }
             }
         }
     }
@@ -541,6 +568,7 @@ __device__ __forceinline__ bool rt_up_tile(const LevelDev<T>& F, const LevelDev<
         rt_store_core<T, G::HL>(F.ec, t.e, F.nx, F.ny, i0, j0, cx, cy);
     } else {
         r2 = 0.0;
+        if constexpr (STAGED) rt_copy_wait();
 #pragma unroll
         for (int r = 0; r < kRtRows; ++r) {
             const int lr = w * kRtRows + r, j = j0 + r;
@@ -550,7 +578,7 @@ __device__ __forceinline__ bool rt_up_tile(const LevelDev<T>& F, const LevelDev<
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 if (!in || i0 + c >= F.nx) continue;
-                phi[k + c] = pv[r][c] + double(t.e[r][c]);
+                phi[k + c] = (STAGED ? st[(4 * r + c) * blockDim.x] : pv[STAGED ? 0 : r][c]) + double(t.e[r][c]);
                 if (!((t.fr[c] >> r) & 1u)) continue;
                 // f - A(phi + e) = r - A e, in the association of k_mg_r0's Laplacian
                 const double e = double(t.e[r][c]);
@@ -562,7 +590,7 @@ __device__ __forceinline__ bool rt_up_tile(const LevelDev<T>& F, const LevelDev<
                     lap = R.cx * ((wv - e) + (ev - e)) + R.rz0[4 * j] * (n - e) + R.rz0[4 * j + 1] * (s - e);
                 else
                     lap = R.cx * ((wv - e) + (ev - e)) + R.cy * ((s - e) + (n - e));
-                const double rr = rv[r][c] - lap;
+                const double rr = (STAGED ? st[(4 * r + 2 + c) * blockDim.x] : rv[STAGED ? 0 : r][c]) - lap;
                 R.r64[k + c] = rr;
                 r2 += rr * rr;
             }
@@ -572,14 +600,16 @@ __device__ __forceinline__ bool rt_up_tile(const LevelDev<T>& F, const LevelDev<
 }
 
 // The phase as a launch; RES: its norm and the loop decision too.
-template <class T, int S, bool CYL, bool RES>
-__global__ void __launch_bounds__(kRtMaxThreads) k_rt_up(LevelDev<T> F, LevelDev<T> C, T omega,
+template <class T, int S, bool CYL, int MODE>
+__global__ void __launch_bounds__(kRtMaxThreads, MODE == kRtResStaged ? 2 : 1) k_rt_up(LevelDev<T> F, LevelDev<T> C, T omega,
                                                          double* __restrict__ phi, ResArgs R,
                                                          const int* stop) {
     __shared__ RtShared<T> sh;
+    extern __shared__ double rt_stage[];
     double r2 = 0.0;
-    if (!rt_up_tile<T, S, CYL, RES>(F, C, omega, phi, R, blockIdx.x, blockIdx.y, sh, r2, RtLaunched{stop})) return;
-    if constexpr (RES) {
+    if (!rt_up_tile<T, S, CYL, MODE>(F, C, omega, phi, R, blockIdx.x, blockIdx.y, sh, rt_stage, r2, RtLaunched{stop}))
+        return;
+    if constexpr (MODE != kRtUp) {
         if (R.decide)
             norm_reduce_decide(r2, 0.0, R.N, R.tol2, R.max_cycles, 0, R.cond, R.use_cond, R.inc, R.fblocks);
     }
@@ -883,12 +913,12 @@ __global__ void __launch_bounds__(kRtMaxThreads, 1) k_rt_rest(const __grid_const
         for (int k = lsingle - 1; k >= 1; --k) {
             double u;
             if (tile(D.lv[k], RtUp<S, false>::core(kRtCols), RtUp<S, false>::core(rt_side()), bx, by))
-                rt_up_tile<T, S, CYL, false>(D.lv[k], D.lv[k + 1], D.omega, nullptr, D.res, bx, by, sh, u, go);
+                rt_up_tile<T, S, CYL, kRtUp>(D.lv[k], D.lv[k + 1], D.omega, nullptr, D.res, bx, by, sh, nullptr, u, go);
             if (!barrier()) return;
         }
         r2 = 0.0;
         if (tile(D.lv[0], RtUp<S, true>::core(kRtCols), RtUp<S, true>::core(rt_side()), bx, by))
-            rt_up_tile<T, S, CYL, true>(D.lv[0], D.lv[1], D.omega, D.phi, D.res, bx, by, sh, r2, go);
+            rt_up_tile<T, S, CYL, kRtRes>(D.lv[0], D.lv[1], D.omega, D.phi, D.res, bx, by, sh, nullptr, r2, go);
         // the norm: the blocks' sums, added by every block in the same order
         r2 = warp_sum(r2);
         if (l == 0) ws[w] = r2;
@@ -937,10 +967,10 @@ static RtInitKernel<T> rt_init_kernel(int s) {
     return k[s];
 }
 
-template <class T, bool CYL, bool RES>
+template <class T, bool CYL, int MODE>
 static RtUpKernel<T> rt_up_kernel(int s) {
-    static const RtUpKernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_up<T, 1, CYL, RES>, k_rt_up<T, 2, CYL, RES>,
-                                                      k_rt_up<T, 3, CYL, RES>};
+    static const RtUpKernel<T> k[kRtMaxSweeps + 1] = {nullptr, k_rt_up<T, 1, CYL, MODE>, k_rt_up<T, 2, CYL, MODE>,
+                                                      k_rt_up<T, 3, CYL, MODE>};
     return k[s];
 }
 
@@ -957,6 +987,8 @@ static RtFused2Kernel<T> rt_up2_kernel(int s) {
                                                         k_rt_up2<T, 3, CYL>};
     return k[s];
 }
+
+static size_t rt_stage_bytes(int threads) { return sizeof(double) * kRtStage * threads; }
 
 template <class T>
 using RtRestKernel = void (*)(const RtRest<T>);

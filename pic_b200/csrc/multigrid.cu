@@ -1992,8 +1992,32 @@ static int configure_direct(MgImpl& M, const std::vector<int>& nxs, const std::v
     return PIC_OK;
 }
 
+// Whether the residual up phase of so many blocks keeps phi and r in shared
+// memory while it smooths: from the second wave on, where two blocks to an SM
+// overlap one's sweeps with the other's loads (2049^2 cycle 120.5 us without,
+// 101.4 staged; FP64 165 and 143; r-z 148 and 125; 641 x 609 28.1 and 26.5).  One
+// wave is faster from registers (513^2 phase 6.9 us, 9.0 staged: a block with
+// 64 KB waits for the SM's smaller split to drain), and so is FP64 r-z, whose
+// coefficients do not fit into 64 registers (1025^2 cycle 56.4 us, 61.7 staged).
+template <class T>
+static bool rt_staged(const MgImpl& M, const RtShape& h) {
+    return h.grid.x * h.grid.y > unsigned(num_sms()) && !(M.rz && sizeof(T) == 8);
+}
+template <class T>
+static RtUpKernel<T> rt_res_kernel(const MgImpl& M, bool staged) {
+    const int s = M.o.post_sweeps;
+    if (M.rz) {
+        if constexpr (sizeof(T) == 4)
+            if (staged) return rt_up_kernel<T, true, kRtResStaged>(s);
+        return rt_up_kernel<T, true, kRtRes>(s);
+    }
+    return staged ? rt_up_kernel<T, false, kRtResStaged>(s) : rt_up_kernel<T, false, kRtRes>(s);
+}
+
 template <class T>
 static int configure_kernels(MgImpl& M) {
+    if (M.o.post_sweeps <= kRtMaxSweeps && !(M.rz && sizeof(T) == 8))
+        PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(rt_res_kernel<T>(M, true)), rt_stage_bytes(kRtMaxThreads)));
     const size_t down = down_smem<T>(M.o.pre_sweeps, M.rz), up = up_smem<T>(M.o.post_sweeps, M.rz);
     const size_t upr = up_smem<T>(M.o.post_sweeps, M.rz, true);
     if (down > 227 * 1024 || upr > 227 * 1024 || M.cl[0].smem > 227 * 1024 || M.cl[1].smem > 227 * 1024)
@@ -2477,7 +2501,7 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
     for (int l = Lsingle - 1; l >= 1; --l) {
         const RtShape h = rtu ? rt_up_shape(post, lv[l].nx, lv[l].ny, false) : tiles(l);
         if (rtu)
-            launch_pdl(M.rz ? rt_up_kernel<T, true, false>(post) : rt_up_kernel<T, false, false>(post), h.grid,
+            launch_pdl(M.rz ? rt_up_kernel<T, true, kRtUp>(post) : rt_up_kernel<T, false, kRtUp>(post), h.grid,
                        dim3(h.threads), 0, st, lv[l], lv[l + 1], omega, (double*)nullptr, ResArgs{}, O.stop);
         else
             launch_pdl(M.rz ? up_kernel<T, true>(post) : up_kernel<T, false>(post), h.grid, dim3(h.threads), up, st,
@@ -2499,9 +2523,10 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
         R.inc = O.inc;
         R.fblocks = O.fblocks;
         const RtShape h = rtu ? rt_up_shape(post, lv[0].nx, lv[0].ny, true) : tiles(0);
+        const bool staged = rtu && rt_staged<T>(M, h);
         if (rtu)
-            launch_pdl(M.rz ? rt_up_kernel<T, true, true>(post) : rt_up_kernel<T, false, true>(post), h.grid,
-                       dim3(h.threads), 0, st, lv[0], lv[1], omega, phi, R, O.stop);
+            launch_pdl(rt_res_kernel<T>(M, staged), h.grid, dim3(h.threads), staged ? rt_stage_bytes(h.threads) : 0, st,
+                       lv[0], lv[1], omega, phi, R, O.stop);
         else
             launch_pdl(M.rz ? up_res_kernel<T, true>(post) : up_res_kernel<T, false>(post), h.grid, dim3(h.threads),
                        up_smem<T>(post, M.rz, true), st, lv[0], lv[1], omega, phi, R);

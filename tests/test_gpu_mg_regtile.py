@@ -235,3 +235,24 @@ def test_cycles_after_the_launched_ones(shape, precision, rz, sw):
             assert abs(ra - rb) <= (1e-3 if precision == "mixed" else 1e-6) * rb + 1e-11
             scale = float(b.abs().max())
             assert float((a - b).abs().max()) <= (1e-9 if precision == "mixed" else 1e-12) * scale
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sw", [1, 2, 3])
+@pytest.mark.parametrize("rz", [False, True])
+def test_cycles_of_more_than_one_wave_of_tiles(rz, sw):
+    """Grids of more tiles than the GPU has SMs, where the residual up phase keeps the
+    potential and the residual in shared memory: FP64 as above; one cycle in FP32 on the
+    same whole-level phases, a hundred operations in a row rounded at 6e-8: 2e-5 of
+    max|phi|."""
+    nx, ny = 705, 641
+    test_cycles_against_whole_level_phases((nx, ny), rz, (sw, sw))
+    free, phi0, f = problem(nx, ny, rz, electrode=True)
+    W = weights(ny, DX, DY, rz)
+    mg = MultigridSolver((~free).astype(np.uint8).reshape(-1), nx, ny, DX, omega=OMEGA, precision="mixed", hy=DY,
+                         pre_sweeps=sw, post_sweeps=sw, geometry="rz" if rz else "cartesian")
+    r = np.where(free, f - (neighbours(phi0, *W[:3]) - W[3][:, None] * phi0), 0.0)
+    want = phi0 + vcycle(r, free, DX, DY, rz, sw, sw)
+    phi = torch.as_tensor(phi0.reshape(-1).copy(), device="cuda")
+    mg.solve(phi, torch.as_tensor(f.reshape(-1), device="cuda"), tol=1e-300, max_cycles=1)
+    np.testing.assert_allclose(phi.cpu().numpy().reshape(ny, nx), want, rtol=0, atol=2e-5 * np.abs(want).max())
