@@ -352,6 +352,35 @@ __device__ __forceinline__ void rt_first_residual(const RtInit& I, const LevelDe
     }
 }
 
+// The decision, the same in every warp; `writer` (one thread of the grid) records
+// it.  True: the solve has stopped, now or before.  ref: ||f||^2.
+__device__ __forceinline__ bool rt_pending_stop(const RtPending& P, bool writer, double& ref) {
+    // a flag that this grid's writer has set already is this decision
+    if (!P.fblocks && stopped(P.N.stop)) return true;
+    const int l = threadIdx.x & 31;
+    double r2 = 0.0, f2 = 0.0;
+#pragma unroll
+    for (int u = 0; u < kRtPendingMax / 32; ++u) {
+        const int q = l + 32 * u;
+        if (q < P.nb) r2 += P.N.partial[q];
+        if (q < P.fblocks) f2 += P.N.fpart[q];
+    }
+    ref = P.fblocks ? 0.0 : P.N.norms[0];
+    r2 = warp_sum(r2);
+    if (P.fblocks) ref = warp_sum(f2);
+    const bool conv = r2 < P.tol2 * (ref > 0.0 ? ref : 1.0);
+    const bool stop = conv || P.done >= P.max_cycles;
+    if (writer) {
+        if (P.fblocks) P.N.norms[0] = ref;
+        P.N.norms[1] = r2;
+        *P.N.cycles = P.done;
+        *P.N.total += P.inc;
+        *P.N.converged = conv ? 1 : 0;
+        *P.N.stop = stop ? 1 : 0;
+    }
+    return stop;
+}
+
 // How a tile's phase follows the one before it.  RtLaunched: a launch of its own
 // in the chain, which waits for its predecessor and does nothing once the solve
 // has stopped.  RtInLoop: a phase of k_rt_rest, after a grid barrier.  Loads of
@@ -363,6 +392,18 @@ struct RtLaunched {
         pdl_trigger();
     }
     __device__ __forceinline__ bool done() const { return stopped(stop); }
+};
+struct RtPendingLaunched {
+    const int* stop;
+    const RtPending& P;
+    __device__ __forceinline__ void wait() const {
+        pdl_wait();
+        pdl_trigger();
+    }
+    __device__ __forceinline__ bool done() const {
+        double ref;
+        return P.nb ? rt_pending_stop(P, threadIdx.x == 0 && blockIdx.x + blockIdx.y == 0, ref) : stopped(stop);
+    }
 };
 struct RtInLoop {
     __device__ __forceinline__ void wait() const {}
@@ -419,9 +460,10 @@ __device__ __forceinline__ void rt_down_tile(const LevelDev<T>& F, const LevelDe
 
 template <class T, int S, bool CYL>
 __global__ void __launch_bounds__(kRtMaxThreads) k_rt_down(LevelDev<T> F, LevelDev<T> C, T omega,
-                                                           const double* __restrict__ g64, const int* stop) {
+                                                           const double* __restrict__ g64, const int* stop,
+                                                           const __grid_constant__ RtPending P) {
     __shared__ RtShared<T> sh;
-    rt_down_tile<T, S, CYL>(F, C, omega, g64, blockIdx.x, blockIdx.y, sh, RtLaunched{stop});
+    rt_down_tile<T, S, CYL>(F, C, omega, g64, blockIdx.x, blockIdx.y, sh, RtPendingLaunched{stop, P});
 }
 
 // The finest down phase of a solve's first cycle: the right-hand side is the
@@ -433,8 +475,7 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_down(LevelDev<T> F, LevelD
 // 49 with two; r-z would spill: 129 x 97 step 1.7 us slower).
 template <class T, int S, bool CYL>
 __global__ void __launch_bounds__(kRtMaxThreads, sizeof(T) == 4 && !CYL ? 2 : 1) k_rt_init(LevelDev<T> F, LevelDev<T> C, T omega, RtInit I, NormState N,
-                                                           double tol2, int max_cycles, int decide,
-                                                           cudaGraphConditionalHandle cond, int use_cond) {
+                                                           double tol2, int max_cycles, int decide) {
     constexpr int HL = RtDown<S>::HL;
     static_assert(HL == RtUp<S, true>::HL, "the first residual's tiles are the residual up phase's");
     __shared__ RtShared<T> sh;
@@ -453,7 +494,7 @@ __global__ void __launch_bounds__(kRtMaxThreads, sizeof(T) == 4 && !CYL ? 2 : 1)
     rt_first_residual<T, HL, CYL>(I, F, i0, j0, cx, cy, t, sh64, r2, f2);
     rt_down_rest<T, S, CYL>(F, C, t, cf, sh, i0, j0, cx, cy, true, cfr);
     if (decide) {
-        norm_reduce_decide(r2, f2, N, tol2, max_cycles, 1, cond, use_cond);
+        norm_reduce_decide(r2, f2, N, tol2, max_cycles, 1, cudaGraphConditionalHandle{}, 0);
         return;
     }
     __shared__ double ws[kRtMaxWarps];
@@ -599,6 +640,18 @@ __device__ __forceinline__ bool rt_up_tile(const LevelDev<T>& F, const LevelDev<
     return true;
 }
 
+// The sum over the block's warps, in thread 0.
+__device__ __forceinline__ double rt_block_sum(double v) {
+    __shared__ double ws[kRtMaxWarps];
+    v = warp_sum(v);
+    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double s = 0.0;
+    if (threadIdx.x == 0)
+        for (int q = 0; q < rt_warps(); ++q) s += ws[q];
+    return s;
+}
+
 // The phase as a launch; RES: its norm and the loop decision too.
 template <class T, int S, bool CYL, int MODE>
 __global__ void __launch_bounds__(kRtMaxThreads, MODE == kRtResStaged ? 2 : 1) k_rt_up(LevelDev<T> F, LevelDev<T> C, T omega,
@@ -610,7 +663,11 @@ __global__ void __launch_bounds__(kRtMaxThreads, MODE == kRtResStaged ? 2 : 1) k
     if (!rt_up_tile<T, S, CYL, MODE>(F, C, omega, phi, R, blockIdx.x, blockIdx.y, sh, rt_stage, r2, RtLaunched{stop}))
         return;
     if constexpr (MODE != kRtUp) {
-        if (R.decide)
+        if (R.decide == 2) {
+            // the block's sum for rt_pending_stop
+            const double s = rt_block_sum(r2);
+            if (threadIdx.x == 0) R.N.partial[blockIdx.y * gridDim.x + blockIdx.x] = s;
+        } else if (R.decide)
             norm_reduce_decide(r2, 0.0, R.N, R.tol2, R.max_cycles, 0, R.cond, R.use_cond, R.inc, R.fblocks);
     }
 }
@@ -840,6 +897,7 @@ struct RtRest {
     DirectDesc<T> direct;
     int direct64;  // its inverse is FP64
     ResArgs res;
+    RtPending pending;
     double* phi;
     T omega;
     GridBar* bar;
@@ -869,14 +927,14 @@ __device__ __forceinline__ void rt_direct(const DirectDesc<T>& D, MT* gs) {
 
 template <class T, int S, bool CYL>
 __global__ void __launch_bounds__(kRtMaxThreads, 1) k_rt_rest(const __grid_constant__ RtRest<T> D) {
-    if (stopped(D.res.N.stop)) return;
+    double f2;
+    if (rt_pending_stop(D.pending, threadIdx.x == 0 && blockIdx.x == 0, f2)) return;
     __shared__ RtShared<T> sh;
     __shared__ double gs[kDirectMaxFree];
-    __shared__ double ws[kRtMaxWarps];
-    const int bid = int(blockIdx.x), nb = int(gridDim.x), w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    const int bid = int(blockIdx.x), nb = int(gridDim.x), l = threadIdx.x & 31;
     const NormState& N = D.res.N;
-    const int before = *N.cycles;
-    const double f2 = N.norms[0], lim = D.res.tol2 * (f2 > 0.0 ? f2 : 1.0);
+    const int before = D.pending.done;
+    const double lim = D.res.tol2 * (f2 > 0.0 ? f2 : 1.0);
     const int lsingle = D.fuse2 ? D.lc - 2 : D.lc;
     const RtInLoop go{};
     int seq = 0, n = 0;
@@ -920,19 +978,12 @@ __global__ void __launch_bounds__(kRtMaxThreads, 1) k_rt_rest(const __grid_const
         if (tile(D.lv[0], RtUp<S, true>::core(kRtCols), RtUp<S, true>::core(rt_side()), bx, by))
             rt_up_tile<T, S, CYL, kRtRes>(D.lv[0], D.lv[1], D.omega, D.phi, D.res, bx, by, sh, nullptr, r2, go);
         // the norm: the blocks' sums, added by every block in the same order
-        r2 = warp_sum(r2);
-        if (l == 0) ws[w] = r2;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double s = 0.0;
-            for (int q = 0; q < rt_warps(); ++q) s += ws[q];
-            N.partial[bid] = s;
-        }
+        r2 = rt_block_sum(r2);
+        if (threadIdx.x == 0) N.partial[bid] = r2;
         if (!barrier()) return;
         r2 = 0.0;
         for (int q = l; q < nb; q += 32) r2 += reinterpret_cast<const volatile double*>(N.partial)[q];
         r2 = warp_sum(r2);
-        r2 = __shfl_sync(0xffffffffu, r2, 0);
         ++n;
         conv = r2 < lim;
     } while (!conv && before + n < D.res.max_cycles);
@@ -950,8 +1001,7 @@ __global__ void __launch_bounds__(kRtMaxThreads, 1) k_rt_rest(const __grid_const
 template <class T>
 using RtUpKernel = void (*)(LevelDev<T>, LevelDev<T>, T, double*, ResArgs, const int*);
 template <class T>
-using RtInitKernel = void (*)(LevelDev<T>, LevelDev<T>, T, RtInit, NormState, double, int, int,
-                              cudaGraphConditionalHandle, int);
+using RtInitKernel = void (*)(LevelDev<T>, LevelDev<T>, T, RtInit, NormState, double, int, int);
 
 template <class T, bool CYL>
 static RtDownKernel<T> rt_down_kernel(int s) {

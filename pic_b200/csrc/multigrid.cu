@@ -108,9 +108,26 @@ struct ResArgs {
     int max_cycles;
     cudaGraphConditionalHandle cond;
     int use_cond;
-    int decide;   // 0: no norm and no decision after this cycle (register tiles)
+    int decide;   // 0: no norm and no decision after this cycle, 2: left to the next kernel (register tiles)
     int inc;      // cycles since the last decision
     int fblocks;  // the solve's first decision: blocks of ||f||^2 partials (NormState::fpart), else 0
+};
+
+// A loop decision left to the kernel after the cycle, on grids of few blocks: the
+// residual up phase only stores its blocks' sums, and the next cycle's finest
+// down phase (or k_rt_rest) adds them in every warp while its own loads are under
+// way.  The decision at the end of the up phase itself (norm_reduce_decide: a
+// fence behind its stores, a counter, the last block's second pass) costs that
+// phase 2.8 us at 129 x 97 (6.1 us against 3.3).
+constexpr int kRtPendingMax = 160;  // blocks
+struct RtPending {
+    NormState N;
+    double tol2;
+    int max_cycles;
+    int nb;       // blocks' sums of r^2; 0: nothing is pending
+    int fblocks;  // the solve's first decision: blocks' sums of f^2, else 0
+    int inc;      // cycles since the last decision
+    int done;     // cycles of the solve so far, where it has not stopped
 };
 
 // The levels as a launch mode uses them: up phases on the levels below
@@ -843,7 +860,7 @@ static UpResKernel<T> up_res_kernel(int s) {
 template <class T>
 using Fused2Kernel = void (*)(LevelDev<T>, LevelDev<T>, LevelDev<T>, T);
 template <class T>
-using RtDownKernel = void (*)(LevelDev<T>, LevelDev<T>, T, const double*, const int*);
+using RtDownKernel = void (*)(LevelDev<T>, LevelDev<T>, T, const double*, const int*, RtPending);
 template <class T>
 using RtFused2Kernel = void (*)(LevelDev<T>, LevelDev<T>, LevelDev<T>, T, const int*);
 
@@ -2397,6 +2414,8 @@ struct CycleOpts {
     int fblocks = 0;            // this is the solve's first decision, after a first residual of so many blocks
     const RtInit* init = nullptr;  // the solve's first cycle: its finest down phase forms the first residual ...
     bool init_decide = false;      // ... and takes the first decision
+    bool defer = false;            // the decision is left to the kernel after the cycle ...
+    RtPending pending{};           // ... as the one before this cycle was (nb > 0)
 };
 
 // Whether a cycle runs on register tiles throughout, with the direct solve.
@@ -2438,8 +2457,7 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
         if (l == 0 && O.init) {
             const RtShape h = rt_up_shape(pre, lv[0].nx, lv[0].ny, true);
             launch_pdl(M.rz ? rt_init_kernel<T, true>(pre) : rt_init_kernel<T, false>(pre), h.grid, dim3(h.threads), 0,
-                       st, lv[0], lv[1], omega, *O.init, M.N, tol * tol, max_cycles, int(O.init_decide), cond,
-                       int(use_cond && O.init_decide));
+                       st, lv[0], lv[1], omega, *O.init, M.N, tol * tol, max_cycles, int(O.init_decide));
         } else if (rtd) {
             // the finest down phase waits for its predecessor to finish before
             // it is placed: launched ahead, its blocks take the SMs the
@@ -2447,8 +2465,8 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
             // 1009 us launched ahead, 942 us this way; 129^2 the same)
             const RtDownKernel<T> kdown = M.rz ? rt_down_kernel<T, true>(pre) : rt_down_kernel<T, false>(pre);
             const RtShape h = rt_down_shape(pre, lv[l].nx, lv[l].ny);
-            if (l == 0) kdown<<<h.grid, h.threads, 0, st>>>(lv[0], lv[1], omega, g64, O.stop);
-            else launch_pdl(kdown, h.grid, dim3(h.threads), 0, st, lv[l], lv[l + 1], omega, g64, O.stop);
+            if (l == 0) kdown<<<h.grid, h.threads, 0, st>>>(lv[0], lv[1], omega, g64, O.stop, O.pending);
+            else launch_pdl(kdown, h.grid, dim3(h.threads), 0, st, lv[l], lv[l + 1], omega, g64, O.stop, RtPending{});
         } else {
             const DownKernel<T> kdown = M.rz ? down_kernel<T, true>(pre) : down_kernel<T, false>(pre);
             const RtShape h = tiles(l);
@@ -2519,7 +2537,7 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
         R.max_cycles = max_cycles;
         R.cond = cond;
         R.use_cond = use_cond;
-        R.decide = O.decide ? 1 : 0;
+        R.decide = O.decide ? (O.defer ? 2 : 1) : 0;
         R.inc = O.inc;
         R.fblocks = O.fblocks;
         const RtShape h = rtu ? rt_up_shape(post, lv[0].nx, lv[0].ny, true) : tiles(0);
@@ -2541,7 +2559,9 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
 // The first cycles of a register-tile solve as plain launches.  The first
 // cycle's finest down phase forms the first residual (no launch of its own).
 // The first min_cycles cycles always run, and the ones before the last of them
-// end without a norm; the others do nothing once the solve has stopped.
+// end without a norm; the others do nothing once the solve has stopped.  rest:
+// a launch of k_rt_rest follows, which takes the last cycle's decision (there
+// are never more than kRtPendingMax blocks then).
 // How many (first_cycles): what the solve is expected to need.  A cycle divides
 // the residual by about 100 where all Dirichlet nodes are on the edges (r-z
 // sometimes takes one more).  A step's guess (min_cycles > 0), extrapolated from
@@ -2564,10 +2584,14 @@ static int first_cycles(int max_cycles, int min_cycles, double tol) {
 template <class T>
 static int launch_first_cycles(MgImpl& M, std::vector<LevelDev<T>>& lv, double* phi, const double* f, double tol,
                                int max_cycles, int min_cycles, cudaGraphConditionalHandle cond, int use_cond,
-                               cudaStream_t st) {
+                               cudaStream_t st, RtPending* rest = nullptr) {
     const int kmin = std::max(0, std::min(min_cycles, max_cycles)), K = first_cycles(max_cycles, kmin, tol);
     const RtInit init{phi, f, M.rz0, M.r64, 1.0 / (M.dx * M.dx), 1.0 / (M.dy * M.dy)};
     const RtShape h0 = rt_up_shape(M.o.pre_sweeps, M.nx, M.ny, true);
+    const RtShape h1 = rt_up_shape(M.o.post_sweeps, M.nx, M.ny, true);
+    const int b0 = int(h0.grid.x * h0.grid.y), b1 = int(h1.grid.x * h1.grid.y);
+    const bool defer = std::max(b0, b1) <= kRtPendingMax;
+    RtPending pending{};
     int last = 0;  // cycles finished at the last decision
     for (int k = 0; k < K; ++k) {
         CycleOpts O;
@@ -2579,13 +2603,19 @@ static int launch_first_cycles(MgImpl& M, std::vector<LevelDev<T>>& lv, double* 
         O.decide = k + 1 >= kmin;
         if (O.decide) {
             O.inc = k + 1 - last;
-            O.fblocks = last == 0 && kmin > 0 ? int(h0.grid.x * h0.grid.y) : 0;
+            O.fblocks = last == 0 && kmin > 0 ? b0 : 0;
             last = k + 1;
         }
+        O.pending = pending;
+        O.defer = defer && O.decide && (k + 1 < K || rest);
+        pending = O.defer ? RtPending{M.N, tol * tol, max_cycles, b1, O.fblocks, O.inc, k + 1} : RtPending{};
         int count = 0;
-        PIC_TRY(launch_cycle(M, lv, phi, f, tol, max_cycles, cond, use_cond, st, count, O));
+        // the last cycle's decision alone sets the loop's condition: it is 0 until
+        // then, and a solve that stops earlier does not reach it
+        PIC_TRY(launch_cycle(M, lv, phi, f, tol, max_cycles, cond, use_cond && k + 1 == K, st, count, O));
         M.body_launches = count;
     }
+    if (rest) *rest = pending;
     return PIC_OK;
 }
 
@@ -2621,7 +2651,7 @@ static int rest_blocks(const MgImpl& M, const std::vector<LevelDev<T>>& lv) {
 
 template <class T>
 static int launch_rest(MgImpl& M, const std::vector<LevelDev<T>>& lv_in, double* phi, double tol, int max_cycles,
-                       int blocks, cudaStream_t st) {
+                       int blocks, const RtPending& pending, cudaStream_t st) {
     const std::vector<LevelDev<T>> lv = with_corrections(lv_in, M.Lc);
     RtRest<T> D{};
     D.lc = M.Lc;
@@ -2636,6 +2666,7 @@ static int launch_rest(MgImpl& M, const std::vector<LevelDev<T>>& lv_in, double*
     D.res.N = M.N;
     D.res.tol2 = tol * tol;
     D.res.max_cycles = max_cycles;
+    D.pending = pending;
     D.phi = phi;
     D.omega = T(M.o.omega);
     D.bar = M.bar;
@@ -2674,8 +2705,11 @@ static int capture_solve(MgImpl& M, std::vector<LevelDev<T>>& lv, double* phi, c
     if (rt && first_cycles(max_cycles, min_cycles, tol) >= max_cycles)  // no loop left
         return launch_first_cycles(M, lv, phi, f, tol, max_cycles, min_cycles, cudaGraphConditionalHandle{}, 0, st);
     if (const int blocks = rt && alone ? rest_blocks(M, lv) : 0) {
-        PIC_TRY(launch_first_cycles(M, lv, phi, f, tol, max_cycles, min_cycles, cudaGraphConditionalHandle{}, 0, st));
-        return launch_rest(M, lv, phi, tol, max_cycles, blocks, st);
+        RtPending pending{};
+        PIC_TRY(launch_first_cycles(M, lv, phi, f, tol, max_cycles, min_cycles, cudaGraphConditionalHandle{}, 0, st,
+                                    &pending));
+        if (!pending.nb) return fail(PIC_ERR_CUDA, "multigrid: no decision left for the cycles after the launched ones");
+        return launch_rest(M, lv, phi, tol, max_cycles, blocks, pending, st);
     }
     cudaGraphConditionalHandle h;
     PIC_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
