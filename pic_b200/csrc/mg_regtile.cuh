@@ -80,23 +80,15 @@ __device__ __forceinline__ unsigned rt_free_bits(const uint32_t* __restrict__ fb
     return __funnelshift_r(lo, hi, unsigned(j & 31)) & mask;
 }
 
-// The coefficients of an over-relaxed Gauss-Seidel update
-//   e <- q e + a (w + e) + bs s + bn n - k g
-// (e + omega (upd - e) with upd = (cx (w + e) + wS s + wN n - g) / diag).
-template <class T>
-struct RtRow {
-    T a, bs, bn, k;
-};
-
-// r-z rows keep {wN, wS, 1/diag, D} in registers; Cartesian rows share one set.
+// The coefficients of an update; r-z rows keep {wN, wS, 1/diag, D} in registers.
 template <class T, int ROWS, bool CYL>
 struct RtCoef {
-    T cx, cy, omega;
-    RtRow<T> c;             // Cartesian
+    T cx, cy, inv_diag, omega;
     T rz[CYL ? ROWS : 1][4];
     __device__ __forceinline__ void load(const LevelDev<T>& L, T om, int j0) {
         cx = L.cx;
         cy = L.cy;
+        inv_diag = L.inv_diag;
         omega = om;
         if constexpr (CYL) {
 #pragma unroll
@@ -106,19 +98,12 @@ struct RtCoef {
 #pragma unroll
                 for (int q = 0; q < 4; ++q) rz[r][q] = in ? __ldg(L.rz + 4 * j + q) : T(0);
             }
-        } else {
-            c.k = om * L.inv_diag;
-            c.a = c.k * L.cx;
-            c.bs = c.bn = c.k * L.cy;
         }
     }
-    __device__ __forceinline__ RtRow<T> row(int r) const {
-        if constexpr (CYL) {
-            const T k = omega * rz[r][2];
-            return RtRow<T>{k * cx, k * rz[r][1], k * rz[r][0], k};
-        } else {
-            return c;
-        }
+    // The over-relaxed value of a node of row r (relaxed, relaxed_rz).
+    __device__ __forceinline__ T update(int r, T old, T ew, T s, T n, T g) const {
+        if constexpr (CYL) return relaxed_rz(old, ew, s, n, g, cx, rz[r][0], rz[r][1], rz[r][2], omega);
+        else return relaxed(old, ew, s, n, g, cx, cy, inv_diag, omega);
     }
 };
 
@@ -154,18 +139,13 @@ __device__ __forceinline__ void rt_exchange(RtTile<T>& t, RtShared<T>& s, int& b
 // One half-sweep (COLOR 0: red, (i + j) even).
 template <class T, int COLOR, bool CYL>
 __device__ __forceinline__ void rt_half_sweep(RtTile<T>& t, const RtCoef<T, kRtRows, CYL>& cf) {
-    const T q = T(1) - cf.omega;
 #pragma unroll
     for (int r = 0; r < kRtRows; ++r) {
         const int c = (r + COLOR) & 1;
-        const RtRow<T> k = cf.row(r);
         const T side = c ? __shfl_down_sync(0xffffffffu, t.e[r][0], 1) : __shfl_up_sync(0xffffffffu, t.e[r][1], 1);
         const T s = r > 0 ? t.e[r - 1][c] : t.up[c];
         const T n = r < kRtRows - 1 ? t.e[r + 1][c] : t.dn[c];
-        T v = q * t.e[r][c] - k.k * t.g[r][c];
-        v += k.a * (side + t.e[r][1 - c]);
-        if constexpr (CYL) v += k.bs * s + k.bn * n;
-        else v += k.bs * (s + n);
+        const T v = cf.update(r, t.e[r][c], side + t.e[r][1 - c], s, n, t.g[r][c]);
         if ((t.fr[c] >> r) & 1u) t.e[r][c] = v;
     }
 }
@@ -185,7 +165,7 @@ __device__ __forceinline__ void rt_sweeps(RtTile<T>& t, const RtCoef<T, kRtRows,
 #pragma unroll
             for (int r = 0; r < kRtRows; ++r) {
                 const int c = r & 1;
-                t.e[r][c] = ((t.fr[c] >> r) & 1u) ? -(cf.row(r).k * t.g[r][c]) : T(0);
+                t.e[r][c] = ((t.fr[c] >> r) & 1u) ? cf.update(r, T(0), T(0), T(0), T(0), t.g[r][c]) : T(0);
                 t.e[r][1 - c] = T(0);
             }
         } else {
@@ -198,14 +178,12 @@ __device__ __forceinline__ void rt_sweeps(RtTile<T>& t, const RtCoef<T, kRtRows,
 }
 
 // The residual g - A e of the region, 0 on Dirichlet nodes (r-z: weighted by
-// the row's volume), returned as its horizontal full weighting at the even
-// columns, h = r/2 + (r_west + r_east)/4.
+// the row's volume).
 template <class T, bool CYL>
-__device__ __forceinline__ void rt_residual_h(const RtTile<T>& t, const RtCoef<T, kRtRows, CYL>& cf,
-                                              T (&h)[kRtRows]) {
+__device__ __forceinline__ void rt_residual(const RtTile<T>& t, const RtCoef<T, kRtRows, CYL>& cf,
+                                            T (&res)[kRtRows][2]) {
 #pragma unroll
     for (int r = 0; r < kRtRows; ++r) {
-        T res[2];
         const T w = __shfl_up_sync(0xffffffffu, t.e[r][1], 1), ea = __shfl_down_sync(0xffffffffu, t.e[r][0], 1);
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
@@ -218,31 +196,54 @@ __device__ __forceinline__ void rt_residual_h(const RtTile<T>& t, const RtCoef<T
                 const T lap = cf.cx * (wv + ev - T(2) * e) + cf.rz[r][0] * (n - e) + cf.rz[r][1] * (s - e);
                 v = cf.rz[r][3] * (t.g[r][c] - lap);
             } else {
-                v = t.g[r][c] - (cf.cx * (wv + ev - T(2) * e) + cf.cy * (s + n - T(2) * e));
+                v = t.g[r][c] - weighted(cf.cx, wv + ev - T(2) * e, cf.cy, s + n - T(2) * e);
             }
-            res[c] = ((t.fr[c] >> r) & 1u) ? v : T(0);
+            res[r][c] = ((t.fr[c] >> r) & 1u) ? v : T(0);
         }
-        const T rw = __shfl_up_sync(0xffffffffu, res[1], 1);
-        h[r] = T(0.5) * res[0] + T(0.25) * (rw + res[1]);
     }
 }
 
-// Full weighting of the coarse rows of this warp (the fine rows 0 and 2) from
-// the horizontal weights; J0: the coarse row of fine row 0.
+// The full weighting of a coarse node from its fine row {west, centre, east}
+// and the rows below and above, in restrict_fw's order.
+template <class T>
+struct RtRow3 {
+    T w, c, e;
+};
+template <class T>
+__device__ __forceinline__ T rt_weight(const RtRow3<T>& s, const RtRow3<T>& m, const RtRow3<T>& n) {
+    T v = T(0.25) * m.c;
+    v += T(0.125) * (m.w + m.e + s.c + n.c);
+    v += T(0.0625) * (s.w + s.e + n.w + n.e);
+    return v;
+}
+
+// Full weighting of the coarse rows of this warp (the fine rows 0 and 2) at
+// the even columns; J0: the coarse row of fine row 0.
 template <class T, bool CYL>
-__device__ __forceinline__ void rt_restrict(const T (&h)[kRtRows], RtShared<T>& sh, int& buf, int J0, T (&out)[kRtRows / 2]) {
+__device__ __forceinline__ void rt_restrict(const T (&res)[kRtRows][2], RtShared<T>& sh, int& buf, int J0,
+                                            T (&out)[kRtRows / 2]) {
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    sh.x[buf][w][1][l] = h[kRtRows - 1];
+    sh.x[buf][w][0][l] = res[kRtRows - 1][0];
+    sh.x[buf][w][1][l] = res[kRtRows - 1][1];
     __syncthreads();
-    const T above = w > 0 ? sh.x[buf][w - 1][1][l] : T(0);
+    RtRow3<T> below{T(0), T(0), T(0)};
+    if (w > 0) {
+        below.c = sh.x[buf][w - 1][0][l];
+        below.e = sh.x[buf][w - 1][1][l];
+        below.w = sh.x[buf][w - 1][1][max(l - 1, 0)];
+    }
     buf ^= 1;
 #pragma unroll
     for (int q = 0; q < kRtRows / 2; ++q) {
-        const T s = q > 0 ? h[2 * q - 1] : above;
-        T v = T(0.5) * h[2 * q] + T(0.25) * (s + h[2 * q + 1]);
+        auto row = [&](int r) {
+            return RtRow3<T>{__shfl_up_sync(0xffffffffu, res[r][1], 1), res[r][0], res[r][1]};
+        };
+        const RtRow3<T> above = row(2 * q + 1);
+        T v = rt_weight(below, row(2 * q), above);
         // r-z: divided by the stencil's weighted volume (2J; 5/16 on the axis)
         if constexpr (CYL) v *= J0 + q == 0 ? T(3.2) : T(0.5) / T(J0 + q);
         out[q] = v;
+        below = above;
     }
 }
 
@@ -425,9 +426,9 @@ __device__ __forceinline__ void rt_down_rest(const LevelDev<T>& F, const LevelDe
     rt_sweeps<T, S, CYL, true, true>(t, cf, sh, buf);
     rt_store_core<T, HL>(F.e, t.e, F.nx, F.ny, i0, j0, cx, cy);
     if (store_g) rt_store_core<T, HL>(F.g, t.g, F.nx, F.ny, i0, j0, cx, cy);
-    T h[kRtRows], out[kRtRows / 2];
-    rt_residual_h<T, CYL>(t, cf, h);
-    rt_restrict<T, CYL>(h, sh, buf, J0, out);
+    T res[kRtRows][2], out[kRtRows / 2];
+    rt_residual<T, CYL>(t, cf, res);
+    rt_restrict<T, CYL>(res, sh, buf, J0, out);
     if (2 * l < HL || 2 * l >= HL + cx || I >= C.nx) return;
 #pragma unroll
     for (int q = 0; q < kRtRows / 2; ++q) {
@@ -702,20 +703,16 @@ __device__ __forceinline__ void rt_c_exchange(RtCTile<T>& t, RtShared<T>& s, int
 template <class T, bool CYL>
 __device__ __forceinline__ void rt_c_half_sweep(RtCTile<T>& t, const RtCoef<T, kRtCRows, CYL>& cf, int color) {
     const bool odd = ((threadIdx.x + color) & 1) != 0;  // which of its rows this lane updates
-    const T q = T(1) - cf.omega;
     // the neighbouring lanes update the other row: they send this lane's
     const T send = odd ? t.e[0] : t.e[1];
     const T wv = __shfl_up_sync(0xffffffffu, send, 1), ev = __shfl_down_sync(0xffffffffu, send, 1);
     const T s = odd ? t.e[0] : t.up, n = odd ? t.dn : t.e[1];
     const T old = odd ? t.e[1] : t.e[0], g = odd ? t.g[1] : t.g[0];
     T v;
-    if constexpr (CYL) {
-        const RtRow<T> ka = cf.row(0), kb = cf.row(1);
-        const T kk = odd ? kb.k : ka.k, bs = odd ? kb.bs : ka.bs, bn = odd ? kb.bn : ka.bn;
-        v = q * old - kk * g + (kk * cf.cx) * (wv + ev) + (bs * s + bn * n);
-    } else {
-        v = q * old - cf.c.k * g + cf.c.a * (wv + ev) + cf.c.bs * (s + n);
-    }
+    if constexpr (CYL)
+        v = relaxed_rz(old, wv + ev, s, n, g, cf.cx, odd ? cf.rz[1][0] : cf.rz[0][0], odd ? cf.rz[1][1] : cf.rz[0][1],
+                       odd ? cf.rz[1][2] : cf.rz[0][2], cf.omega);
+    else v = cf.update(0, old, wv + ev, s, n, g);
     if (!odd && (t.fr & 1u)) t.e[0] = v;
     if (odd && (t.fr & 2u)) t.e[1] = v;
 }
@@ -757,9 +754,9 @@ __device__ __forceinline__ void rt_down2_tile(const LevelDev<T>& F, const LevelD
     int buf = 0;
     rt_sweeps<T, S, CYL, true, true>(t, cf, sh, buf);
     rt_store_core<T, G::HL>(F.e, t.e, F.nx, F.ny, i0, j0, cx, cy);
-    T h[kRtRows], out[kRtCRows];
-    rt_residual_h<T, CYL>(t, cf, h);
-    rt_restrict<T, CYL>(h, sh, buf, J0, out);
+    T res[kRtRows][2], out[kRtCRows];
+    rt_residual<T, CYL>(t, cf, res);
+    rt_restrict<T, CYL>(res, sh, buf, J0, out);
 #pragma unroll
     for (int q = 0; q < kRtCRows; ++q) {
         ct.g[q] = ((ct.fr >> q) & 1u) ? out[q] : T(0);
@@ -776,8 +773,8 @@ __device__ __forceinline__ void rt_down2_tile(const LevelDev<T>& F, const LevelD
         C.e[K] = ct.e[q];
         C.g[K] = ct.g[q];
     }
-    // C's residual, weighted along the row at the even columns (even lanes)
-    T hc[kRtCRows];
+    // C's residual
+    RtRow3<T> rc[kRtCRows];
 #pragma unroll
     for (int q = 0; q < kRtCRows; ++q) {
         const T e = ct.e[q];
@@ -788,20 +785,23 @@ __device__ __forceinline__ void rt_down2_tile(const LevelDev<T>& F, const LevelD
             const T lap = cc.cx * (wv + ev - T(2) * e) + cc.rz[q][0] * (n - e) + cc.rz[q][1] * (s - e);
             v = cc.rz[q][3] * (ct.g[q] - lap);
         } else {
-            v = ct.g[q] - (cc.cx * (wv + ev - T(2) * e) + cc.cy * (s + n - T(2) * e));
+            v = ct.g[q] - weighted(cc.cx, wv + ev - T(2) * e, cc.cy, s + n - T(2) * e);
         }
         const T r = ((ct.fr >> q) & 1u) ? v : T(0);
-        const T rw = __shfl_up_sync(0xffffffffu, r, 1), re = __shfl_down_sync(0xffffffffu, r, 1);
-        hc[q] = T(0.5) * r + T(0.25) * (rw + re);
+        rc[q] = RtRow3<T>{__shfl_up_sync(0xffffffffu, r, 1), r, __shfl_down_sync(0xffffffffu, r, 1)};
     }
-    sh.x[buf][w][1][l] = hc[1];
+    sh.x[buf][w][1][l] = rc[1].c;
     __syncthreads();
-    const T above = w > 0 ? sh.x[buf][w - 1][1][l] : T(0);
+    RtRow3<T> below{T(0), T(0), T(0)};
+    if (w > 0) {
+        const T* x = sh.x[buf][w - 1][1];
+        below = RtRow3<T>{x[max(l - 1, 0)], x[l], x[min(l + 1, 31)]};
+    }
     buf ^= 1;
     // one C2 row per warp, on the even lanes
     const int I2 = I >> 1, J2 = J0 >> 1, lr = w * kRtRows;
     if ((l & 1) || !ccol || I2 >= C2.nx || lr < G::HL || lr >= G::HL + cy || J2 >= C2.ny) return;
-    T v = T(0.5) * hc[0] + T(0.25) * (above + hc[1]);
+    T v = rt_weight(below, rc[0], rc[1]);
     if constexpr (CYL) v *= J2 == 0 ? T(3.2) : T(0.5) / T(J2);
     C2.g[long(J2) * C2.nx + I2] = (c2fr & 1u) ? v : T(0);
 }
@@ -842,20 +842,19 @@ __device__ __forceinline__ void rt_up2_tile(const LevelDev<T>& F, const LevelDev
         // C2's correction prolonged onto C: an odd column takes the mean of
         // its own C2 column and the next lane's
         const int I2 = I >> 1, J2 = J0 >> 1;
-        T v2[2];
+        T v2[2], e2[2];
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
             const int J = J2 + q;
             const bool in = J >= 0 && J < C2.ny && I2 >= 0 && I2 < C2.nx;
-            const T v = in ? C2.ec[long(J) * C2.nx + I2] : T(0);
-            const T e = __shfl_down_sync(0xffffffffu, v, 1);
-            v2[q] = (l & 1) ? T(0.5) * (v + e) : v;
+            v2[q] = in ? C2.ec[long(J) * C2.nx + I2] : T(0);
+            e2[q] = __shfl_down_sync(0xffffffffu, v2[q], 1);
         }
+        const bool odd = (l & 1) != 0;
+        const T v[kRtCRows] = {odd ? T(0.5) * (v2[0] + e2[0]) : v2[0],
+                               odd ? T(0.25) * (v2[0] + e2[0] + v2[1] + e2[1]) : T(0.5) * (v2[0] + v2[1])};
 #pragma unroll
-        for (int q = 0; q < kRtCRows; ++q) {
-            const T v = q ? T(0.5) * (v2[0] + v2[1]) : v2[0];
-            ct.e[q] = ((ct.fr >> q) & 1u) ? ct.e[q] + v : T(0);
-        }
+        for (int q = 0; q < kRtCRows; ++q) ct.e[q] = ((ct.fr >> q) & 1u) ? ct.e[q] + v[q] : T(0);
     }
     if (sync.done()) return;
     int buf = 0;

