@@ -24,7 +24,6 @@
 #include <algorithm>
 #include <climits>
 #include <cmath>
-#include <cstdlib>
 #include <cstddef>
 #include <vector>
 
@@ -1887,8 +1886,7 @@ static int run_pass(SimImpl& S, cudaStream_t st, int kick, int mcc, int drift, i
             if (full) k_push<true, true><<<S.push_grid, kPushThreads, S.push_smem, st>>>(A);
             else k_push<true, false><<<S.push_grid, kPushThreads, S.push_smem, st>>>(A);
         } else {
-            const int eg = S.in_ensemble && getenv("T_G") ? std::min(S.push_grid, atoi(getenv("T_G"))) : S.push_grid;
-            if (full) k_push<false, true><<<eg, kPushThreads, S.push_smem, st>>>(A);
+            if (full) k_push<false, true><<<S.push_grid, kPushThreads, S.push_smem, st>>>(A);
             else k_push<false, false><<<S.push_grid, kPushThreads, S.push_smem, st>>>(A);
         }
     }
