@@ -1800,6 +1800,7 @@ struct MgImpl {
     int Lp = 0;
     size_t solve_smem = 0;
     int solve_grid = 0;
+    int partials = 0;  // blocks that NormState::partial holds sums for
     // cluster-resident solve
     bool cluster_ok = false;
     int cluster_size = 0;
@@ -2382,10 +2383,10 @@ int mg_create(int nx, int ny, double dx, double dy, const uint8_t* h_mask, const
     if (st != PIC_OK) return bail(st);
     M.grd0 = dim3(div_up(nx, M.blk0.x), div_up(ny, M.blk0.y * kR0Rows));
     // block partials of the residual norm: one pair per block of the level-0
-    // tiling (k_mg_r0, k_mg_up_res) or of the persistent grid (k_mg_solve),
-    // whichever is larger
-    const int nb = std::max(std::max(int(M.grd0.x * M.grd0.y), div_up(nx, 16) * div_up(ny, 16)),
-                            M.solve_grid);
+    // tiling (k_mg_r0, k_mg_up_res, k_rt_up), of the persistent grid (k_mg_solve)
+    // or of k_rt_rest (rest_blocks: at most one block per SM), whichever is largest
+    const int nb = std::max({int(M.grd0.x * M.grd0.y), div_up(nx, 16) * div_up(ny, 16), M.solve_grid, num_sms()});
+    M.partials = nb;
     if (cudaMalloc(&M.N.partial, sizeof(double) * 2 * nb) != cudaSuccess)
         return bail(fail(PIC_ERR_CUDA, "pic_mg_create: out of device memory"));
     M.allocs.push_back(M.N.partial);
@@ -2677,6 +2678,8 @@ static int rest_blocks(const MgImpl& M, const std::vector<LevelDev<T>>& lv) {
 template <class T>
 static int launch_rest(MgImpl& M, const std::vector<LevelDev<T>>& lv_in, double* phi, double tol, int max_cycles,
                        int blocks, const RtPending& pending, cudaStream_t st) {
+    if (blocks > M.partials)
+        return fail(PIC_ERR_CUDA, "multigrid: %d blocks and room for the sums of %d", blocks, M.partials);
     const std::vector<LevelDev<T>> lv = with_corrections(lv_in, M.Lc);
     RtRest<T> D{};
     D.lc = M.Lc;
