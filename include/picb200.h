@@ -216,12 +216,13 @@ int pic_mg_read_info(pic_mg* mg, double tol, pic_mg_info* info);
 /* The launch mode solves actually use (PIC_MG_CLUSTER falls back to
  * PIC_MG_GRAPH_LOOP where the cluster solve does not apply). */
 int pic_mg_effective_launch_mode(pic_mg* mg, int* mode);
-/* Failure detection of the persistent solve (PIC_MG_PERSISTENT; the
- * reference's host loop, src/multigrid.py:445-455, has no device wait to
- * bound): polls a grid barrier makes before the solve gives up, sets a device
- * error flag and returns, and the solve returns PIC_ERR_TIMEOUT (the flag is
- * then cleared and the solver stays usable).  polls < 0 restores the default
- * (2^24 polls, about a second). */
+/* Failure detection of the cooperative launches (PIC_MG_PERSISTENT, and the
+ * cycles a simulation's or an adjoint problem's solve needs past those it
+ * launches in line; the reference's host loop, src/multigrid.py:445-455, has no
+ * device wait to bound): polls a grid barrier makes before the solve gives up,
+ * sets a device error flag and returns, and the solve returns PIC_ERR_TIMEOUT
+ * (the flag is then cleared and the solver stays usable).  polls < 0 restores
+ * the default (2^24 polls, about a second). */
 int pic_mg_set_wait_limit(pic_mg* mg, long long polls);
 /* The shared-memory tile geometry the multigrid's tile kernels use for
  * `sweeps` red-black sweeps (1..8), in nodes, as PIC_MG_GEOMETRY_VALUES ints:

@@ -928,6 +928,9 @@ template <class T, int S, bool CYL>
 __global__ void __launch_bounds__(kRtMaxThreads, 1) k_rt_rest(const __grid_constant__ RtRest<T> D) {
     double f2;
     if (rt_pending_stop(D.pending, threadIdx.x == 0 && blockIdx.x == 0, f2)) return;
+    // after a barrier that gave up its counter is not in order: nothing runs in
+    // here, and solves end unconverged, until the host has read the error
+    if (*reinterpret_cast<const volatile int*>(D.error)) return;
     __shared__ RtShared<T> sh;
     __shared__ double gs[kDirectMaxFree];
     const int bid = int(blockIdx.x), nb = int(gridDim.x), l = threadIdx.x & 31;

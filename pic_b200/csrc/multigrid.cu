@@ -1807,7 +1807,7 @@ struct MgImpl {
     size_t cluster_smem = 0;
     GridBar* bar = nullptr;
     int* error = nullptr;
-    unsigned long long wait_polls = kBarrierPolls;  // grid-barrier wait limit of the persistent solve
+    unsigned long long wait_polls = kBarrierPolls;  // grid-barrier wait limit of the cooperative launches
     cudaStream_t side = nullptr;
     cudaStream_t cap = nullptr;
     // cached solve graphs: [0] on the first pair of buffers a solve was given
@@ -2699,7 +2699,7 @@ static int launch_rest(MgImpl& M, const std::vector<LevelDev<T>>& lv_in, double*
     D.omega = T(M.o.omega);
     D.bar = M.bar;
     D.error = M.error;
-    D.polls = kBarrierPolls;
+    D.polls = M.wait_polls;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(blocks);
     cfg.blockDim = dim3(kRtMaxThreads);
@@ -2973,7 +2973,7 @@ int mg_read_info(MgImpl& M, pic_mg_info* info) {
         PIC_CUDA(cudaMemset(M.bar, 0, sizeof(GridBar)));
         PIC_CUDA(cudaMemset(M.error, 0, 6 * sizeof(int)));
         return fail(PIC_ERR_TIMEOUT,
-                    "multigrid: grid barrier %d of the persistent solve timed out (block %d saw count %d, "
+                    "multigrid: grid barrier %d of a cooperative launch timed out (block %d saw count %d, "
                     "generation %d, waited on %d)",
                     err[1], err[2], err[3], err[4], err[5]);
     }
@@ -3149,6 +3149,11 @@ int pic_mg_set_wait_limit(pic_mg* mg, long long polls) {
     clear_error();
     if (!mg) return fail(PIC_ERR_BAD_ARG, "pic_mg_set_wait_limit: mg is NULL");
     mg->m.wait_polls = polls < 0 ? kBarrierPolls : (unsigned long long)polls;
+    // cached graphs hold the old limit in their kernels' arguments
+    for (auto& g : mg->m.graph) {
+        if (g.exec) PIC_CUDA(cudaGraphExecDestroy(g.exec));
+        g.exec = nullptr;
+    }
     return PIC_OK;
 }
 

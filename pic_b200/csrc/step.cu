@@ -2753,8 +2753,10 @@ int pic_sim_read_counters(pic_sim* sim, pic_sim_counters* out, void* stream) {
     PIC_CUDA(cudaMemcpy(&err, S.error, sizeof err, cudaMemcpyDeviceToHost));
     if (err) {
         PIC_CUDA(cudaMemset(S.error, 0, sizeof err));
-        return fail(PIC_ERR_TIMEOUT, "particle pass: a wait on a bulk copy into shared memory gave up after %llu polls",
-                    S.wait_limit);
+        // one report for all that the limit cut short: the field solve's barriers are cleared with it
+        const bool solve = mg_info(S.mg, &S.last) == PIC_ERR_TIMEOUT;
+        return fail(PIC_ERR_TIMEOUT, "particle pass: a wait on a bulk copy into shared memory gave up after %llu polls%s",
+                    S.wait_limit, solve ? "; so did a grid barrier of the field solve" : "");
     }
     unsigned long long c[kCtrCount];
     PIC_CUDA(cudaMemcpy(c, S.ctr, sizeof c, cudaMemcpyDeviceToHost));
@@ -2785,7 +2787,7 @@ int pic_sim_set_wait_limit(pic_sim* sim, long long polls) {
     SimImpl& S = sim->s;
     PIC_CUDA(cudaDeviceSynchronize());
     S.wait_limit = polls < 0 ? kWaitLimit : (unsigned long long)polls;
-    PIC_TRY(pic_mg_set_wait_limit(S.mg, polls));  // the persistent solve's grid barriers
+    PIC_TRY(pic_mg_set_wait_limit(S.mg, polls));  // the field solve's grid barriers
     // the captured steps hold the old limits in their kernel arguments
     if (S.g_step) cudaGraphExecDestroy(S.g_step);
     if (S.g_sort_step) cudaGraphExecDestroy(S.g_sort_step);

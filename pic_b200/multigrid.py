@@ -66,7 +66,7 @@ class MultigridSolver:
         return {v: k for k, v in _lib.MG_LAUNCH_MODES.items()}[m.value]
 
     def set_wait_limit(self, polls=-1):
-        """Polls a grid barrier of the persistent solve makes before the solve
+        """Polls a grid barrier of a cooperative launch makes before the solve
         gives up with PIC_ERR_TIMEOUT (raised as PicError); -1 restores the default."""
         _lib.call("pic_mg_set_wait_limit", self._h, int(polls))
 

@@ -243,7 +243,7 @@ class PICSimulation:
 
     def set_wait_limit(self, polls=-1):
         """Polls a bounded device wait (the particle pass's bulk copies, the
-        persistent solve's grid barriers) makes before it gives up; the next
+        field solve's grid barriers) makes before it gives up; the next
         counters() raises PicError(PIC_ERR_TIMEOUT).  -1 restores the default."""
         _lib.call("pic_sim_set_wait_limit", self._h, int(polls))
 

@@ -14,14 +14,24 @@ Tolerance: both residuals at FP64's floor, 1e-9 of ||f|| (a V-cycle divides the 
 """
 import numpy as np
 import pytest
+import torch
 
-from pic_b200 import Consts
+from pic_b200 import Consts, _lib
 from pic_b200.simulation import PICSimulation
 
 DX, CYCLES = 1e-4, 12
 
 
-def make(nx, ny, rz, precision="mixed", sweeps=2, seed=1, **options):
+def load(sim):
+    rng = np.random.default_rng(1)
+    n = sim.species[0]["capacity"]
+    for s in (0, 1):
+        sim.load(s, rng.uniform(1, sim.nx - 2, n), rng.uniform(1, sim.ny - 2, n),
+                 *[rng.normal(0, 1e4, n) for _ in range(3)])
+    sim.init()
+
+
+def make(nx, ny, rz, precision="mixed", sweeps=2):
     mask = np.zeros((ny, nx), np.uint8)
     mask[-1] = mask[:, 0] = mask[:, -1] = 1
     if not rz:
@@ -29,13 +39,9 @@ def make(nx, ny, rz, precision="mixed", sweeps=2, seed=1, **options):
     n = 20_000
     sp = [dict(name=k, charge=q, mass=m, np2c=1e4, capacity=n)
           for k, q, m in (("e", -Consts.qe, Consts.me), ("i", Consts.qe, 40 * Consts.mp))]
-    sim = PICSimulation(nx, ny, DX, DX, 1e-12, sp, mask, **dict(dict(
-        tol=1e-300, max_cycles=CYCLES, precision=precision, pre_sweeps=sweeps, post_sweeps=sweeps, use_graph=True,
-        geometry="rz" if rz else "cartesian"), **options))
-    rng = np.random.default_rng(seed)
-    for s in (0, 1):
-        sim.load(s, rng.uniform(1, nx - 2, n), rng.uniform(1, ny - 2, n), *[rng.normal(0, 1e4, n) for _ in range(3)])
-    sim.init()
+    sim = PICSimulation(nx, ny, DX, DX, 1e-12, sp, mask, tol=1e-300, max_cycles=CYCLES, precision=precision,
+                        pre_sweeps=sweeps, post_sweeps=sweeps, use_graph=True, geometry="rz" if rz else "cartesian")
+    load(sim)
     return sim, mask
 
 
@@ -62,4 +68,32 @@ def test_cycles_past_those_in_line(shape, precision, sweeps):
         c = sim.counters()
         assert c["last_cycles"] == CYCLES
         assert c["last_rel_res"] < 1e-9 and (rz or residual(sim, mask) < 1e-9)
+    sim.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rz", [False, True])
+def test_barrier_timeout_is_reported_and_cleared(rz):
+    """With the wait limit lowered to one poll the launch's barriers give up; the error is
+    reported once, and the simulation steps as before with the default limit.  (The limit
+    is the particle pass's too: one report names both.)"""
+    sim, mask = make(129, 97, rz)
+    sim.step(1)
+    sim.counters()
+    sim.set_wait_limit(1)
+    sim.step(3)
+    said = []
+    for _ in range(3):
+        try:
+            sim.counters()
+        except _lib.PicError as e:
+            assert e.code == _lib.PIC_ERR_TIMEOUT
+            said.append(str(e))
+    assert len(said) == 1 and "grid barrier" in said[0], said
+    torch.cuda.synchronize()  # the context is intact
+    sim.set_wait_limit(-1)
+    load(sim)
+    sim.step(2)
+    c = sim.counters()
+    assert c["last_cycles"] == CYCLES and c["last_rel_res"] < 1e-9
     sim.close()
