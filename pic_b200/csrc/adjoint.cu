@@ -33,6 +33,7 @@
 // steps; the backward pass recomputes each segment of C steps from its
 // checkpoint, keeping the segment's positions and fields, then walks it back.
 #include <climits>
+#include <numeric>
 #include <vector>
 
 #include "sort_internal.cuh"
@@ -678,6 +679,10 @@ static int adj_create(const pic_adj_desc* d, AdjImpl& J) {
     PIC_TRY(adalloc(J, &J.V, size_t(PIC_ADJ_MAX_SEGMENTS)));
     PIC_TRY(adalloc(J, &J.red, size_t(2 + PIC_ADJ_MAX_SEGMENTS)));
     PIC_TRY(adalloc(J, &J.failures, 1));
+    // until a species' particles are set, its slots are the caller's
+    std::vector<uint32_t> slots(n);
+    std::iota(slots.begin(), slots.end(), 0u);
+    PIC_CUDA(cudaMemcpy(J.perm, slots.data(), sizeof(uint32_t) * n, cudaMemcpyHostToDevice));
     std::vector<uint8_t> spv(n, 0);
     for (int s = 0; s < d->nspecies; ++s)
         for (int p = J.first[s]; p < J.first[s + 1]; ++p) spv[p] = uint8_t(s);
