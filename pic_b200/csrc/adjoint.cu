@@ -33,6 +33,7 @@
 // steps; the backward pass recomputes each segment of C steps from its
 // checkpoint, keeping the segment's positions and fields, then walks it back.
 #include <climits>
+#include <mutex>
 #include <numeric>
 #include <vector>
 
@@ -585,6 +586,10 @@ struct AdjImpl {
     // one segment of positions and fields (states a+1 .. a+C)
     double* seg_xy = nullptr;
     int* sort_cnt = nullptr;  // digit counts of the cell order's sort, their totals and the two counts
+    // every species' sort works in the same scratch: on whatever streams and
+    // threads species are set, one sort follows the other
+    std::mutex sort_mutex;
+    cudaEvent_t sorted = nullptr;
     AdQuad* seg_E = nullptr;
     // grids
     uint8_t* mask = nullptr;
@@ -616,6 +621,8 @@ static void adj_free(AdjImpl& J) {
     J.mg = J.mga = nullptr;
     for (void* p : J.allocs) cudaFree(p);
     J.allocs.clear();
+    if (J.sorted) cudaEventDestroy(J.sorted);
+    J.sorted = nullptr;
 }
 
 static int adj_create(const pic_adj_desc* d, AdjImpl& J) {
@@ -666,6 +673,7 @@ static int adj_create(const pic_adj_desc* d, AdjImpl& J) {
     const size_t C = size_t(std::min(d->checkpoint_every, d->steps));
     PIC_TRY(adalloc(J, &J.seg_xy, C * 2 * n));
     PIC_TRY(adalloc(J, &J.seg_E, C * G));
+    PIC_CUDA(cudaEventCreateWithFlags(&J.sorted, cudaEventDisableTiming));
     PIC_TRY(adalloc(J, &J.sort_cnt, (size_t(num_sms() + 1) << kSortDigitMax) + 2));
     PIC_TRY(adalloc(J, &J.mask, G));
     PIC_CUDA(cudaMemcpy(J.mask, mask.data(), G, cudaMemcpyHostToDevice));
@@ -933,6 +941,12 @@ static int set_species(AdjImpl& J, int s, const double* const src[6], cudaStream
     const int b = J.first[s], n = J.first[s + 1] - b;
     // the sort's scratch: keys and slots in the segment's position arrays (16
     // bytes per particle, used by the backward pass alone)
+    std::lock_guard<std::mutex> lock(J.sort_mutex);
+    // (in a capture the graph orders them: an event recorded outside cannot be waited on)
+    cudaStreamCaptureStatus cs;
+    PIC_CUDA(cudaStreamIsCapturing(st, &cs));
+    const bool capturing = cs != cudaStreamCaptureStatusNone;
+    if (!capturing) PIC_CUDA(cudaStreamWaitEvent(st, J.sorted, 0));
     SortImpl R;
     PIC_TRY(sort_geometry(n, J.d.nx, J.d.ny, kAdTile, num_sms(), &R));
     uint32_t* scratch = reinterpret_cast<uint32_t*>(J.seg_xy);
@@ -951,6 +965,7 @@ static int set_species(AdjImpl& J, int s, const double* const src[6], cudaStream
     for (int q = 0; q < 6; ++q) k_ad_gather<<<grid_blocks(n, 256), 256, 0, st>>>(src[q], perm, n, dst[q] + b);
     k_ad_slots<<<grid_blocks(n, 256), 256, 0, st>>>(perm, n, uint32_t(b), J.perm + b);
     PIC_LAUNCH_CHECK();
+    if (!capturing) PIC_CUDA(cudaEventRecord(J.sorted, st));
     return PIC_OK;
 }
 
