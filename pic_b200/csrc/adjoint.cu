@@ -43,8 +43,7 @@ namespace pic {
 
 int grid_blocks(long n, int threads);
 int mg_create(int nx, int ny, double dx, double dy, const uint8_t* h_mask, const pic_mg_options* opts, pic_mg** out);
-int mg_launch_graph(pic_mg* mg, double* phi, const double* f, double tol, int max_cycles, int min_cycles,
-                    cudaStream_t st);
+int mg_launch_cold(pic_mg* mg, double* phi, const double* f, double tol, int max_cycles, cudaStream_t st);
 const int* mg_device_converged(pic_mg* mg);
 int mg_info(pic_mg* mg, pic_mg_info* info);
 
@@ -711,7 +710,7 @@ static int pass_blocks(const AdjImpl& J) {
 static int field_of(AdjImpl& J, double* phi, AdQuad* E, cudaStream_t st) {
     k_ad_rhs<<<grid_blocks(J.G, 256), 256, 0, st>>>(J.rho, J.mask, -1.0 / J.d.eps0, J.f, J.G);
     PIC_LAUNCH_CHECK();
-    PIC_TRY(mg_launch_graph(J.mg, phi, J.f, J.d.tol, J.d.max_cycles, 0, st));
+    PIC_TRY(mg_launch_cold(J.mg, phi, J.f, J.d.tol, J.d.max_cycles, st));
     dim3 g;
     const int t = grid2(J, g);
     k_ad_efield<<<g, t, 0, st>>>(phi, E, J.d.nx, J.d.ny, J.d.dx, J.d.dy,
@@ -829,7 +828,7 @@ static int field_adj(AdjImpl& J, cudaStream_t st) {
     const int t = grid2(J, g);
     k_ad_gradT<<<g, t, 0, st>>>(J.lE, J.mask, J.lphi, J.fa, J.d.nx, J.d.ny, J.d.dx, J.d.dy);
     PIC_LAUNCH_CHECK();
-    PIC_TRY(mg_launch_graph(J.mga, J.mu, J.fa, J.d.tol, J.d.max_cycles, 0, st));
+    PIC_TRY(mg_launch_cold(J.mga, J.mu, J.fa, J.d.tol, J.d.max_cycles, st));
     k_ad_dV<<<g, t, 0, st>>>(J.lphi, J.mu, J.mask, J.segid, J.d.nx, J.d.ny, 1.0 / (J.d.dx * J.d.dx),
                              1.0 / (J.d.dy * J.d.dy), J.red + 2, J.lE,
                              J.d.tol > 0 ? mg_device_converged(J.mga) : nullptr, J.failures);

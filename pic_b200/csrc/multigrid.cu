@@ -1818,6 +1818,7 @@ struct MgImpl {
         const double* f = nullptr;
         double tol = 0;
         int max = -1, min = -1;
+        bool cold = false;
     } graph[2];
     double *s_phi = nullptr, *s_f = nullptr;
 };
@@ -2582,7 +2583,7 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
     return PIC_OK;
 }
 
-// The first cycles of a register-tile solve as plain launches.  The first
+// The first K cycles of a register-tile solve (K >= 1) as plain launches.  The first
 // cycle's finest down phase forms the first residual (no launch of its own).
 // The first min_cycles cycles always run, and the ones before the last of them
 // end without a norm; the others do nothing once the solve has stopped.  rest:
@@ -2592,26 +2593,34 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
 // the residual by about 100 where all Dirichlet nodes are on the edges (r-z
 // sometimes takes one more).  A step's guess (min_cycles > 0), extrapolated from
 // the last two potentials, starts near 1e-2: 2, 3 and 4 cycles at tolerances
-// 1e-6, 1e-8 and 1e-10 from 97 x 65 to 2049^2.  Any other guess is taken as
-// cold.  A cycle that turns out not to be needed costs a launch of about 1 us
-// per phase (129 x 97 step at 1e-8: 63.5 us with one cycle more in line, 57.2
-// without; 2049^2: 703 and 624), one that was not launched 5.5 us more than
-// here in the graph's WHILE node (a second cycle in the node's body costs large
-// grids more than it saves: 2049^2 solve 1008 us against 942) and 10 more in
-// k_rt_rest.
+// 1e-6, 1e-8 and 1e-10 from 97 x 65 to 2049^2.  cold: the caller knows its guess
+// to be poor (the adjoint's solves).  What a cycle costs that turns out not to be
+// needed grows with the grid (a launch per phase and its loads: 6 us at 129 x 97,
+// 11 at 513^2, 52 at 2049^2), what one in line saves does not (5.5 us an iteration
+// of the graph's WHILE node, 10 more in k_rt_rest): a solve whose guess may be
+// anything, a converged one among it, launches none ahead (to 1e-9, six ahead
+// and none: from the converged potential 77 and 44 us at 129 x 97, 108 and 47 at
+// 513^2, 392 and 78 at 2049^2; from zero, five cycles, 103 and 124, 149 and 164,
+// 632 and 602).  (A second
+// cycle in the node's body costs large grids more than it saves: 2049^2 solve 1008
+// us against 942.)
 constexpr int kMaxAheadCycles = 8;
 
-static int first_cycles(int max_cycles, int min_cycles, double tol) {
-    const double d = tol > 0.0 ? std::min(-0.5 * std::log10(tol), double(kMaxAheadCycles)) : double(kMaxAheadCycles);
-    const int k = min_cycles > 0 ? std::max(min_cycles, int(std::ceil(d - 1.0))) : std::max(2, int(std::ceil(d + 1.0)));
-    return std::min(max_cycles, std::max(min_cycles, std::min(k, kMaxAheadCycles)));
+static int first_cycles(int max_cycles, int min_cycles, double tol, bool cold) {
+    int k = min_cycles;
+    if (min_cycles > 0 || cold) {
+        const double d = tol > 0.0 ? std::min(-0.5 * std::log10(tol), double(kMaxAheadCycles)) : double(kMaxAheadCycles);
+        k = min_cycles > 0 ? int(std::ceil(d - 1.0)) : std::max(2, int(std::ceil(d + 1.0)));
+        k = std::max(min_cycles, std::min(k, kMaxAheadCycles));
+    }
+    return std::max(0, std::min(max_cycles, k));
 }
 
 template <class T>
 static int launch_first_cycles(MgImpl& M, std::vector<LevelDev<T>>& lv, double* phi, const double* f, double tol,
-                               int max_cycles, int min_cycles, cudaGraphConditionalHandle cond, int use_cond,
+                               int max_cycles, int min_cycles, int K, cudaGraphConditionalHandle cond, int use_cond,
                                cudaStream_t st, RtPending* rest = nullptr) {
-    const int kmin = std::max(0, std::min(min_cycles, max_cycles)), K = first_cycles(max_cycles, kmin, tol);
+    const int kmin = std::max(0, std::min(min_cycles, max_cycles));
     const RtInit init{phi, f, M.rz0, M.r64, 1.0 / (M.dx * M.dx), 1.0 / (M.dy * M.dy)};
     const RtShape h0 = rt_up_shape(M.o.pre_sweeps, M.nx, M.ny, true);
     const RtShape h1 = rt_up_shape(M.o.post_sweeps, M.nx, M.ny, true);
@@ -2722,27 +2731,29 @@ static int launch_rest(MgImpl& M, const std::vector<LevelDev<T>>& lv_in, double*
 // 257 x 193: 10 steps 4643 us against 3830).
 template <class T>
 static int capture_solve(MgImpl& M, std::vector<LevelDev<T>>& lv, double* phi, const double* f, double tol,
-                         int max_cycles, int min_cycles, bool alone, cudaStream_t st) {
+                         int max_cycles, int min_cycles, bool cold, bool alone, cudaStream_t st) {
     cudaStreamCaptureStatus cs;
     cudaGraph_t g = nullptr;
     const cudaGraphNode_t* deps = nullptr;
     size_t nd = 0;
     PIC_CUDA(cudaStreamGetCaptureInfo(st, &cs, nullptr, &g, &deps, &nd));
     if (cs != cudaStreamCaptureStatusActive) return fail(PIC_ERR_BAD_ARG, "multigrid: stream is not capturing");
-    const bool rt = rt_cycles(M) && max_cycles > 0;
-    if (rt && first_cycles(max_cycles, min_cycles, tol) >= max_cycles)  // no loop left
-        return launch_first_cycles(M, lv, phi, f, tol, max_cycles, min_cycles, cudaGraphConditionalHandle{}, 0, st);
+    const int ahead = rt_cycles(M) ? first_cycles(max_cycles, min_cycles, tol, cold) : 0;
+    const bool rt = ahead > 0;
+    if (rt && ahead >= max_cycles)  // no loop left
+        return launch_first_cycles(M, lv, phi, f, tol, max_cycles, min_cycles, ahead, cudaGraphConditionalHandle{}, 0,
+                                   st);
     if (const int blocks = rt && alone ? rest_blocks(M, lv) : 0) {
         RtPending pending{};
-        PIC_TRY(launch_first_cycles(M, lv, phi, f, tol, max_cycles, min_cycles, cudaGraphConditionalHandle{}, 0, st,
-                                    &pending));
+        PIC_TRY(launch_first_cycles(M, lv, phi, f, tol, max_cycles, min_cycles, ahead, cudaGraphConditionalHandle{}, 0,
+                                    st, &pending));
         if (!pending.nb) return fail(PIC_ERR_CUDA, "multigrid: no decision left for the cycles after the launched ones");
         return launch_rest(M, lv, phi, tol, max_cycles, blocks, pending, st);
     }
     cudaGraphConditionalHandle h;
     PIC_CUDA(cudaGraphConditionalHandleCreate(&h, g, 0, cudaGraphCondAssignDefault));
     if (rt) {
-        PIC_TRY(launch_first_cycles(M, lv, phi, f, tol, max_cycles, min_cycles, h, 1, st));
+        PIC_TRY(launch_first_cycles(M, lv, phi, f, tol, max_cycles, min_cycles, ahead, h, 1, st));
     } else {
         const int K = std::max(0, std::min(min_cycles, max_cycles));
         launch_r0(M, lv, phi, f, tol, max_cycles, 1, h, K == 0, st);
@@ -2886,8 +2897,8 @@ static int launch_dst(MgImpl& M, double* phi, const double* f, double tol, int m
     return PIC_OK;
 }
 
-int mg_capture(MgImpl& M, double* phi, const double* f, double tol, int max_cycles, int min_cycles, bool alone,
-               cudaStream_t st) {
+int mg_capture(MgImpl& M, double* phi, const double* f, double tol, int max_cycles, int min_cycles, bool cold,
+               bool alone, cudaStream_t st) {
     if (M.dst) return launch_dst(M, phi, f, tol, max_cycles, st);
     if (M.o.launch_mode == PIC_MG_CLUSTER && M.cluster_ok) return launch_cluster(M, phi, f, tol, max_cycles, st);
     if (M.o.launch_mode == PIC_MG_PERSISTENT)
@@ -2895,21 +2906,22 @@ int mg_capture(MgImpl& M, double* phi, const double* f, double tol, int max_cycl
                                            : launch_persistent(M, M.ld, phi, f, tol, max_cycles, st);
     if (M.o.launch_mode == PIC_MG_HOST_LOOP)
         return fail(PIC_ERR_BAD_ARG, "multigrid: the host-driven loop cannot be captured in a graph");
-    return M.precision == PIC_MG_MIXED ? capture_solve(M, M.lf, phi, f, tol, max_cycles, min_cycles, alone, st)
-                                       : capture_solve(M, M.ld, phi, f, tol, max_cycles, min_cycles, alone, st);
+    return M.precision == PIC_MG_MIXED ? capture_solve(M, M.lf, phi, f, tol, max_cycles, min_cycles, cold, alone, st)
+                                       : capture_solve(M, M.ld, phi, f, tol, max_cycles, min_cycles, cold, alone, st);
 }
 
 // A solve's graph, built again where its buffers or limits change.
 static int ensure_graph(MgImpl& M, MgImpl::Graph& G, double* phi, const double* f, double tol, int max_cycles,
-                        int min_cycles) {
-    if (G.exec && G.phi == phi && G.f == f && G.tol == tol && G.max == max_cycles && G.min == min_cycles)
+                        int min_cycles, bool cold) {
+    if (G.exec && G.phi == phi && G.f == f && G.tol == tol && G.max == max_cycles && G.min == min_cycles &&
+        G.cold == cold)
         return PIC_OK;
     if (G.exec) {
         cudaGraphExecDestroy(G.exec);
         G.exec = nullptr;
     }
     PIC_CUDA(cudaStreamBeginCapture(M.cap, cudaStreamCaptureModeThreadLocal));
-    const int rc = mg_capture(M, phi, f, tol, max_cycles, min_cycles, true, M.cap);
+    const int rc = mg_capture(M, phi, f, tol, max_cycles, min_cycles, cold, true, M.cap);
     cudaGraph_t g = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(M.cap, &g);
     if (rc != PIC_OK) {
@@ -2925,6 +2937,7 @@ static int ensure_graph(MgImpl& M, MgImpl::Graph& G, double* phi, const double* 
     G.tol = tol;
     G.max = max_cycles;
     G.min = min_cycles;
+    G.cold = cold;
     return PIC_OK;
 }
 
@@ -2932,7 +2945,7 @@ static int ensure_graph(MgImpl& M, MgImpl::Graph& G, double* phi, const double* 
 // buffers other than the first pair do not get one of their own: they are
 // copied to the solver's and back (a copy takes a few microseconds at 513^2, 16
 // at 2049^2).
-static int launch_graph(MgImpl& M, double* phi, const double* f, double tol, int max_cycles, int min_cycles,
+static int launch_graph(MgImpl& M, double* phi, const double* f, double tol, int max_cycles, int min_cycles, bool cold,
                         cudaStream_t st) {
     const size_t nodes = size_t(M.nx) * M.ny, bytes = sizeof(double) * nodes;
     MgImpl::Graph& own = M.graph[0];
@@ -2949,11 +2962,11 @@ static int launch_graph(MgImpl& M, double* phi, const double* f, double tol, int
         }
     }
     if (!copy) {
-        PIC_TRY(ensure_graph(M, own, phi, f, tol, max_cycles, min_cycles));
+        PIC_TRY(ensure_graph(M, own, phi, f, tol, max_cycles, min_cycles, cold));
         PIC_CUDA(cudaGraphLaunch(own.exec, st));
         return PIC_OK;
     }
-    PIC_TRY(ensure_graph(M, M.graph[1], M.s_phi, M.s_f, tol, max_cycles, min_cycles));
+    PIC_TRY(ensure_graph(M, M.graph[1], M.s_phi, M.s_f, tol, max_cycles, min_cycles, cold));
     PIC_CUDA(cudaMemcpyAsync(M.s_phi, phi, bytes, cudaMemcpyDeviceToDevice, st));
     PIC_CUDA(cudaMemcpyAsync(M.s_f, f, bytes, cudaMemcpyDeviceToDevice, st));
     PIC_CUDA(cudaGraphLaunch(M.graph[1].exec, st));
@@ -3017,7 +3030,8 @@ static int solve_eager(MgImpl& M, std::vector<LevelDev<T>>& lv, double* phi, con
     return PIC_OK;
 }
 
-int mg_launch(MgImpl& M, double* phi, const double* f, double tol, int max_cycles, int min_cycles, cudaStream_t st) {
+int mg_launch(MgImpl& M, double* phi, const double* f, double tol, int max_cycles, int min_cycles, cudaStream_t st,
+              bool cold = false) {
     if (M.dst) return launch_dst(M, phi, f, tol, max_cycles, st);
     if (M.o.launch_mode == PIC_MG_CLUSTER && M.cluster_ok) return launch_cluster(M, phi, f, tol, max_cycles, st);
     if (M.o.launch_mode == PIC_MG_PERSISTENT)
@@ -3026,7 +3040,7 @@ int mg_launch(MgImpl& M, double* phi, const double* f, double tol, int max_cycle
     if (M.o.launch_mode == PIC_MG_HOST_LOOP)
         return M.precision == PIC_MG_MIXED ? solve_eager(M, M.lf, phi, f, tol, max_cycles, min_cycles, st)
                                            : solve_eager(M, M.ld, phi, f, tol, max_cycles, min_cycles, st);
-    return launch_graph(M, phi, f, tol, max_cycles, min_cycles, st);
+    return launch_graph(M, phi, f, tol, max_cycles, min_cycles, cold, st);
 }
 
 int mg_solve(MgImpl& M, double* phi, const double* f, double tol, int max_cycles, pic_mg_info* info,
@@ -3061,13 +3075,17 @@ int mg_fixed_launches(pic_mg* mg) {
 }
 int mg_capture_into(pic_mg* mg, double* phi, const double* f, double tol, int max_cycles, int min_cycles, bool alone,
                     cudaStream_t st) {
-    return mg_capture(mg->m, phi, f, tol, max_cycles, min_cycles, alone, st);
+    return mg_capture(mg->m, phi, f, tol, max_cycles, min_cycles, false, alone, st);
 }
 bool mg_uses_graph(pic_mg* mg) { return mg->m.o.launch_mode != PIC_MG_HOST_LOOP; }
 bool mg_is_rz(pic_mg* mg) { return mg->m.rz; }
 int mg_launch_graph(pic_mg* mg, double* phi, const double* f, double tol, int max_cycles, int min_cycles,
                     cudaStream_t st) {
     return mg_launch(mg->m, phi, f, tol, max_cycles, min_cycles, st);
+}
+// A solve whose guess is known to need about as many cycles as the tolerance has powers of 100.
+int mg_launch_cold(pic_mg* mg, double* phi, const double* f, double tol, int max_cycles, cudaStream_t st) {
+    return mg_launch(mg->m, phi, f, tol, max_cycles, 0, st, true);
 }
 int mg_info(pic_mg* mg, pic_mg_info* info) { return mg_read_info(mg->m, info); }
 const int* mg_device_converged(pic_mg* mg) { return mg->m.N.converged; }
