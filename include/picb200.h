@@ -244,7 +244,8 @@ int pic_mg_tile_geometry(int sweeps, int* out);
  * preconditions each iteration (NULL: none).  pic_cg_solve keeps phi on the
  * Dirichlet nodes, iterates until ||f - lap(phi)|| / ||f|| < tol over the free
  * nodes or max_iter (info->cycles = iterations), waits for `stream` once per
- * iteration (for the one before it) and at the end, and returns PIC_ERR_NOT_CONVERGED if tol is not reached. */
+ * iteration (without a preconditioner for the one before it) and at the end, and
+ * returns PIC_ERR_NOT_CONVERGED if tol is not reached. */
 typedef struct pic_cg pic_cg;
 int pic_cg_create(int nx, int ny, double dx, double dy, const uint8_t* h_dirichlet, pic_mg* precond, pic_cg** out);
 int pic_cg_solve(pic_cg* cg, double* d_phi, const double* d_f, double tol, int max_iter, pic_mg_info* info,

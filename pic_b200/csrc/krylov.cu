@@ -12,10 +12,13 @@
 // The scalars (beta, alpha, the norms, the iteration count and the decision to
 // stop) stay on the device: each kernel's last block to finish adds the block
 // partials in a fixed order and derives what the next kernel needs, so an
-// iteration is three launches besides the V-cycle's and no host round trip
-// (three of about 20 us each before; 385 x 257, tol 1e-9: the call 691 -> 435 us).  The
-// host runs one iteration ahead of the stop flag it reads back; what is enqueued
-// past the end does nothing.
+// iteration is three launches besides the V-cycle's and one host round trip
+// (three before; 385 x 257 to 1e-9: the call 855 -> 426 us).  With a
+// preconditioner the host waits for the decision before it enqueues an iteration:
+// one ahead of it is a V-cycle too many per solve, which costs what the waits of
+// four iterations do at 65^2 and more on larger grids (513^2: 359 us ahead, 331
+// waiting; from the converged potential 137 and 49).  Without one the host runs one
+// iteration ahead, whose three kernels do nothing past the end.
 #include <cmath>
 #include <utility>
 #include <vector>
@@ -49,7 +52,7 @@ struct CgImpl {
     double *r = nullptr, *r_prev = nullptr, *z = nullptr, *p = nullptr, *p2 = nullptr, *q = nullptr, *x = nullptr;
     double* part = nullptr;  // [2][blocks]
     CgState* state = nullptr;
-    int* h_stop = nullptr;  // page-locked: the stop flag after each of the last two iterations
+    CgState* h_state = nullptr;  // page-locked: the state after each of the last two iterations
     cudaEvent_t ev[2] = {nullptr, nullptr};
     int blocks = 0;
     std::vector<void*> allocs;
@@ -215,8 +218,8 @@ int grid_blocks(long n, int threads);
 static void cg_release(CgImpl& C) {
     for (void* a : C.allocs) cudaFree(a);
     C.allocs.clear();
-    if (C.h_stop) cudaFreeHost(C.h_stop);
-    C.h_stop = nullptr;
+    if (C.h_state) cudaFreeHost(C.h_state);
+    C.h_state = nullptr;
     for (cudaEvent_t& e : C.ev) {
         if (e) cudaEventDestroy(e);
         e = nullptr;
@@ -266,7 +269,7 @@ int pic_cg_create(int nx, int ny, double dx, double dy, const uint8_t* h_dirichl
         ok = ok && alloc(reinterpret_cast<void**>(v), vb);
     ok = ok && alloc(reinterpret_cast<void**>(&C.part), sizeof(double) * 2 * size_t(C.blocks)) &&
          alloc(reinterpret_cast<void**>(&C.state), sizeof(CgState)) &&
-         cudaMallocHost(reinterpret_cast<void**>(&C.h_stop), 2 * sizeof(int)) == cudaSuccess;
+         cudaMallocHost(reinterpret_cast<void**>(&C.h_state), 2 * sizeof(CgState)) == cudaSuccess;
     for (cudaEvent_t& e : C.ev) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
     if (!ok) {
         cg_release(C);
@@ -298,7 +301,24 @@ int pic_cg_solve(pic_cg* h, double* d_phi, const double* d_f, double tol, int ma
     PIC_CUDA(cudaMemsetAsync(C.state, 0, sizeof(CgState), st));
     k_cg_init<<<B, kCgThreads, 0, st>>>(d_phi, d_f, C.free_, C.nx, C.G, C.cx, C.cy, C.r, C.x, z, tol, C.part, C.state);
     PIC_LAUNCH_CHECK();
+    // the state after the newest launches, on its way to the host, and whether it says stop
+    int slot = 0;
+    auto post = [&]() -> int {
+        slot ^= 1;
+        PIC_CUDA(cudaMemcpyAsync(C.h_state + slot, C.state, sizeof(CgState), cudaMemcpyDeviceToHost, st));
+        PIC_CUDA(cudaEventRecord(C.ev[slot], st));
+        return PIC_OK;
+    };
+    auto wait = [&](int s, bool& stop) -> int {
+        PIC_CUDA(cudaEventSynchronize(C.ev[s]));
+        stop = C.h_state[s].stop != 0;
+        return PIC_OK;
+    };
+    PIC_TRY(post());
     for (int it = 0; it < max_iter; ++it) {
+        bool stop = false;
+        if (C.mg || it == 0) PIC_TRY(wait(slot, stop));
+        if (stop) break;
         if (C.mg) PIC_TRY(mg_launch_graph(C.mg, C.z, C.r, 1e-300, 1, 1, st));
         const double* zz = C.mg ? C.z : C.r;
         k_cg_beta<<<B, kCgThreads, 0, st>>>(C.r, C.r_prev, zz, C.free_, C.G, C.part, C.state);
@@ -307,20 +327,16 @@ int pic_cg_solve(pic_cg* h, double* d_phi, const double* d_f, double tol, int ma
                                               C.state);
         std::swap(C.p, C.p2);
         PIC_LAUNCH_CHECK();
-        const int slot = it & 1;
-        PIC_CUDA(cudaMemcpyAsync(C.h_stop + slot, &C.state->stop, sizeof(int), cudaMemcpyDeviceToHost, st));
-        PIC_CUDA(cudaEventRecord(C.ev[slot], st));
-        // the iteration before this one decides whether there is another
-        if (it > 0) {
-            PIC_CUDA(cudaEventSynchronize(C.ev[slot ^ 1]));
-            if (C.h_stop[slot ^ 1]) break;
-        }
+        PIC_TRY(post());
+        // without a preconditioner, the iteration before this one decides whether there is another
+        if (!C.mg && it > 0) PIC_TRY(wait(slot ^ 1, stop));
+        if (stop) break;
     }
     k_cg_finish<<<grid_blocks(C.G, kCgThreads), kCgThreads, 0, st>>>(d_phi, C.x, C.free_, C.G);
     PIC_LAUNCH_CHECK();
-    CgState S{};
-    PIC_CUDA(cudaMemcpyAsync(&S, C.state, sizeof S, cudaMemcpyDeviceToHost, st));
+    PIC_TRY(post());
     PIC_CUDA(cudaStreamSynchronize(st));
+    const CgState& S = C.h_state[slot];
     pic_mg_info loc{};
     const double ref = S.f2 > 0.0 ? S.f2 : 1.0;
     loc.cycles = S.it;

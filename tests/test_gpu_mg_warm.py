@@ -58,6 +58,23 @@ def test_converged_guess_is_cheap(n, precision):
     assert warm < 0.5 * cold, (warm, cold)
 
 
+@pytest.mark.parametrize("preconditioned", [True, False])
+@pytest.mark.parametrize("n", [65, 513])
+def test_converged_guess_is_cheap_for_conjugate_gradients(n, preconditioned):
+    """No iteration from the converged potential: below a third of the solve from zero (an
+    iteration enqueued ahead of the decision made it 0.4 of it)."""
+    mask, f = box(n)
+    mg = MultigridSolver(mask, n, n, DX, precision="fp64") if preconditioned else None
+    cg = ConjugateGradientSolver(mask, n, n, DX, precond=mg)
+    done, phi = torch.zeros_like(f), torch.zeros_like(f)
+    cg.solve(done, f, tol=1e-10, max_iter=2000)
+    solve = lambda: cg.solve(phi, f, tol=1e-8, max_iter=2000)[1][0]  # noqa: E731
+    warm, none = fastest(solve, phi, done)
+    cold, some = fastest(solve, phi, torch.zeros_like(f))
+    assert none == 0 and some >= 4
+    assert warm < cold / 3, (warm, cold)
+
+
 def residual(phi, rho, mask):
     ny, nx = mask.shape
     phi, rho = (a.cpu().numpy().astype(np.float64).reshape(ny, nx) for a in (phi, rho))
