@@ -1810,8 +1810,9 @@ struct MgImpl {
     unsigned long long wait_polls = kBarrierPolls;  // grid-barrier wait limit of the cooperative launches
     cudaStream_t side = nullptr;
     cudaStream_t cap = nullptr;
-    // cached solve graphs: [0] on the first pair of buffers a solve was given
-    // (its limits may change), [1] on the solver's own copies
+    // cached solve graphs: [0] on a pair of buffers that solves were given (the
+    // first, or the last to come twice in a row; its limits may change), [1] on
+    // the solver's own copies
     struct Graph {
         cudaGraphExec_t exec = nullptr;
         double* phi = nullptr;
@@ -1821,6 +1822,8 @@ struct MgImpl {
         bool cold = false;
     } graph[2];
     double *s_phi = nullptr, *s_f = nullptr;
+    // the pair of the last solve, where it ran on the copies
+    const double *other_phi = nullptr, *other_f = nullptr;
 };
 
 }  // namespace pic
@@ -2942,14 +2945,14 @@ static int ensure_graph(MgImpl& M, MgImpl::Graph& G, double* phi, const double* 
 }
 
 // A graph-loop solve.  Building a graph takes several hundred microseconds, so
-// buffers other than the first pair do not get one of their own: they are
+// buffers that change from call to call do not get one of their own: they are
 // copied to the solver's and back (a copy takes a few microseconds at 513^2, 16
-// at 2049^2).
+// at 2049^2).  A pair that comes a second time in a row takes the first graph over.
 static int launch_graph(MgImpl& M, double* phi, const double* f, double tol, int max_cycles, int min_cycles, bool cold,
                         cudaStream_t st) {
     const size_t nodes = size_t(M.nx) * M.ny, bytes = sizeof(double) * nodes;
     MgImpl::Graph& own = M.graph[0];
-    bool copy = own.phi && (own.phi != phi || own.f != f);
+    bool copy = own.phi && (own.phi != phi || own.f != f) && (M.other_phi != phi || M.other_f != f);
     if (copy && !M.s_phi) {
         double* b = nullptr;
         if (cudaMalloc(&b, 2 * bytes) == cudaSuccess) {
@@ -2961,6 +2964,8 @@ static int launch_graph(MgImpl& M, double* phi, const double* f, double tol, int
             copy = false;
         }
     }
+    M.other_phi = copy ? phi : nullptr;
+    M.other_f = copy ? f : nullptr;
     if (!copy) {
         PIC_TRY(ensure_graph(M, own, phi, f, tol, max_cycles, min_cycles, cold));
         PIC_CUDA(cudaGraphLaunch(own.exec, st));
