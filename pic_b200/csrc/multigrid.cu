@@ -1854,9 +1854,28 @@ static std::vector<double> rz_rows(int ny, double hx, double hy) {
     return r;
 }
 
+// The free nodes (not Dirichlet, not on a grid edge; in r-z the axis row is free)
+// as bit columns, a thread per word of 32 rows.
+__global__ void __launch_bounds__(128) k_free_bits(const uint8_t* __restrict__ mask, int nx, int ny, int axis_free,
+                                                   uint32_t* __restrict__ fb) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j0 = 32 * int(blockIdx.y);
+    if (i >= nx) return;
+    uint32_t w = 0u;
+    if (i > 0 && i < nx - 1) {
+        const int first = max(j0, axis_free ? 0 : 1), end = min(j0 + 32, ny - 1);
+        for (int j = first; j < end; ++j) w |= uint32_t(mask[long(j) * nx + i] == 0) << (j - j0);
+    }
+    fb[long(blockIdx.y) * nx + i] = w;
+}
+
 template <class T>
 static int alloc_levels(MgImpl& M, std::vector<LevelDev<T>>& lv, const std::vector<std::vector<uint8_t>>& masks,
                         const std::vector<int>& nxs, const std::vector<int>& nys) {
+    size_t words = 0;
+    for (int l = 0; l < M.L; ++l) words += size_t(div_up(nys[l], 32)) * nxs[l];
+    uint32_t* fb = nullptr;
+    PIC_CUDA(cudaMalloc(&fb, words * sizeof(uint32_t)));
+    M.allocs.push_back(fb);
     for (int l = 0; l < M.L; ++l) {
         LevelDev<T> v{};
         v.nx = nxs[l];
@@ -1872,20 +1891,10 @@ static int alloc_levels(MgImpl& M, std::vector<LevelDev<T>>& lv, const std::vect
         M.allocs.push_back(mk);
         PIC_CUDA(cudaMemcpy(mk, masks[l].data(), G, cudaMemcpyHostToDevice));
         v.mask = mk;
-        // the free nodes (not Dirichlet, not on a grid edge; in r-z the axis
-        // row is free) as bit columns
-        std::vector<uint32_t> fb(size_t((v.ny + 31) / 32) * v.nx, 0u);
-        for (int j = M.rz ? 0 : 1; j < v.ny - 1; ++j) {
-            const uint8_t* __restrict__ m = masks[l].data() + size_t(j) * v.nx;
-            uint32_t* __restrict__ w = fb.data() + size_t(j >> 5) * v.nx;
-            const int n = v.nx - 1, bit = j & 31;
-            for (int i = 1; i < n; ++i) w[i] |= uint32_t(m[i] == 0) << bit;
-        }
-        uint32_t* fbd = nullptr;
-        PIC_CUDA(cudaMalloc(&fbd, fb.size() * sizeof(uint32_t)));
-        M.allocs.push_back(fbd);
-        PIC_CUDA(cudaMemcpy(fbd, fb.data(), fb.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
-        v.fb = fbd;
+        v.fb = fb;
+        k_free_bits<<<dim3(div_up(v.nx, 128), div_up(v.ny, 32)), 128>>>(mk, v.nx, v.ny, M.rz ? 1 : 0, fb);
+        PIC_LAUNCH_CHECK();
+        fb += size_t(div_up(v.ny, 32)) * v.nx;
         // padded to 16 bytes: the coarse kernel reads g in 16-byte words
         const size_t bytes = (G * sizeof(T) + 15) / 16 * 16;
         PIC_CUDA(cudaMalloc(&v.e, bytes));
@@ -1915,6 +1924,7 @@ static int alloc_levels(MgImpl& M, std::vector<LevelDev<T>>& lv, const std::vect
         }
         lv.push_back(v);
     }
+    PIC_CUDA(cudaStreamSynchronize(nullptr));  // solves may come on any stream
     return PIC_OK;
 }
 
@@ -2391,12 +2401,10 @@ int mg_create(int nx, int ny, double dx, double dy, const uint8_t* h_mask, const
     // or of k_rt_rest (rest_blocks: at most one block per SM), whichever is largest
     const int nb = std::max({int(M.grd0.x * M.grd0.y), div_up(nx, 16) * div_up(ny, 16), M.solve_grid, num_sms()});
     M.partials = nb;
-    if (cudaMalloc(&M.N.partial, sizeof(double) * 2 * nb) != cudaSuccess)
+    if (cudaMalloc(&M.N.partial, sizeof(double) * 3 * nb) != cudaSuccess)
         return bail(fail(PIC_ERR_CUDA, "pic_mg_create: out of device memory"));
     M.allocs.push_back(M.N.partial);
-    if (cudaMalloc(&M.N.fpart, sizeof(double) * nb) != cudaSuccess)
-        return bail(fail(PIC_ERR_CUDA, "pic_mg_create: out of device memory"));
-    M.allocs.push_back(M.N.fpart);
+    M.N.fpart = M.N.partial + 2 * size_t(nb);
     if (cudaMalloc(&M.r64, sizeof(double) * size_t(nx) * ny) != cudaSuccess)
         return bail(fail(PIC_ERR_CUDA, "pic_mg_create: out of device memory"));
     M.allocs.push_back(M.r64);
