@@ -224,8 +224,10 @@ int pic_mg_effective_launch_mode(pic_mg* mg, int* mode);
  * (the flag is then cleared and the solver stays usable).  polls < 0 restores
  * the default (2^24 polls, about a second). */
 int pic_mg_set_wait_limit(pic_mg* mg, long long polls);
-/* The shared-memory tile geometry the multigrid's tile kernels use for
- * `sweeps` red-black sweeps (1..8), in nodes, as PIC_MG_GEOMETRY_VALUES ints:
+/* The geometry of the multigrid's shared-memory tiles (the persistent solve's,
+ * and the graph and host loops' for more than three sweeps on a side; up to three
+ * run on register tiles) for `sweeps` red-black sweeps (1..8), in nodes, as
+ * PIC_MG_GEOMETRY_VALUES ints:
  * tile side; down phase halo and width; up phase halo, width and coarse
  * window width; the same for the finest up phase with the residual; the
  * two-level down launch's coarse halo and width and fine halo and width; the

@@ -25,7 +25,6 @@ constexpr int kRtRows = 4;       // rows per warp
 constexpr int kRtMaxWarps = 16;
 constexpr int kRtMaxThreads = 32 * kRtMaxWarps;
 constexpr int kRtCols = 64;      // region columns, = 2 * 32
-constexpr int kRtMaxSweeps = 3;
 constexpr unsigned kRtRowMask = (1u << kRtRows) - 1u;
 
 // How far a phase of S sweeps reaches into the region, from its border (depth

@@ -53,6 +53,7 @@ int grid_blocks(long n, int threads);
 constexpr int kMgTile = 32;
 constexpr int kMgThreads = 512;
 constexpr int kMgMaxSweeps = 8;
+constexpr int kRtMaxSweeps = 3;  // of the register tiles (mg_regtile.cuh); the shared-memory tiles take more
 constexpr int kMgMaxCoarseLevels = 8;
 constexpr int kCoarseThreads = 1024;
 constexpr long kCoarseMaxNodes32 = 33L * 33L;    // FP32 levels at or below this size run in the single-CTA kernel
@@ -856,30 +857,29 @@ using UpKernel = void (*)(LevelDev<T>, LevelDev<T>, T, double*);
 template <class T>
 using UpResKernel = void (*)(LevelDev<T>, LevelDev<T>, T, double*, ResArgs);
 
+// The shared-memory tiles' launches, of more sweeps than register tiles take:
+// s = kRtMaxSweeps + 1 .. kMgMaxSweeps.
 template <class T, bool CYL>
 static DownKernel<T> down_kernel(int s) {
-    static const DownKernel<T> k[kMgMaxSweeps + 1] = {
-        nullptr,                 k_mg_down<T, 1, CYL>, k_mg_down<T, 2, CYL>, k_mg_down<T, 3, CYL>,
-        k_mg_down<T, 4, CYL>,    k_mg_down<T, 5, CYL>, k_mg_down<T, 6, CYL>, k_mg_down<T, 7, CYL>,
-        k_mg_down<T, 8, CYL>};
-    return k[s];
+    static const DownKernel<T> k[kMgMaxSweeps - kRtMaxSweeps] = {k_mg_down<T, 4, CYL>, k_mg_down<T, 5, CYL>,
+                                                                k_mg_down<T, 6, CYL>, k_mg_down<T, 7, CYL>,
+                                                                k_mg_down<T, 8, CYL>};
+    return k[s - kRtMaxSweeps - 1];
 }
 
 template <class T, bool CYL>
 static UpKernel<T> up_kernel(int s) {
-    static const UpKernel<T> k[kMgMaxSweeps + 1] = {
-        nullptr,              k_mg_up<T, 1, CYL>, k_mg_up<T, 2, CYL>, k_mg_up<T, 3, CYL>, k_mg_up<T, 4, CYL>,
-        k_mg_up<T, 5, CYL>,   k_mg_up<T, 6, CYL>, k_mg_up<T, 7, CYL>, k_mg_up<T, 8, CYL>};
-    return k[s];
+    static const UpKernel<T> k[kMgMaxSweeps - kRtMaxSweeps] = {
+        k_mg_up<T, 4, CYL>, k_mg_up<T, 5, CYL>, k_mg_up<T, 6, CYL>, k_mg_up<T, 7, CYL>, k_mg_up<T, 8, CYL>};
+    return k[s - kRtMaxSweeps - 1];
 }
 
 template <class T, bool CYL>
 static UpResKernel<T> up_res_kernel(int s) {
-    static const UpResKernel<T> k[kMgMaxSweeps + 1] = {
-        nullptr,                  k_mg_up_res<T, 1, CYL>, k_mg_up_res<T, 2, CYL>, k_mg_up_res<T, 3, CYL>,
-        k_mg_up_res<T, 4, CYL>,   k_mg_up_res<T, 5, CYL>, k_mg_up_res<T, 6, CYL>, k_mg_up_res<T, 7, CYL>,
-        k_mg_up_res<T, 8, CYL>};
-    return k[s];
+    static const UpResKernel<T> k[kMgMaxSweeps - kRtMaxSweeps] = {k_mg_up_res<T, 4, CYL>, k_mg_up_res<T, 5, CYL>,
+                                                                 k_mg_up_res<T, 6, CYL>, k_mg_up_res<T, 7, CYL>,
+                                                                 k_mg_up_res<T, 8, CYL>};
+    return k[s - kRtMaxSweeps - 1];
 }
 
 template <class T>
@@ -891,18 +891,16 @@ using RtFused2Kernel = void (*)(LevelDev<T>, LevelDev<T>, LevelDev<T>, T, const 
 
 template <class T>
 static Fused2Kernel<T> down2_kernel(int s) {
-    static const Fused2Kernel<T> k[kMgMaxSweeps + 1] = {
-        nullptr,           k_mg_down2<T, 1>, k_mg_down2<T, 2>, k_mg_down2<T, 3>, k_mg_down2<T, 4>,
-        k_mg_down2<T, 5>,  k_mg_down2<T, 6>, k_mg_down2<T, 7>, k_mg_down2<T, 8>};
-    return k[s];
+    static const Fused2Kernel<T> k[kMgMaxSweeps - kRtMaxSweeps] = {
+        k_mg_down2<T, 4>, k_mg_down2<T, 5>, k_mg_down2<T, 6>, k_mg_down2<T, 7>, k_mg_down2<T, 8>};
+    return k[s - kRtMaxSweeps - 1];
 }
 
 template <class T>
 static Fused2Kernel<T> up2_kernel(int s) {
-    static const Fused2Kernel<T> k[kMgMaxSweeps + 1] = {
-        nullptr,         k_mg_up2<T, 1>, k_mg_up2<T, 2>, k_mg_up2<T, 3>, k_mg_up2<T, 4>,
-        k_mg_up2<T, 5>,  k_mg_up2<T, 6>, k_mg_up2<T, 7>, k_mg_up2<T, 8>};
-    return k[s];
+    static const Fused2Kernel<T> k[kMgMaxSweeps - kRtMaxSweeps] = {k_mg_up2<T, 4>, k_mg_up2<T, 5>, k_mg_up2<T, 6>,
+                                                                  k_mg_up2<T, 7>, k_mg_up2<T, 8>};
+    return k[s - kRtMaxSweeps - 1];
 }
 
 template <class T>
@@ -2004,10 +2002,11 @@ static std::vector<double> dense_operator(const MgImpl& M, int l, int nx, int ny
 // where their shared memory fits.
 template <class T>
 static int configure_fuse2(MgImpl& M) {
-    const size_t d = down2_smem<T>(M.o.pre_sweeps), u = up2_smem<T>(M.o.post_sweeps);
+    const int pre = M.o.pre_sweeps, post = M.o.post_sweeps;
+    const size_t d = pre > kRtMaxSweeps ? down2_smem<T>(pre) : 0, u = post > kRtMaxSweeps ? up2_smem<T>(post) : 0;
     if (d > 227 * 1024 || u > 227 * 1024) return PIC_OK;
-    PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(down2_kernel<T>(M.o.pre_sweeps)), d));
-    PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(up2_kernel<T>(M.o.post_sweeps)), u));
+    if (d) PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(down2_kernel<T>(pre)), d));
+    if (u) PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(up2_kernel<T>(post)), u));
     M.fuse2 = true;
     return PIC_OK;
 }
@@ -2073,23 +2072,27 @@ static RtUpKernel<T> rt_res_kernel(const MgImpl& M, bool staged) {
 
 template <class T>
 static int configure_kernels(MgImpl& M) {
-    if (M.o.post_sweeps <= kRtMaxSweeps && !(M.rz && sizeof(T) == 8))
-        PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(rt_res_kernel<T>(M, true)), rt_stage_bytes(kRtMaxThreads)));
-    const size_t down = down_smem<T>(M.o.pre_sweeps, M.rz), up = up_smem<T>(M.o.post_sweeps, M.rz);
-    const size_t upr = up_smem<T>(M.o.post_sweeps, M.rz, true);
+    const int pre = M.o.pre_sweeps, post = M.o.post_sweeps;
+    const size_t down = down_smem<T>(pre, M.rz), up = up_smem<T>(post, M.rz), upr = up_smem<T>(post, M.rz, true);
     if (down > 227 * 1024 || upr > 227 * 1024 || M.cl[0].smem > 227 * 1024 || M.cl[1].smem > 227 * 1024)
-        return fail(PIC_ERR_BAD_ARG, "multigrid: shared memory too large (sweeps %d/%d)", M.o.pre_sweeps,
-                    M.o.post_sweeps);
+        return fail(PIC_ERR_BAD_ARG, "multigrid: shared memory too large (sweeps %d/%d)", pre, post);
+    if (post <= kRtMaxSweeps && !(M.rz && sizeof(T) == 8))
+        PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(rt_res_kernel<T>(M, true)),
+                                 rt_stage_bytes(kRtMaxThreads)));
+    if (pre > kRtMaxSweeps) {
+        const DownKernel<T> k = M.rz ? down_kernel<T, true>(pre) : down_kernel<T, false>(pre);
+        PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(k), down));
+    }
+    if (post > kRtMaxSweeps) {
+        const UpKernel<T> k = M.rz ? up_kernel<T, true>(post) : up_kernel<T, false>(post);
+        const UpResKernel<T> r = M.rz ? up_res_kernel<T, true>(post) : up_res_kernel<T, false>(post);
+        PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(k), up));
+        PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(r), upr));
+    }
     if (M.rz) {
-        PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(down_kernel<T, true>(M.o.pre_sweeps)), down));
-        PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(up_kernel<T, true>(M.o.post_sweeps)), up));
-        PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(up_res_kernel<T, true>(M.o.post_sweeps)), upr));
         PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(k_mg_coarse<T, true>), M.cl[0].smem));
         return PIC_OK;  // r-z solves use the graph and host loops only
     }
-    PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(down_kernel<T, false>(M.o.pre_sweeps)), down));
-    PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(up_kernel<T, false>(M.o.post_sweeps)), up));
-    PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(up_res_kernel<T, false>(M.o.post_sweeps)), upr));
     PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(k_mg_coarse<T, false>), M.cl[0].smem));
     M.solve_smem = std::max(std::max(down, up), M.cl[1].smem);
     PIC_TRY(raise_smem_limit(reinterpret_cast<const void*>(k_mg_solve<T>), M.solve_smem));
