@@ -599,7 +599,10 @@ __device__ __forceinline__ bool rt_up_tile(const LevelDev<T>& F, const LevelDev<
             const T y = __shfl_down_sync(0xffffffffu, cv[q], 1);
             ce[q] = l == 31 ? x : y;
         }
-        if (sync.done()) return false;
+        if (sync.done()) {
+            if constexpr (STAGED) rt_copy_wait();  // no block ends with copies into it under way
+            return false;
+        }
         rt_prolong(t, cv, ce);
     }
     int buf = 0;
