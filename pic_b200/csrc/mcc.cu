@@ -241,8 +241,8 @@ int pic_mcc_apply(pic_mcc* m, int s, const float* d_x, const float* d_y, float* 
                births->capacity};
     const uint2 key = make_uint2(uint32_t(seed), uint32_t(seed >> 32));
     const int blocks = div_up(n, long(kMccBlockSegments) * kMccSegment);
-    k_mcc_apply<<<blocks, kMccBlockSegments, 0, as_stream(stream)>>>(m->h.dev, s, d_x, d_y, d_vx, d_vy, d_vz, n, step, key, B,
-                                                       d_counters);
+    k_mcc_apply<<<blocks, kMccBlockSegments, 0, as_stream(stream)>>>(m->h.dev, s, d_x, d_y, d_vx, d_vy, d_vz, n, step,
+                                                                     key, B, d_counters);
     PIC_LAUNCH_CHECK();
     return PIC_OK;
 }

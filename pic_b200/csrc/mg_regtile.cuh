@@ -246,8 +246,7 @@ __device__ __forceinline__ void rt_restrict(const T (&res)[kRtRows][2], RtShared
     }
 }
 
-// Loads g of the region (from g64, the FP64 residual, when given) and the
-// free bits.
+// Loads the free bits of a lane's rows, per column.
 template <class T>
 __device__ __forceinline__ void rt_load_bits(const LevelDev<T>& L, int i0, int j0, RtTile<T>& t) {
     const int nw = (L.ny + 31) >> 5;
@@ -474,8 +473,8 @@ __global__ void __launch_bounds__(kRtMaxThreads) k_rt_down(LevelDev<T> F, LevelD
 // Two blocks to an SM where 64 registers hold it (2049^2 69 us with one block,
 // 49 with two; r-z would spill: 129 x 97 step 1.7 us slower).
 template <class T, int S, bool CYL>
-__global__ void __launch_bounds__(kRtMaxThreads, sizeof(T) == 4 && !CYL ? 2 : 1) k_rt_init(LevelDev<T> F, LevelDev<T> C, T omega, RtInit I, NormState N,
-                                                           double tol2, int max_cycles, int decide) {
+__global__ void __launch_bounds__(kRtMaxThreads, sizeof(T) == 4 && !CYL ? 2 : 1)
+    k_rt_init(LevelDev<T> F, LevelDev<T> C, T omega, RtInit I, NormState N, double tol2, int max_cycles, int decide) {
     constexpr int HL = RtDown<S>::HL;
     static_assert(HL == RtUp<S, true>::HL, "the first residual's tiles are the residual up phase's");
     __shared__ RtShared<T> sh;
@@ -657,9 +656,8 @@ __device__ __forceinline__ double rt_block_sum(double v) {
 
 // The phase as a launch; RES: its norm and the loop decision too.
 template <class T, int S, bool CYL, int MODE>
-__global__ void __launch_bounds__(kRtMaxThreads, MODE == kRtResStaged ? 2 : 1) k_rt_up(LevelDev<T> F, LevelDev<T> C, T omega,
-                                                         double* __restrict__ phi, ResArgs R,
-                                                         const int* stop) {
+__global__ void __launch_bounds__(kRtMaxThreads, MODE == kRtResStaged ? 2 : 1)
+    k_rt_up(LevelDev<T> F, LevelDev<T> C, T omega, double* __restrict__ phi, ResArgs R, const int* stop) {
     __shared__ RtShared<T> sh;
     extern __shared__ double rt_stage[];
     double r2 = 0.0;
@@ -1078,7 +1076,9 @@ static RtShape rt_shape(int nx, int ny, Core core) {
     return best;
 }
 static RtShape rt_down_shape(int s, int nx, int ny) {
-    return rt_shape(nx, ny, [=](int n) { return s == 1 ? RtDown<1>::core(n) : s == 2 ? RtDown<2>::core(n) : RtDown<3>::core(n); });
+    return rt_shape(nx, ny, [=](int n) {
+        return s == 1 ? RtDown<1>::core(n) : s == 2 ? RtDown<2>::core(n) : RtDown<3>::core(n);
+    });
 }
 static RtShape rt_up_shape(int s, int nx, int ny, bool res) {
     return rt_shape(nx, ny, [=](int n) {
@@ -1087,10 +1087,14 @@ static RtShape rt_up_shape(int s, int nx, int ny, bool res) {
     });
 }
 static RtShape rt_down2_shape(int s, int nx, int ny) {
-    return rt_shape(nx, ny, [=](int n) { return s == 1 ? RtDown2<1>::core(n) : s == 2 ? RtDown2<2>::core(n) : RtDown2<3>::core(n); });
+    return rt_shape(nx, ny, [=](int n) {
+        return s == 1 ? RtDown2<1>::core(n) : s == 2 ? RtDown2<2>::core(n) : RtDown2<3>::core(n);
+    });
 }
 static RtShape rt_up2_shape(int s, int nx, int ny) {
-    return rt_shape(nx, ny, [=](int n) { return s == 1 ? RtUp2<1>::core(n) : s == 2 ? RtUp2<2>::core(n) : RtUp2<3>::core(n); });
+    return rt_shape(nx, ny, [=](int n) {
+        return s == 1 ? RtUp2<1>::core(n) : s == 2 ? RtUp2<2>::core(n) : RtUp2<3>::core(n);
+    });
 }
 
 }  // namespace pic

@@ -2597,12 +2597,22 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
     return PIC_OK;
 }
 
+// Blocks of the first residual (s: pre_sweeps) and of the residual up phase
+// (post_sweeps), and whether a cycle's decision can be left to the kernel after it.
+static int rt_res_blocks(int s, const MgImpl& M) {
+    const RtShape h = rt_up_shape(s, M.nx, M.ny, true);
+    return int(h.grid.x * h.grid.y);
+}
+static bool rt_defers(const MgImpl& M) {
+    return std::max(rt_res_blocks(M.o.pre_sweeps, M), rt_res_blocks(M.o.post_sweeps, M)) <= kRtPendingMax;
+}
+
 // The first K cycles of a register-tile solve (K >= 1) as plain launches.  The first
 // cycle's finest down phase forms the first residual (no launch of its own).
 // The first min_cycles cycles always run, and the ones before the last of them
 // end without a norm; the others do nothing once the solve has stopped.  rest:
-// a launch of k_rt_rest follows, which takes the last cycle's decision (there
-// are never more than kRtPendingMax blocks then).
+// a launch of k_rt_rest follows, which takes the last cycle's decision (only
+// where rt_defers).
 // How many (first_cycles): what the solve is expected to need.  A cycle divides
 // the residual by about 100 where all Dirichlet nodes are on the edges (r-z
 // sometimes takes one more).  A step's guess (min_cycles > 0), extrapolated from
@@ -2636,10 +2646,8 @@ static int launch_first_cycles(MgImpl& M, std::vector<LevelDev<T>>& lv, double* 
                                cudaStream_t st, RtPending* rest = nullptr) {
     const int kmin = std::max(0, std::min(min_cycles, max_cycles));
     const RtInit init{phi, f, M.rz0, M.r64, 1.0 / (M.dx * M.dx), 1.0 / (M.dy * M.dy)};
-    const RtShape h0 = rt_up_shape(M.o.pre_sweeps, M.nx, M.ny, true);
-    const RtShape h1 = rt_up_shape(M.o.post_sweeps, M.nx, M.ny, true);
-    const int b0 = int(h0.grid.x * h0.grid.y), b1 = int(h1.grid.x * h1.grid.y);
-    const bool defer = std::max(b0, b1) <= kRtPendingMax;
+    const int b0 = rt_res_blocks(M.o.pre_sweeps, M), b1 = rt_res_blocks(M.o.post_sweeps, M);
+    const bool defer = rt_defers(M);
     RtPending pending{};
     int last = 0;  // cycles finished at the last decision
     for (int k = 0; k < K; ++k) {
@@ -2670,14 +2678,14 @@ static int launch_first_cycles(MgImpl& M, std::vector<LevelDev<T>>& lv, double* 
 
 // Blocks of k_rt_rest for a solver: as many as the phase with the most tiles has
 // (and the direct solve can use); 0 where the WHILE node is used instead: more
-// tiles than SMs, sweeps that differ before and after, or a Dirichlet node off
-// the edges, where a solve takes twice the cycles that are launched in line
-// (385 x 193 FP64 with an electrode, to 1e-9: 432 us with k_rt_rest, 329
-// without).
+// tiles than SMs, more blocks than a decision can be left to the next kernel
+// with, sweeps that differ before and after, or a Dirichlet node off the edges,
+// where a solve takes twice the cycles that are launched in line (385 x 193 FP64
+// with an electrode, to 1e-9: 432 us with k_rt_rest, 329 without).
 template <class T>
 static int rest_blocks(const MgImpl& M, const std::vector<LevelDev<T>>& lv) {
     const int s = M.o.pre_sweeps;
-    if (!rt_cycles(M) || M.o.post_sweeps != s || !M.edges_only) return 0;
+    if (!rt_cycles(M) || M.o.post_sweeps != s || !M.edges_only || !rt_defers(M)) return 0;
     const int side = kRtRows * kRtMaxWarps, lsingle = M.fuse2 ? M.Lc - 2 : M.Lc;
     auto core = [&](auto k1, auto k2, auto k3, int n) { return s == 1 ? k1(n) : s == 2 ? k2(n) : k3(n); };
     auto tiles = [&](int l, int cx, int cy) { return long(div_up(lv[l].nx, cx)) * div_up(lv[l].ny, cy); };
