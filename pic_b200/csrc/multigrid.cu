@@ -97,6 +97,7 @@ struct NormState {
     int* stop;         // converged or at the cycle limit: cycles launched ahead of the test do nothing
     int* cycles;       // V-cycles of the current solve
     long long* total;  // V-cycles since creation
+    long long* loop;   // those that a graph's loop node or the host loop ran; null in a cycle in line
 };
 
 // The finest up phase fused with the FP64 residual (k_mg_up_res).
@@ -789,6 +790,7 @@ __device__ void norm_reduce_decide(double a, double b, const NormState& N, doubl
                 }
                 cyc += inc;
                 *N.total = tot + inc;
+                if (N.loop) *N.loop += inc;
             }
             *N.cycles = cyc;
             N.norms[1] = r2;
@@ -1794,6 +1796,7 @@ struct MgImpl {
     CoarseLayout cl[2];  // the coarse kernel's levels (from Lc) and the persistent/cluster ones (from Lp)
     long long launches = 0;  // kernels executed by solves
     int body_launches = 0;   // kernels per V-cycle (graph and host loops)
+    int fixed_launches = 1;  // kernels of a solve besides its loop's V-cycles, as last enqueued or captured
     // persistent cooperative solve
     int Lp = 0;
     size_t solve_smem = 0;
@@ -2422,6 +2425,7 @@ int mg_create(int nx, int ny, double dx, double dy, const uint8_t* h_mask, const
     M.N.converged = reinterpret_cast<int*>(small + 28);
     M.N.cycles = reinterpret_cast<int*>(small + 32);
     M.N.stop = reinterpret_cast<int*>(small + 36);
+    M.N.loop = reinterpret_cast<long long*>(small + 72);
     M.bar = reinterpret_cast<GridBar*>(small + 40);
     M.error = reinterpret_cast<int*>(small + 48);
     if (cudaStreamCreateWithFlags(&M.side, cudaStreamNonBlocking) != cudaSuccess ||
@@ -2453,6 +2457,7 @@ struct CycleOpts {
     bool decide = true;         // the cycle ends with the norm and the loop decision
     int inc = 1;                // cycles since the last decision
     int fblocks = 0;            // this is the solve's first decision, after a first residual of so many blocks
+    bool in_line = false;       // its launches count with the solve's, not with a loop's cycles
     const RtInit* init = nullptr;  // the solve's first cycle: its finest down phase forms the first residual ...
     bool init_decide = false;      // ... and takes the first decision
     bool defer = false;            // the decision is left to the kernel after the cycle ...
@@ -2574,6 +2579,7 @@ static int launch_cycle(MgImpl& M, std::vector<LevelDev<T>>& lv_in, double* phi,
         R.cx = 1.0 / (M.dx * M.dx);
         R.cy = 1.0 / (M.dy * M.dy);
         R.N = M.N;
+        if (O.in_line) R.N.loop = nullptr;
         R.tol2 = tol * tol;
         R.max_cycles = max_cycles;
         R.cond = cond;
@@ -2652,6 +2658,7 @@ static int launch_first_cycles(MgImpl& M, std::vector<LevelDev<T>>& lv, double* 
     int last = 0;  // cycles finished at the last decision
     for (int k = 0; k < K; ++k) {
         CycleOpts O;
+        O.in_line = true;
         if (k == 0) {
             O.init = &init;
             O.init_decide = kmin == 0;
@@ -2671,8 +2678,12 @@ static int launch_first_cycles(MgImpl& M, std::vector<LevelDev<T>>& lv, double* 
         // then, and a solve that stops earlier does not reach it
         PIC_TRY(launch_cycle(M, lv, phi, f, tol, max_cycles, cond, use_cond && k + 1 == K, st, count, O));
         M.body_launches = count;
+        M.fixed_launches = k ? M.fixed_launches + count : count;
     }
-    if (rest) *rest = pending;
+    if (rest) {
+        *rest = pending;
+        M.fixed_launches += 1;
+    }
     return PIC_OK;
 }
 
@@ -2778,6 +2789,7 @@ static int capture_solve(MgImpl& M, std::vector<LevelDev<T>>& lv, double* phi, c
         PIC_TRY(launch_first_cycles(M, lv, phi, f, tol, max_cycles, min_cycles, ahead, h, 1, st));
     } else {
         const int K = std::max(0, std::min(min_cycles, max_cycles));
+        M.fixed_launches = 1;
         launch_r0(M, lv, phi, f, tol, max_cycles, 1, h, K == 0, st);
         PIC_LAUNCH_CHECK();
         for (int k = 0; k < K; ++k) {
@@ -3090,12 +3102,15 @@ int mg_body_launches(pic_mg* mg) {
                             (M.o.launch_mode == PIC_MG_CLUSTER && M.cluster_ok);
     return one_kernel ? 0 : M.body_launches;
 }
-// Kernels a solve runs besides its V-cycles: the first residual (the first
-// cycle's own on register tiles), or the three sine-transform kernels and the
-// residual.
-int mg_fixed_launches(pic_mg* mg) {
-    if (!mg) return 1;
-    return mg->m.dst ? 4 : mg->m.o.launch_mode == PIC_MG_GRAPH_LOOP && rt_cycles(mg->m) ? 0 : 1;
+// Kernels a solve runs besides the V-cycles of its loop: the first residual, or the
+// cycles launched in line (the first forms it) and what follows them, or the three
+// sine-transform kernels and the residual.
+int mg_fixed_launches(pic_mg* mg) { return mg ? mg->m.dst ? 4 : mg->m.fixed_launches : 1; }
+// V-cycles of loops since creation.
+long long mg_loop_cycles(pic_mg* mg) {
+    long long t = 0;
+    if (mg) cudaMemcpy(&t, mg->m.N.loop, sizeof t, cudaMemcpyDeviceToHost);
+    return t;
 }
 int mg_capture_into(pic_mg* mg, double* phi, const double* f, double tol, int max_cycles, int min_cycles, bool alone,
                     cudaStream_t st) {

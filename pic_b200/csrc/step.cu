@@ -43,6 +43,7 @@ int mg_create(int nx, int ny, double dx, double dy, const uint8_t* h_mask, const
 int mg_body_launches(pic_mg* mg);
 int mg_fixed_launches(pic_mg* mg);
 long long mg_total_cycles(pic_mg* mg);
+long long mg_loop_cycles(pic_mg* mg);
 int mg_capture_into(pic_mg* mg, double* phi, const double* f, double tol, int max_cycles, int min_cycles, bool alone,
                     cudaStream_t st);
 int mg_launch_graph(pic_mg* mg, double* phi, const double* f, double tol, int max_cycles, int min_cycles,
@@ -1690,7 +1691,8 @@ struct SimImpl {
     bool kick_pending = false;
     long long steps = 0;
     long long launches = 0;  // launches outside the multigrid loop
-    long long solves = 0;    // multigrid solves issued (each runs 1 + cycles * body kernels)
+    long long solve_launches = 0;  // of the field solves, but for the V-cycles of their loops
+    long long step_solve = 0;      // those of a captured step
     bool profiling = false;
     cudaStream_t cap = nullptr, cap2 = nullptr;  // capture stream and the side branch of a captured step
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -1936,7 +1938,7 @@ static int field_solve(SimImpl& S, cudaStream_t st, bool capturing) {
         PIC_TRY(launch_update_E(S.phi, S.Ex, S.Ey, S.E2, S.ep, S.nx, S.ny, S.d.dx, S.d.dy, st, S.rz));
     }
     S.launches += 2;
-    S.solves += 1;
+    S.solve_launches += mg_fixed_launches(S.mg);
     return PIC_OK;
 }
 
@@ -1994,7 +1996,7 @@ static int sort_all_graph(SimImpl& S, cudaStream_t st) {
 static int capture_step(SimImpl& S, bool sort_next, cudaGraphExec_t* out) {
     const bool prof = S.profiling;
     S.profiling = false;
-    const long long l0 = S.launches, s0 = S.solves;
+    const long long l0 = S.launches, s0 = S.solve_launches;
     PIC_CUDA(cudaStreamBeginCapture(S.cap, cudaStreamCaptureModeThreadLocal));
     int rc = run_pass(S, S.cap, 1, 1, 1, 1, 1.0);
     bool forked = false;
@@ -2012,7 +2014,8 @@ static int capture_step(SimImpl& S, bool sort_next, cudaGraphExec_t* out) {
     const cudaError_t ec = cudaStreamEndCapture(S.cap, &g);
     S.profiling = prof;
     S.launches = l0;  // counted when the graph is launched
-    S.solves = s0;
+    S.step_solve = S.solve_launches - s0;
+    S.solve_launches = s0;
     if (rc != PIC_OK) {
         if (g) cudaGraphDestroy(g);
         return rc;
@@ -2301,6 +2304,7 @@ struct EnsImpl {
     long long* d_steps = nullptr;
     EnsControl* d_ctl = nullptr;
     cudaGraphExec_t exec = nullptr;
+    std::vector<long long> step_solve;         // per member, SimImpl::step_solve of the ensemble's step
     std::vector<long long> per_step_launches;  // per member, without the sort
     std::vector<long long> sort_launches;
     // one particle pass over every member (when every member uses the ring
@@ -2396,16 +2400,18 @@ static int ens_capture(EnsImpl& E) {
     std::vector<bool> prof;
     for (SimImpl* S : E.m) {
         l0.push_back(S->launches);
-        s0.push_back(S->solves);
+        s0.push_back(S->solve_launches);
         prof.push_back(S->profiling);
         S->profiling = false;
         S->in_ensemble = true;
     }
     const int rc = ens_capture_body(E);
+    E.step_solve.clear();
     for (size_t i = 0; i < E.m.size(); ++i) {
         E.m[i]->in_ensemble = false;
         E.m[i]->launches = l0[i];
-        E.m[i]->solves = s0[i];
+        E.step_solve.push_back(E.m[i]->solve_launches - s0[i]);
+        E.m[i]->solve_launches = s0[i];
         E.m[i]->profiling = prof[i];
     }
     return rc;
@@ -2636,7 +2642,7 @@ int pic_sim_step(pic_sim* sim, int n_steps, void* stream) {
             // items and the pass (with collisions: candidate bits and k_collide), the RHS and E
             S.launches +=
                 2 + (S.have_mcc ? 2 : 0) + 2 + (sort_next ? 1 + (long long)S.ns * (5 + 3 * S.sorter.passes) : 0);
-            S.solves += 1;
+            S.solve_launches += S.step_solve;
             S.prepared = true;
         } else {
             const int k = S.kick_pending ? 1 : 0;
@@ -2847,8 +2853,7 @@ long long pic_sim_kernel_launches(pic_sim* sim) {
     if (!sim) return 0;
     SimImpl& S = sim->s;
     cudaDeviceSynchronize();
-    // each solve runs its residual kernel plus `body` kernels per V-cycle
-    return S.launches + S.solves * mg_fixed_launches(S.mg) + mg_total_cycles(S.mg) * mg_body_launches(S.mg);
+    return S.launches + S.solve_launches + mg_loop_cycles(S.mg) * mg_body_launches(S.mg);
 }
 
 int pic_sim_set_profiling(pic_sim* sim, int enable) {
@@ -2996,7 +3001,8 @@ int pic_ens_step(pic_ens* e, int n_steps, void* stream) {
     PIC_CUDA(cudaGraphLaunch(E.exec, st));
     // the ensemble's body prepares each pass itself
     for (SimImpl* S : E.m) S->prepared = false;
-    for (SimImpl* S : E.m) {
+    for (size_t i = 0; i < E.m.size(); ++i) {
+        SimImpl* S = E.m[i];
         long long sorts = 0;
         if (S->d.sort_interval > 0)
             for (long long k = S->steps; k < S->steps + n_steps; ++k) sorts += (k % S->d.sort_interval == 0);
@@ -3007,7 +3013,7 @@ int pic_ens_step(pic_ens* e, int n_steps, void* stream) {
         S->launches += n_steps * (1LL + pass + (S->have_mcc ? 2 : 0) + 2) +
                        sorts * (1 + (long long)S->ns * (5 + 3 * S->sorter.passes));
         if (S->d.sort_interval > 0) S->launches += n_steps;  // the sort condition
-        S->solves += n_steps;
+        S->solve_launches += n_steps * E.step_solve[i];
         S->steps += n_steps;
     }
     return PIC_OK;
