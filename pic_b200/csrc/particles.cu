@@ -1,6 +1,7 @@
 // Stateless particle and grid operators: the drop-in kernels behind
 // Particles2D.update_R / update_V, Grid2D.update_density / update_E and the
 // Poisson right-hand side.  Positions are float32 grid units, velocities m/s.
+#include <algorithm>
 #include <cstring>
 #include <string>
 
@@ -117,6 +118,10 @@ __global__ void k_deposit(const float* __restrict__ x, const float* __restrict__
 // (4M on 513^2: 82 -> 25 us, 81 -> 40 us); the node sums and the pairs cost
 // about 3 us each once per call.
 
+// Blocks of a pass over the nodes, a row each while a grid can have so many (any
+// number of rows is accepted).
+static dim3 node_grid(int nx, int ny) { return dim3(div_up(nx, 128), std::min(ny, 65535)); }
+
 // cells[j * nx + i] += scale * (w00, w10, w01, w11) of each live particle.
 __global__ void k_deposit_cells(const float* __restrict__ x, const float* __restrict__ y, int n, float scale,
                                 float4* __restrict__ cells, int nx, int ny) {
@@ -135,24 +140,28 @@ __global__ void k_deposit_cells(const float* __restrict__ x, const float* __rest
 // of the last column or row holds particles on the edge itself, whose weights
 // for the nodes beyond are exactly zero.)
 __global__ void k_cells_density(const float4* __restrict__ cells, float* __restrict__ rho, int nx, int ny) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nx) return;
-    const long k = long(j) * nx + i;
-    const bool w = i > 0, s = j > 0;
-    double v = double(cells[k].x);
-    if (w) v += double(cells[k - 1].y);
-    if (s) v += double(cells[k - nx].z);
-    if (w && s) v += double(cells[k - nx - 1].w);
-    rho[k] = float(v);
+    for (int j = blockIdx.y; j < ny; j += gridDim.y) {
+        const long k = long(j) * nx + i;
+        const bool w = i > 0, s = j > 0;
+        double v = double(cells[k].x);
+        if (w) v += double(cells[k - 1].y);
+        if (s) v += double(cells[k - nx].z);
+        if (w && s) v += double(cells[k - nx - 1].w);
+        rho[k] = float(v);
+    }
 }
 
 // pairs[k] = (Ex, Ey) at node k and at its east neighbour (itself on the last column).
 __global__ void k_field_pairs(const float* __restrict__ Ex, const float* __restrict__ Ey, float4* __restrict__ pairs,
                               int nx, int ny) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nx) return;
-    const long k = long(j) * nx + i, e = i + 1 < nx ? k + 1 : k;
-    pairs[k] = make_float4(Ex[k], Ey[k], Ex[e], Ey[e]);
+    for (int j = blockIdx.y; j < ny; j += gridDim.y) {
+        const long k = long(j) * nx + i, e = i + 1 < nx ? k + 1 : k;
+        pairs[k] = make_float4(Ex[k], Ey[k], Ex[e], Ey[e]);
+    }
 }
 
 // k_update_V from node pairs: the same arithmetic, two loads per particle.
@@ -341,8 +350,8 @@ int pic_cells_density(const float* d_cells, float* d_rho, int nx, int ny, void* 
     clear_error();
     if (nx < 2 || ny < 2 || !d_rho || !d_cells || (reinterpret_cast<uintptr_t>(d_cells) & 15))
         return fail(PIC_ERR_BAD_ARG, "pic_cells_density: bad arguments");
-    k_cells_density<<<dim3(div_up(nx, 128), ny), 128, 0, as_stream(stream)>>>(
-        reinterpret_cast<const float4*>(d_cells), d_rho, nx, ny);
+    k_cells_density<<<node_grid(nx, ny), 128, 0, as_stream(stream)>>>(reinterpret_cast<const float4*>(d_cells), d_rho, nx,
+                                                                      ny);
     PIC_LAUNCH_CHECK();
     return PIC_OK;
 }
@@ -351,8 +360,8 @@ int pic_field_pairs(const float* d_Ex, const float* d_Ey, float* d_pairs, int nx
     clear_error();
     if (nx < 2 || ny < 2 || !d_Ex || !d_Ey || !d_pairs || (reinterpret_cast<uintptr_t>(d_pairs) & 15))
         return fail(PIC_ERR_BAD_ARG, "pic_field_pairs: bad arguments");
-    k_field_pairs<<<dim3(div_up(nx, 128), ny), 128, 0, as_stream(stream)>>>(d_Ex, d_Ey,
-                                                                           reinterpret_cast<float4*>(d_pairs), nx, ny);
+    k_field_pairs<<<node_grid(nx, ny), 128, 0, as_stream(stream)>>>(d_Ex, d_Ey, reinterpret_cast<float4*>(d_pairs), nx,
+                                                                    ny);
     PIC_LAUNCH_CHECK();
     return PIC_OK;
 }
