@@ -107,10 +107,12 @@ class MccOperator:
         self.seed = int(seed)
         self.step = 0
         dev = "cuda"
-        # the birth buffer's arrays are rows of one tensor, so that taking births is one copy
-        self._births = torch.zeros((6, birth_capacity), dtype=torch.float32, device=dev)
-        self.bx, self.by, self.bvx, self.bvy, self.bvz = self._births[:5].unbind()
-        self.bspecies = self._births[5].view(torch.int32)
+        # the birth buffer's arrays are rows of one tensor, so that taking births is one
+        # copy; of a multiple of 128 floats, each is aligned as a tensor of its own
+        self._births = torch.zeros((6, -(-birth_capacity // 128) * 128), dtype=torch.float32, device=dev)
+        rows = self._births[:, :birth_capacity]
+        self.bx, self.by, self.bvx, self.bvy, self.bvz = rows[:5].unbind()
+        self.bspecies = rows[5].view(torch.int32)
         self.bcount = torch.zeros(1, dtype=torch.int32, device=dev)
         self.counters = torch.zeros(30, dtype=torch.int64, device=dev)
         self._bb = _lib.BirthBuffer(self.bx.data_ptr(), self.by.data_ptr(), self.bvx.data_ptr(), self.bvy.data_ptr(),
@@ -131,7 +133,7 @@ class MccOperator:
 
     def take_births(self):
         k = min(int(self.bcount.item()), self.bx.numel())
-        rows = self._births[:, :k].clone()
+        rows = self._births[:, : -(-k // 128) * 128].clone()[:, :k]
         out = (rows[5].view(torch.int32), *rows[:5].unbind())
         self.bcount.zero_()
         return out
