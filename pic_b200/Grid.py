@@ -60,9 +60,7 @@ class Grid2D:
     def update_density(self, particles):
         """CIC charge deposit of every species, rho in C/m^3 (src/Grid.py:246-294);
         r-z: divided by the node volumes (pic_rz_density)."""
-        if self._dense(particles):
-            if self._cells is None:
-                self._cells = torch.empty((self.node_count, 4), dtype=torch.float32, device=DEVICE)
+        if self._dense(particles) and self._scratch("_cells"):
             self._cells.zero_()
             fn, target = "pic_deposit_cells", self._cells
         else:
@@ -84,12 +82,19 @@ class Grid2D:
         n = sum(s.n for s in particles.species)
         return n >= max(DENSE_PARTICLES, DENSE_PER_NODE * self.node_count)
 
+    def _scratch(self, name):
+        """Whether the dense path's scratch is there: made at first use, if the device has room for it."""
+        if getattr(self, name) is None:
+            try:
+                setattr(self, name, torch.empty((self.node_count, 4), dtype=torch.float32, device=DEVICE))
+            except torch.OutOfMemoryError:
+                return False
+        return True
+
     def field_pairs(self, particles):
         """E as node pairs (pic_field_pairs) for the gather of `particles`, or None where the planes serve better."""
-        if self.node_count > PAIR_NODES or not self._dense(particles):
+        if self.node_count > PAIR_NODES or not self._dense(particles) or not self._scratch("_pairs"):
             return None
-        if self._pairs is None:
-            self._pairs = torch.empty((self.node_count, 4), dtype=torch.float32, device=DEVICE)
         _lib.call("pic_field_pairs", _lib.ptr(self.E[0]), _lib.ptr(self.E[1]), _lib.ptr(self._pairs), self.m, self.n,
                   _lib.stream_ptr())
         return self._pairs
