@@ -2,7 +2,7 @@
 
 A solve that starts from the converged potential does no cycle: it must cost well under
 half of the five-cycle solve from zero (launches that only find out that there is nothing
-to do made it 0.65 to 0.8 of it).  Fastest of 30 calls each, so that a busy host does not
+to do made it 0.65 to 0.8 of it).  Fastest of 100 calls each, so that a busy host does not
 decide.
 
 A simulation's in-line cycles: the step's reported residual is below the tolerance and is
@@ -35,7 +35,7 @@ def box(n):
 
 def fastest(solve, phi, guess):
     best = 1.0
-    for _ in range(30):
+    for _ in range(100):
         phi.copy_(guess)
         torch.cuda.synchronize()
         t = time.perf_counter()
