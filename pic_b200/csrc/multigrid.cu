@@ -12,10 +12,9 @@
 //
 // Kernels per V-cycle in the graph and host loops (7 launches for a 513^2
 // grid):
-//   down(l)     2*pre red/black half-sweeps on a 32x32 tile held in shared
-//               memory with a halo wide enough for them, then the residual
-//               and its full-weighting restriction to level l+1; on level 0
-//               the right-hand side is the FP64 residual r
+//   down(l)     2*pre red/black half-sweeps on a tile with a halo wide enough for
+//               them, then the residual and its full-weighting restriction to
+//               level l+1; on level 0 the right-hand side is the FP64 residual r
 //   down2       the down phases of two levels (129^2 and 65^2 at 513^2) in
 //               one launch, over halos wide enough that the coarser level's
 //               tile equals what two launches give
@@ -25,15 +24,20 @@
 //   up2         the up phases of the same two levels in one launch
 //   up(l)       prolongation-add of level l+1 and 2*post half-sweeps
 //   up_res      the finest up phase: phi += e, the FP64 residual updated on
-//               the tile (r -= A e), its norm (deterministic last-block
-//               reduction) and the loop decision
-//   r0          once per solve, before the first cycle: r = f - A phi in
-//               FP64, its norm and the first loop decision
+//               the tile (r -= A e), its norm and the loop decision
+// Up to three sweeps run on register tiles (k_rt_*, mg_regtile.cuh), more on
+// 32 x 32 tiles in shared memory (k_mg_*, here; also the persistent solve's).
+// The first residual, r = f - A phi in FP64:
+//   r0          a launch of its own with the first loop decision, where a solve
+//               may have nothing to do (pic_mg_solve, a step with min_cycles 0)
+//   k_rt_init   formed by the first cycle's finest down phase, where cycles are
+//               launched in line (steps, the adjoint's solves; first_cycles)
 // The single-CTA coarse kernel (every level of at most 33^2 nodes in shared
 // memory, down to a dense solve) serves grids that small and the persistent
 // and cluster modes.  The loop is a CUDA-graph conditional WHILE node whose
-// condition up_res (r0 before the first cycle) sets, so a solve issues no
-// host synchronisation.
+// condition up_res (r0 before the first cycle) sets, or, after cycles in line on
+// grids of one wave of tiles, one cooperative launch (k_rt_rest); either way a
+// solve issues no host synchronisation.
 #include <cooperative_groups.h>
 #include <cuda/atomic>
 
