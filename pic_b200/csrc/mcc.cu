@@ -101,19 +101,25 @@ void mcc_free(MccHost* H) {
 // The collision operator on its own.  What bounds it is the chain of one
 // candidate (draws, the bin's table loads, Philox rounds, the scattering), so
 // the block gives every thread a segment to draw and then every thread a
-// candidate, however the candidates fall on the segments: kMccBlockSegments
-// segments of 256 slots per block, the candidates numbered by a scan of the
-// segments' counts.  Counts are summed in shared memory first.  (One lane in
-// sixteen drawing, the block then stepping over its slots: 20.5 us for 4M
-// electrons; this way 8.5 us.)
-constexpr int kMccBlockSegments = 128;
+// candidate, however the candidates fall on the segments: `segs` segments of 256
+// slots per block, the candidates numbered by a scan of the segments' counts.
+// Counts are summed in shared memory first.  (One lane in sixteen drawing, the
+// block then stepping over its slots: 20.5 us for 4M electrons; this way 8.5 us.)
+// segs (mcc_segments): as many as a block has threads where few slots collide; in
+// a dense gas only so many that a thread has kMccPerThread candidates on average,
+// but never so few that the blocks (kMccResident to an SM) make a second wave, as
+// drawing then leaves most of a block idle.  Measured, with 128 segments and by
+// this rule: a candidate in two slots, 200k electrons 382 and 80 us, 1M 383 and 93,
+// 16M 503 and 327; one in fifteen, 200k 77 and 33; one in 400, 4M 24 and 24.
+constexpr int kMccBlockSegments = 128;  // most segments of a block, and its threads
+constexpr int kMccPerThread = 2, kMccResident = 7;
 constexpr int kMccWords = int(kMccSegment) / 32;
 
 __global__ void __launch_bounds__(kMccBlockSegments) k_mcc_apply(const __grid_constant__ MccDev M, int s,
                                                                  const float* __restrict__ x,
                                                                  const float* __restrict__ y, float* __restrict__ vx,
                                                                  float* __restrict__ vy, float* __restrict__ vz, int n,
-                                                                 uint32_t step, uint2 key, BirthDev B,
+                                                                 uint32_t step, uint2 key, BirthDev B, int segs,
                                                                  unsigned long long* __restrict__ ctr) {
     __shared__ unsigned bits[kMccBlockSegments * (kMccWords + 1)];  // a segment's words, padded against bank conflicts
     __shared__ int first[kMccBlockSegments + 1];                    // the number of each segment's first candidate
@@ -121,13 +127,13 @@ __global__ void __launch_bounds__(kMccBlockSegments) k_mcc_apply(const __grid_co
     __shared__ unsigned cnt[PIC_MAX_PROCESSES + 3];  // collisions, candidates, overflows, dropped births
     const MccSpeciesDev& S = M.sp[s];
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const long g = long(blockIdx.x) * kMccBlockSegments + t;
+    const long g = long(blockIdx.x) * segs + t;
     unsigned* mine = bits + t * (kMccWords + 1);
 #pragma unroll
     for (int q = 0; q < kMccWords; ++q) mine[q] = 0u;
     if (t < PIC_MAX_PROCESSES + 3) cnt[t] = 0u;
     const long b = g * long(kMccSegment);
-    if (b < n)
+    if (t < segs && b < n)
         mcc_mark_segment(S, uint32_t(s), g, n, int(b), int(min(long(n), b + long(kMccSegment))), step, key, mine);
     int c = 0;
 #pragma unroll
@@ -147,7 +153,7 @@ __global__ void __launch_bounds__(kMccBlockSegments) k_mcc_apply(const __grid_co
     __syncthreads();
     const int total = first[kMccBlockSegments];
     for (int k = t; k < total; k += kMccBlockSegments) {
-        int lo = 0, hi = kMccBlockSegments - 1;  // the last segment whose first candidate is <= k
+        int lo = 0, hi = segs - 1;  // the last segment whose first candidate is <= k
         while (lo < hi) {
             const int mid = (lo + hi + 1) >> 1;
             if (first[mid] <= k) lo = mid;
@@ -157,7 +163,7 @@ __global__ void __launch_bounds__(kMccBlockSegments) k_mcc_apply(const __grid_co
         int r = k - first[lo], q = 0;
         const unsigned* words = bits + lo * (kMccWords + 1);
         while (r >= __popc(words[q])) r -= __popc(words[q++]);
-        const int p = int((long(blockIdx.x) * kMccBlockSegments + lo) * long(kMccSegment)) + 32 * q +
+        const int p = int((long(blockIdx.x) * segs + lo) * long(kMccSegment)) + 32 * q +
                       int(__fns(words[q], 0u, r + 1));
         const float px = x[p], py = y[p];
         if (!is_live(px)) continue;
@@ -184,6 +190,16 @@ __global__ void __launch_bounds__(kMccBlockSegments) k_mcc_apply(const __grid_co
                                                     : kCtrDropped;
         atomicAdd(ctr + at, (unsigned long long)cnt[t]);
     }
+}
+
+// Segments of a block of k_mcc_apply.
+static int mcc_segments(int n, double p) {
+    const double one_wave = double(n) / (double(kMccSegment) * kMccResident * num_sms());
+    int segs = kMccBlockSegments;
+    while (segs > 1 && segs / 2 >= one_wave &&
+           segs * double(kMccSegment) * p > kMccPerThread * double(kMccBlockSegments))
+        segs /= 2;
+    return segs;
 }
 
 }  // namespace pic
@@ -240,9 +256,10 @@ int pic_mcc_apply(pic_mcc* m, int s, const float* d_x, const float* d_y, float* 
     BirthDev B{births->x, births->y, births->vx, births->vy, births->vz, births->species, births->count,
                births->capacity};
     const uint2 key = make_uint2(uint32_t(seed), uint32_t(seed >> 32));
-    const int blocks = div_up(n, long(kMccBlockSegments) * kMccSegment);
+    const int segs = mcc_segments(n, m->h.p_null[s]);
+    const int blocks = div_up(n, long(segs) * kMccSegment);
     k_mcc_apply<<<blocks, kMccBlockSegments, 0, as_stream(stream)>>>(m->h.dev, s, d_x, d_y, d_vx, d_vy, d_vz, n, step,
-                                                                     key, B, d_counters);
+                                                                     key, B, segs, d_counters);
     PIC_LAUNCH_CHECK();
     return PIC_OK;
 }
