@@ -755,11 +755,12 @@ __device__ void norm_reduce_decide(double a, double b, const NormState& N, doubl
     __threadfence();
     // the solve's state and every block partial, loaded together
     int cyc = 0;
-    long long tot = 0;
+    long long tot = 0, loop = 0;
     double ref0 = 0.0;
     if (t == 0) {
         cyc = *reinterpret_cast<volatile int*>(N.cycles);
         tot = *reinterpret_cast<volatile long long*>(N.total);
+        if (N.loop) loop = *reinterpret_cast<volatile long long*>(N.loop);
         ref0 = *reinterpret_cast<volatile double*>(N.norms);
     }
     const volatile double* P = N.partial;
@@ -794,7 +795,7 @@ __device__ void norm_reduce_decide(double a, double b, const NormState& N, doubl
                 }
                 cyc += inc;
                 *N.total = tot + inc;
-                if (N.loop) *N.loop += inc;
+                if (N.loop) *N.loop = loop + inc;
             }
             *N.cycles = cyc;
             N.norms[1] = r2;
