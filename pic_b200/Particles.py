@@ -25,6 +25,14 @@ from . import _lib
 DEVICE = "cuda"
 
 
+# Particles in cell order gather from the field's planes as fast as from node pairs,
+# which take a pass to build: up to about two cells of spread (1M + 1M particles on
+# 257^2 nodes: in order 11.8 us against 13.0, spread by one cell 14.6 and 15.1, by
+# three 18.1 and 17.2, unordered 38.4 and 23.6).  Electrons of 2 eV spread by two
+# cells in some 40 steps.
+SORTED_MOVES = 40
+
+
 class Species:
     """One species' SoA arrays (capacity slots; the first n are in use)."""
 
@@ -58,6 +66,7 @@ class Particles2D:
         self.mcc_count = 0
         self._gen = torch.Generator(device="cpu")
         self._gen.manual_seed(0)
+        self._moves = None  # update_R calls since the last sort; None: in no known order
 
     # ---- species tables (src/Particles.py:318-352) ----
     def add_species(self, species_name: str, species_mass: float, species_charge: float, collision_model: int = 0):
@@ -137,6 +146,7 @@ class Particles2D:
         for dst, src in zip(s.arrays(), cols):
             dst[s.n:s.n + n].copy_(src.reshape(-1))
         s.n += n
+        self._moves = None
 
     def uniform_species_load(self, x1, y1, x2, y2, n, species, grid=None):
         """Uniform positions in [x1,x2]x[y1,y2]; vx one U(-0.1,0.1) value, vy = 0,
@@ -186,6 +196,8 @@ class Particles2D:
     def update_R(self, dt):
         """x += v dt (src/Particles.py:359-367); r-z: the drift of pic_update_R_rz."""
         g = self._require_grid()
+        if self._moves is not None:
+            self._moves += 1
         for s in self.species:
             if not s.n:
                 continue
@@ -210,7 +222,8 @@ class Particles2D:
     def update_V(self, grid, dt):
         """Gather E at each particle and kick v += q/m E dt (src/Particles.py:378-410)."""
         self.grid = grid
-        pairs = grid.field_pairs(self) if hasattr(grid, "field_pairs") else None
+        sorted_ = self._moves is not None and self._moves <= SORTED_MOVES
+        pairs = grid.field_pairs(self) if hasattr(grid, "field_pairs") and not sorted_ else None
         for s in self.species:
             if not s.n:
                 continue
@@ -271,4 +284,5 @@ class Particles2D:
             finally:
                 torch.cuda.synchronize()
                 _lib.load().pic_sorter_destroy(sorter)
+        self._moves = 0
         return perms
